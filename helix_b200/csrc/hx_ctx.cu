@@ -62,6 +62,7 @@ void release(hx_ctx* c)
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
+    if (c->flag_pin) cudaFreeHost(c->flag_pin);
     if (c->state_pinned) cudaFreeHost(c->state_pinned);
     if (c->own_stream) cudaStreamDestroy(c->own_stream);
     delete c;
@@ -321,24 +322,39 @@ int launch_stage_core(hx_ctx* c, const double2* u, const double2* rho, double2* 
     return 1;
 }
 
-// Enqueue one integrator step (Horner form of the order-m Taylor polynomial).
-int enqueue_step(hx_ctx* c)
+// Whole steps of a small-slab hierarchy run in one launch (hx_small.cu).
+bool runs_whole_steps(const hx_ctx* c) { return c->use_small_step && !c->closure; }
+
+// Enqueue nsteps steps of such a hierarchy; trace / obs as in launch_small_run.
+void enqueue_run(hx_ctx* c, uint64_t nsteps, double2* trace, double* obs)
 {
-    const int m = c->order;
-    int launched = 0;
-    if (c->use_small_step && !c->closure) {
+    constexpr uint64_t kMostSteps = 4096;  // of one launch
+    for (uint64_t done = 0; done < nsteps;) {
+        const int n = static_cast<int>(std::min(nsteps - done, kMostSteps));
         hx::StepWait w;
         if (c->stall_next_step) {  // test hook: one arrival more than the CTAs make, a short wait
             w.skew = 1;
             w.max_polls = 1u << 12;
             c->stall_next_step = false;
         }
-        if (hx::launch_small_step(hx::fused_args_of(c), c->rho, c->ua, c->ub, c->dt, m, c->gbar, c->stream, false,
-                                  w) != 1)
+        if (hx::launch_small_run(hx::fused_args_of(c), c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->sm_count,
+                                 c->stream, false, trace ? trace + done * c->slab : nullptr,
+                                 obs ? obs + 3 * done : nullptr, w) != 1)
             c->launch_failed = true;
         c->counters.kernel_launches += 1;
-        c->counters.stage_launches += m;
-        c->steps_done += 1;
+        c->counters.stage_launches += static_cast<uint64_t>(c->order) * n;
+        c->steps_done += n;
+        done += n;
+    }
+}
+
+// Enqueue one integrator step (Horner form of the order-m Taylor polynomial).
+int enqueue_step(hx_ctx* c)
+{
+    const int m = c->order;
+    int launched = 0;
+    if (runs_whole_steps(c)) {
+        enqueue_run(c, 1, nullptr, nullptr);
         return HX_OK;
     }
     if (m == 1) {
@@ -361,12 +377,18 @@ int enqueue_step(hx_ctx* c)
     return HX_OK;
 }
 
-// Energy and trace of rho_0 into out[0..2].
-void launch_obs(hx_ctx* c, double* out)
+// Energy and trace of rho_0 into out[0..2]; rho_0 itself into copy (if not nullptr), by the same kernel
+// where the slab is small enough for one block (d <= 64).
+int launch_obs(hx_ctx* c, double* out, double2* copy = nullptr)
 {
-    if (c->use_csr || c->dense)
+    const bool csr = c->use_csr || c->dense;
+    const bool fold = copy && !csr && c->logd <= hx::kMaxLogD;
+    if (csr)
         hx::launch_observables_csr(c->rho, c->logd, c->csr_ptr, c->csr_col, c->csr_val, out, c->stream);
-    else hx::launch_observables(c->rho, c->logd, c->herm, c->hdiag, c->hflip, nullptr, out, c->stream);
+    else hx::launch_observables(c->rho, c->logd, c->herm, c->hdiag, c->hflip, fold ? copy : nullptr, out, c->stream);
+    if (copy && !fold)
+        HX_CUDA_TRY(cudaMemcpyAsync(copy, c->rho, c->slab_store * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
+    return HX_OK;
 }
 
 int check_launch(const char* what)
@@ -376,21 +398,34 @@ int check_launch(const char* what)
     return HX_OK;
 }
 
-int read_error_flag(hx_ctx* c)
+// Enqueue the copy of the error word that flag_status reads after the next synchronisation.
+int enqueue_flag(hx_ctx* c)
+{
+    if (!c->flag_pin) HX_CUDA_TRY(cudaMallocHost(&c->flag_pin, sizeof(int)));
+    HX_CUDA_TRY(cudaMemcpyAsync(c->flag_pin, c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    return HX_OK;
+}
+
+int flag_status(hx_ctx* c)
 {
     if (c->launch_failed) {
         c->launch_failed = false;
-        return fail(HX_ERR_UNSUPPORTED_EXECUTION, "the tensor-core product of a stage could not be enqueued");
+        return fail(HX_ERR_UNSUPPORTED_EXECUTION, "a kernel of a stage could not be enqueued");
     }
-    int flag = 0;
-    HX_CUDA_TRY(cudaMemcpyAsync(&flag, c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    if (flag != 0) {
+    if (*c->flag_pin != 0) {
         cudaMemsetAsync(c->error_flag, 0, sizeof(int), c->stream);
         if (c->gbar) cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);  // a barrier that gave up
         return fail(HX_ERR_DEVICE_TIMEOUT, "a device-side wait ran out of its iteration budget");
     }
     return HX_OK;
+}
+
+int read_error_flag(hx_ctx* c)
+{
+    const int rc = enqueue_flag(c);
+    if (rc != HX_OK) return rc;
+    HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    return flag_status(c);
 }
 
 // Packed slab from a full row-major complex matrix (2 d^2 doubles); false
@@ -458,20 +493,21 @@ int state_staging(hx_ctx* c, size_t elems)
     return HX_OK;
 }
 
-// count slabs of a packed device buffer into full matrices on the host.
+// count slabs of a packed device buffer into full matrices on the host; reports the error word too.
 int read_herm(hx_ctx* c, const double2* src, size_t count, double* out)
 {
     const size_t n = count * c->slab_store;
     int rc = state_staging(c, n);
     if (rc != HX_OK) return rc;
     HX_CUDA_TRY(cudaMemcpyAsync(c->state_pinned, src, n * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
+    if ((rc = enqueue_flag(c)) != HX_OK) return rc;
     HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->counters.d2h_bytes += n * sizeof(double2);
     const double2* pk = c->state_pinned;
     parallel_for(static_cast<long long>(count), [&](long long k) {
         hx::unpack_herm_host(pk + k * c->slab_store, c->logd, out + 2 * k * c->slab);
     });
-    return HX_OK;
+    return flag_status(c);
 }
 
 // One operator in compressed rows, host side, before upload.
@@ -1022,7 +1058,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             // small slabs: every up neighbour in the entry lists (no up-term pass)
             const bool want_small = small_ok && all_pauli;
             hx::launch_entries(c->rows, c->edges, c->acoef, c->bcoef, c->bath_off, c->H, M, J,
-                               static_cast<int>(p->max_depth) + (want_small ? 1 : 0), c->ent_count,
+                               static_cast<int>(p->max_depth) + (small_ok ? 1 : 0), c->ent_count,
                                c->ent_slab,
                                c->ent_bath, c->ent_wc, c->ent_wa, c->ado_keep, c->stream);
             rc = check_launch("fused-kernel setup");
@@ -1064,15 +1100,18 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             c->up_slots = S;
             c->use_fused = (rc == HX_OK) && fused_ok;
             c->use_small = (rc == HX_OK) && want_small;
-            // small slabs: the whole step in one cooperative launch when every ADO fits the resident CTAs
+            // small slabs: whole steps in one launch when the hierarchy fits the resident CTAs
             const char* step_env = std::getenv("HX_SMALL_STEP");
-            if (c->use_small && c->order >= 2 && !(step_env && step_env[0] == '0') &&
+            if (rc == HX_OK && small_ok && c->order >= 2 && !(step_env && step_env[0] == '0') &&
                 (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
                 e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
                 if (e != cudaSuccess) rc = hx::cuda_fail(e, "grid barrier counter");
                 else
-                    c->use_small_step = hx::launch_small_step(hx::fused_args_of(c), c->rho, c->ua, c->ub, c->dt,
-                                                              c->order, c->gbar, c->stream, true) == 1;
+                    c->use_small_step = hx::launch_small_run(hx::fused_args_of(c), c->rho, c->ua, c->ub, c->dt,
+                                                             c->order, 1, c->gbar, c->sm_count, c->stream, true,
+                                                             nullptr, nullptr) == 1;
+                if (rc == HX_OK && c->use_small_step && (rc = dev_alloc(c, &c->order_perm, H)) == HX_OK)
+                    hx::launch_run_order(c->ent_count, c->H, c->order_perm, c->stream);
             }
             // single-precision copies of the operators for the mixed band kernel
             if (rc == HX_OK && c->mixed) {
@@ -1142,7 +1181,7 @@ int hx_ctx_info(const hx_ctx* c, hx_info* info)
     int per_stage = (c->use_flip || c->use_csr || (c->use_fused && c->up_slots > 0)) ? 2 : 1;
     if (c->use_large) per_stage = 1 + (c->up_slots > 0 ? 1 : 0) + (c->mixed ? 1 : 0) + (c->dense ? 2 : 0);
     info->kernels_per_step = static_cast<uint32_t>(c->order) * per_stage;
-    if (c->use_small_step && !c->closure) info->kernels_per_step = 1;
+    if (runs_whole_steps(c)) info->kernels_per_step = 1;
     info->stage_path = c->dense     ? HX_PATH_DENSE
                        : c->use_csr ? HX_PATH_CSR
                        : c->use_flip ? HX_PATH_FLIP
@@ -1163,14 +1202,15 @@ int hx_ctx_counters(const hx_ctx* c, hx_counters* out)
 int hx_ctx_step(hx_ctx* c, uint64_t nsteps)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    for (uint64_t s = 0; s < nsteps; ++s) enqueue_step(c);
+    if (runs_whole_steps(c)) enqueue_run(c, nsteps, nullptr, nullptr);
+    else
+        for (uint64_t s = 0; s < nsteps; ++s) enqueue_step(c);
     return check_launch("stage kernel launch");
 }
 
 int hx_ctx_sync(hx_ctx* c)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     return read_error_flag(c);
 }
 
@@ -1180,7 +1220,8 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
     // chunk of steps buffered on the device: at most 256 steps and 64 MB of rho_0 copies
     const uint64_t by_bytes = std::max<uint64_t>(1, (uint64_t(64) << 20) / (c->slab * sizeof(double2)));
     const int cap = static_cast<int>(std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(nsteps, 1), 256), by_bytes));
-    if (c->trace_cap < cap) {
+    const bool whole = runs_whole_steps(c);
+    if (c->trace_cap < cap || (!whole && !c->trace_buf)) {
         if (c->trace_buf) cudaFree(c->trace_buf);
         if (c->energy_buf) cudaFree(c->energy_buf);
         if (c->pinned) cudaFreeHost(c->pinned);
@@ -1188,8 +1229,10 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
         c->energy_buf = nullptr;
         c->pinned = nullptr;
         c->trace_cap = 0;
-        HX_CUDA_TRY(cudaMalloc(&c->trace_buf, cap * c->slab * sizeof(double2)));
-        HX_CUDA_TRY(cudaMalloc(&c->energy_buf, cap * 3 * sizeof(double)));
+        if (!whole) {
+            HX_CUDA_TRY(cudaMalloc(&c->trace_buf, cap * c->slab * sizeof(double2)));
+            HX_CUDA_TRY(cudaMalloc(&c->energy_buf, cap * 3 * sizeof(double)));
+        }
         c->pinned_bytes = cap * (c->slab * sizeof(double2) + 3 * sizeof(double));
         HX_CUDA_TRY(cudaMallocHost(&c->pinned, c->pinned_bytes));
         c->trace_cap = cap;
@@ -1199,26 +1242,33 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
     uint64_t done = 0;
     while (done < nsteps) {
         const int chunk = static_cast<int>(std::min<uint64_t>(nsteps - done, c->trace_cap));
-        for (int t = 0; t < chunk; ++t) {
+        if (whole) {
+            // the run writes its records straight into the pinned staging
+            enqueue_run(c, chunk, rho0_trace ? reinterpret_cast<double2*>(pin_rho) : nullptr,
+                        energy_trace ? pin_en : nullptr);
+            c->counters.d2h_bytes += chunk * ((rho0_trace ? c->slab * sizeof(double2) : 0) +
+                                              (energy_trace ? 3 * sizeof(double) : 0));
+        }
+        for (int t = 0; !whole && t < chunk; ++t) {
             enqueue_step(c);
-            launch_obs(c, c->energy_buf + 3 * t);
+            const int rc = launch_obs(c, c->energy_buf + 3 * t,
+                                      rho0_trace ? c->trace_buf + static_cast<size_t>(t) * c->slab_store : nullptr);
+            if (rc != HX_OK) return rc;
             c->counters.kernel_launches += 1;
-            if (rho0_trace)
-                HX_CUDA_TRY(cudaMemcpyAsync(c->trace_buf + static_cast<size_t>(t) * c->slab_store, c->rho,
-                                            c->slab_store * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
         }
         int rc = check_launch("trace step");
         if (rc != HX_OK) return rc;
-        if (rho0_trace) {
+        if (rho0_trace && !whole) {
             HX_CUDA_TRY(cudaMemcpyAsync(pin_rho, c->trace_buf, chunk * c->slab_store * sizeof(double2),
                                         cudaMemcpyDeviceToHost, c->stream));
             c->counters.d2h_bytes += chunk * c->slab_store * sizeof(double2);
         }
-        if (energy_trace) {
+        if (energy_trace && !whole) {
             HX_CUDA_TRY(cudaMemcpyAsync(pin_en, c->energy_buf, chunk * 3 * sizeof(double), cudaMemcpyDeviceToHost,
                                         c->stream));
             c->counters.d2h_bytes += chunk * 3 * sizeof(double);
         }
+        if ((rc = enqueue_flag(c)) != HX_OK) return rc;
         HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
         if (rho0_trace && c->herm) {
             for (int t = 0; t < chunk; ++t)
@@ -1230,6 +1280,7 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
         if (energy_trace)
             for (int t = 0; t < chunk; ++t) energy_trace[done + t] = pin_en[3 * t];
         done += chunk;
+        if (done == nsteps) return flag_status(c);
     }
     return read_error_flag(c);
 }
@@ -1239,11 +1290,9 @@ int hx_ctx_read_rho0(hx_ctx* c, double* out, uint64_t n)
     if (!c || !out) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL argument");
     if (n < 2 * c->slab) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "output buffer too small");
     if (c->herm) {
-        const int rc = read_herm(c, c->rho, 1, out);
-        return rc != HX_OK ? rc : read_error_flag(c);
+        return read_herm(c, c->rho, 1, out);
     }
     HX_CUDA_TRY(cudaMemcpyAsync(out, c->rho, c->slab * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-    HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->counters.d2h_bytes += c->slab * sizeof(double2);
     return read_error_flag(c);
 }
@@ -1251,17 +1300,17 @@ int hx_ctx_read_rho0(hx_ctx* c, double* out, uint64_t n)
 int hx_ctx_observables(hx_ctx* c, double* energy, double* trace_re, double* trace_im)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    launch_obs(c, c->obs);
+    if (const int rc = launch_obs(c, c->obs)) return rc;
     c->counters.kernel_launches += 1;
     int rc = check_launch("observables kernel");
     if (rc != HX_OK) return rc;
     double h[3];
     HX_CUDA_TRY(cudaMemcpyAsync(h, c->obs, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-    HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
+    if ((rc = read_error_flag(c)) != HX_OK) return rc;
     if (energy) *energy = h[0];
     if (trace_re) *trace_re = h[1];
     if (trace_im) *trace_im = h[2];
-    return read_error_flag(c);
+    return HX_OK;
 }
 
 int hx_ctx_read_state(hx_ctx* c, double* out, uint64_t n)
@@ -1274,11 +1323,9 @@ int hx_ctx_read_state(hx_ctx* c, double* out, uint64_t n)
         return rc != HX_OK ? rc : read_error_flag(c);
     }
     if (c->herm) {
-        const int rc = read_herm(c, c->rho, static_cast<size_t>(c->H), out);
-        return rc != HX_OK ? rc : read_error_flag(c);
+        return read_herm(c, c->rho, static_cast<size_t>(c->H), out);
     }
     HX_CUDA_TRY(cudaMemcpyAsync(out, c->rho, count * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
-    HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
     c->counters.d2h_bytes += count * sizeof(double2);
     return read_error_flag(c);
 }
@@ -1558,7 +1605,7 @@ int hx_ctx_state_device_ptr(hx_ctx* c, void** ptr)
 int hx_ctx_inject_wait_timeout(hx_ctx* c)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    if (!c->use_small_step || c->closure)
+    if (!runs_whole_steps(c) || !c->use_small)
         return fail(HX_ERR_UNSUPPORTED_EXECUTION, "no grid-barrier waits in this context's steps");
     c->stall_next_step = true;
     return HX_OK;
@@ -1591,8 +1638,7 @@ int hx_ctx_rhs(hx_ctx* c, double* out, uint64_t n)
         return rc != HX_OK ? rc : read_error_flag(c);
     }
     if (c->herm) {
-        rc = read_herm(c, c->ua, static_cast<size_t>(c->H), out);
-        return rc != HX_OK ? rc : read_error_flag(c);
+        return read_herm(c, c->ua, static_cast<size_t>(c->H), out);
     }
     HX_CUDA_TRY(cudaMemcpyAsync(out, c->ua, count * sizeof(double2), cudaMemcpyDeviceToHost, c->stream));
     HX_CUDA_TRY(cudaStreamSynchronize(c->stream));

@@ -190,19 +190,23 @@ void launch_transpose_bf16(const void* in, int rows, int cols, int ld_in, void* 
 // d <= 16, full slabs, sigma_z couplings, every up term in the entry lists: batched gathers (hx_small.cu)
 size_t small_smem(int logd, int M);
 bool small_supported(int logd, int M, int pauli);
-// The same, one cooperative launch per integrator step (order >= 2), stages separated by grid barriers on
-// an arrival counter (*gcount, zeroed by the caller once; every launch leaves it at zero).  Returns 1 when
-// launched (with dry: when it would launch), 0 when the ADOs do not fit the resident CTAs (up to 4 per
-// CTA), -1 when refused.
-size_t small_step_smem(int logd, int M, int per);
-// Grid-barrier waits of small_step_kernel: polls before giving up (and setting the error word), and an
+// Grid-barrier waits of small_run_kernel: polls before giving up (and setting the error word), and an
 // offset added to every barrier's arrival target (nonzero only to make the waits run out on purpose).
 struct StepWait {
     unsigned skew = 0;
-    unsigned max_polls = 1u << 24;
+    unsigned max_polls = 1u << 22;
 };
-int launch_small_step(const FusedArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order,
-                      unsigned* gcount, cudaStream_t s, bool dry, StepWait w = StepWait{});
+// nsteps whole integrator steps of a small-slab hierarchy (d <= 16, diagonal couplings, order >= 2) in one
+// launch: in one CTA when the hierarchy is tiny, else cooperatively with the stages separated by grid
+// barriers on an arrival counter (*gcount, zeroed by the caller once; every launch leaves it at zero).
+// trace (nsteps x d*d) and obs (nsteps x 3: energy, trace), device or pinned host memory, receive rho_0 and
+// its observables after every step; either may be nullptr.  Returns 1 when launched (with dry, called once
+// at creation: when it would launch), 0 when the hierarchy does not fit the resident CTAs, -1 when refused.
+int launch_small_run(const FusedArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
+                     unsigned* gcount, int sms, cudaStream_t s, bool dry, double2* trace, double* obs,
+                     StepWait w = StepWait{});
+// order[k] = the ADO with the k-th most neighbour entries (FusedArgs::order of launch_small_run).
+void launch_run_order(const int* ent_count, long long H, int32_t* order, cudaStream_t s);
 bool launch_small(const FusedArgs& a, const double2* u, const double2* rho, double2* out, double alpha,
                   int base_kind, cudaStream_t s);
 bool prepare_fused(int logd, int M, int J, int herm);  // raises the shared-memory limit; call before stream capture
@@ -417,8 +421,8 @@ struct hx_ctx {
     // fused stage-kernel tables (d = 32, 64)
     bool use_fused = false;
     bool use_small = false;       // d <= 16 sigma_z stage kernel (hx_small.cu)
-    bool use_small_step = false;  // ... as one cooperative launch per step (small_step_kernel)
-    unsigned* gbar = nullptr;     // grid-barrier arrival counter of small_step_kernel
+    bool use_small_step = false;  // d <= 16: whole steps in one launch (small_run_kernel)
+    unsigned* gbar = nullptr;     // grid-barrier arrival counter of small_run_kernel
     bool stall_next_step = false; // hx_ctx_inject_wait_timeout: the next step's barriers cannot complete
     int sm_count = 0;
     int up_slots = 0;             // ADOs in tier L-1
@@ -443,6 +447,7 @@ struct hx_ctx {
     double* energy_buf = nullptr;
     int trace_cap = 0;
     double* pinned = nullptr;     // pinned staging for traces
+    int* flag_pin = nullptr;      // pinned copy of the error word
     size_t pinned_bytes = 0;
     double2* state_pinned = nullptr; // pinned staging for packed whole-state transfers
     double* pack_scale = nullptr;    // [H] per-slab scale of the device-side packer (first use)

@@ -131,3 +131,40 @@ def test_step_kernel_wait_timeout_is_reported_and_the_context_recovers(monkeypat
         with pytest.raises(capi.HxError) as e:
             plain.inject_wait_timeout()
         assert e.value.status == "UnsupportedExecution"
+
+
+@pytest.mark.parametrize("collective", [False, True])
+@pytest.mark.parametrize("n,baths,K,depth", [
+    (1, 1, 1, 3),   # 10 ADOs at d = 2: one CTA
+    (3, 2, 1, 2),   # 15 ADOs, 960 elements: one CTA
+    (3, 1, 1, 4),   # 15 ADOs with one bath
+    (3, 3, 0, 3),   # 20 ADOs, 1280 elements: the smallest grids, 4 ADOs per CTA
+    (4, 3, 1, 4),   # 210 ADOs at d = 16: two slabs per CTA
+    (4, 2, 3, 4),   # 495 ADOs, up to 16 entries each
+    (4, 4, 3, 3),   # 969 ADOs: several slabs per CTA one after the other, all entries staged
+    (4, 4, 6, 2),   # 28 modes, 435 ADOs: more entries than the staging area holds at once
+])
+def test_whole_step_runs_match_oracle(n, baths, K, depth, collective):
+    """Whole steps in one launch, sigma_z and general diagonal couplings, with
+    and without records: the trajectory against the oracle, and the recorded
+    run equal to the unrecorded one."""
+    p = S.spin_glass(n, seed=70 + n, depth=depth, K=K, h=0.8, dt=0.01)
+    p.baths = p.baths[:baths]
+    if collective:
+        rng = np.random.default_rng(n)
+        for b in p.baths:
+            b.v_diag = rng.uniform(-0.7, 0.7, p.dim)
+    steps = 4
+    o = O.Oracle(p)
+    rho_ref, en_ref = o.run(steps, trace=True)
+    want = o.state()
+    o.close()
+    with capi.Context(p) as a, capi.Context(p) as b:
+        assert a.get_info().kernels_per_step == 1
+        rho, en = a.step_trace(steps)
+        b.step(steps)
+        b.sync()
+        assert np.array_equal(a.state(), b.state())
+        assert np.max(np.abs(a.state() - want)) <= TOL
+    assert np.max(np.abs(rho - rho_ref)) <= TOL
+    assert np.max(np.abs(en - en_ref)) <= TOL
