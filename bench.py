@@ -242,13 +242,15 @@ def stage_kernels_label(ctx, p, packed: bool, per_stage: int) -> str:
         return "csr_comm_kernel + csr_combine_kernel per stage (general sparse operators)"
     if path == "band":
         return "band kernels per stage" + (" (Hermitian-packed slabs)" if packed else "")
+    if path == "fused" and int(ctx.info.kernels_per_step) == 1:
+        return f"herm_run_kernel<{logd}> (whole steps in one cooperative launch, Hermitian-packed slabs)"
     if path == "fused":
         k = f"herm_kernel<{logd}>" if packed else f"fused_kernel<{logd}>"
         return k + (" + upterm_kernel" if per_stage == 2 else "") + " per stage" + \
             (" (Hermitian-packed slabs)" if packed else "")
     if path == "small":
         if int(ctx.info.kernels_per_step) == 1:
-            return "small_step_kernel per step (d <= 16; the 4 stages in one cooperative launch, grid barriers)"
+            return "small_run_kernel (d <= 16; whole steps in one launch, grid barriers between the stages)"
         return "small_kernel per stage (d <= 16, batched neighbour gathers)"
     return "stage_kernel per stage (generic path)"
 

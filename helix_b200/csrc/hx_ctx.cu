@@ -58,7 +58,7 @@ void release(hx_ctx* c)
                     c->up_slab, c->up_bath, c->U, c->vflip, c->Bbuf, c->rho32, c->ua32, c->ub32,
                     c->U32, c->diag32, c->vdiag32, c->hflip32, c->diag_herm, c->vbit, c->csr_ptr, c->csr_col,
                     c->csr_val, c->pack_scale, c->pack_bad, c->dense_hr, c->dense_hr_lo, c->dense_y,
-                    c->dense_h64, c->dense_z0, c->gbar};
+                    c->dense_h64, c->dense_z0, c->gbar, c->cl_coef, c->cl_slot};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
@@ -287,8 +287,10 @@ int launch_stage_any(hx_ctx* c, const double2* u, const double2* rho, double2* o
 {
     int k = launch_stage_core(c, u, rho, out, alpha, base);
     if (c->closure) {
-        hx::closure_stage(c->closure, c, u, out, alpha, c->stream);
-        k += 1;  // the elementwise closure kernel (the coefficient table is rebuilt only after training)
+        // the coefficients change only after training
+        if (hx::closure_update(c) != HX_OK) c->launch_failed = true;
+        else hx::closure_stage(c, u, out, alpha);
+        k += 1;
     }
     return k;
 }
@@ -322,12 +324,14 @@ int launch_stage_core(hx_ctx* c, const double2* u, const double2* rho, double2* 
     return 1;
 }
 
-// Whole steps of a small-slab hierarchy run in one launch (hx_small.cu).
-bool runs_whole_steps(const hx_ctx* c) { return c->use_small_step && !c->closure; }
-
-// Enqueue nsteps steps of such a hierarchy; trace / obs as in launch_small_run.
+// Enqueue nsteps steps of a hierarchy whose steps run in one launch (use_run); trace / obs as in
+// launch_small_run.
 void enqueue_run(hx_ctx* c, uint64_t nsteps, double2* trace, double* obs)
 {
+    if (c->closure && hx::closure_update(c) != HX_OK) c->launch_failed = true;
+    hx::RunClosure cl;
+    if (c->closure && c->cl_on) cl = hx::RunClosure{c->cl_coef, c->cl_slot};
+    auto* launch = c->herm ? hx::launch_herm_run : hx::launch_small_run;
     constexpr uint64_t kMostSteps = 4096;  // of one launch
     for (uint64_t done = 0; done < nsteps;) {
         const int n = static_cast<int>(std::min(nsteps - done, kMostSteps));
@@ -337,9 +341,8 @@ void enqueue_run(hx_ctx* c, uint64_t nsteps, double2* trace, double* obs)
             w.max_polls = 1u << 12;
             c->stall_next_step = false;
         }
-        if (hx::launch_small_run(hx::fused_args_of(c), c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->sm_count,
-                                 c->stream, false, trace ? trace + done * c->slab : nullptr,
-                                 obs ? obs + 3 * done : nullptr, w) != 1)
+        if (launch(hx::fused_args_of(c), cl, c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->sm_count, c->stream,
+                   false, trace ? trace + done * c->slab_store : nullptr, obs ? obs + 3 * done : nullptr, w) != 1)
             c->launch_failed = true;
         c->counters.kernel_launches += 1;
         c->counters.stage_launches += static_cast<uint64_t>(c->order) * n;
@@ -353,7 +356,7 @@ int enqueue_step(hx_ctx* c)
 {
     const int m = c->order;
     int launched = 0;
-    if (runs_whole_steps(c)) {
+    if (c->use_run) {
         enqueue_run(c, 1, nullptr, nullptr);
         return HX_OK;
     }
@@ -1055,16 +1058,21 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             bool all_pauli = true;
             for (int j = 0; j < J; ++j) all_pauli = all_pauli && (bits[j] = hx::pauli_spin(vd.data() + static_cast<size_t>(j) * d, c->d)) >= 0;
             if (rc == HX_OK && all_pauli && (rc = dev_alloc(c, &c->vbit, J)) == HX_OK) rc = upload(c, c->vbit, bits);
-            // small slabs: every up neighbour in the entry lists (no up-term pass)
             const bool want_small = small_ok && all_pauli;
+            // whole steps in one launch while the hierarchy fits the resident CTAs (d <= 16) and L2 (d = 32, 64)
+            const char* step_env = std::getenv("HX_SMALL_STEP");
+            const bool herm_run = c->herm && fused_ok && c->order >= 2 && !(step_env && step_env[0] == '0') &&
+                                  hx::herm_run_fits(logd, M, J, all_pauli ? 1 : 0, c->H, c->sm_count);
+            // every up neighbour in the entry lists (no up-term pass)
+            const bool all_up = small_ok || herm_run;
             hx::launch_entries(c->rows, c->edges, c->acoef, c->bcoef, c->bath_off, c->H, M, J,
-                               static_cast<int>(p->max_depth) + (small_ok ? 1 : 0), c->ent_count,
+                               static_cast<int>(p->max_depth) + (all_up ? 1 : 0), c->ent_count,
                                c->ent_slab,
                                c->ent_bath, c->ent_wc, c->ent_wa, c->ado_keep, c->stream);
             rc = check_launch("fused-kernel setup");
             // tier L-1 slots: count them first, then size the per-slot tables and U
             int S = 0;
-            if (rc == HX_OK && p->max_depth >= 2 && !small_ok) {
+            if (rc == HX_OK && p->max_depth >= 2 && !all_up) {
                 int32_t *tmp_slab = nullptr, *tmp_bath = nullptr;
                 e = cudaMalloc(&tmp_slab, H * M * sizeof(int32_t));
                 if (e == cudaSuccess) e = cudaMalloc(&tmp_bath, H * M * sizeof(int32_t));
@@ -1100,17 +1108,15 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             c->up_slots = S;
             c->use_fused = (rc == HX_OK) && fused_ok;
             c->use_small = (rc == HX_OK) && want_small;
-            // small slabs: whole steps in one launch when the hierarchy fits the resident CTAs
-            const char* step_env = std::getenv("HX_SMALL_STEP");
-            if (rc == HX_OK && small_ok && c->order >= 2 && !(step_env && step_env[0] == '0') &&
+            if (rc == HX_OK && (herm_run || (small_ok && c->order >= 2 && !(step_env && step_env[0] == '0'))) &&
                 (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
+                auto* launch = herm_run ? hx::launch_herm_run : hx::launch_small_run;
                 e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
                 if (e != cudaSuccess) rc = hx::cuda_fail(e, "grid barrier counter");
                 else
-                    c->use_small_step = hx::launch_small_run(hx::fused_args_of(c), c->rho, c->ua, c->ub, c->dt,
-                                                             c->order, 1, c->gbar, c->sm_count, c->stream, true,
-                                                             nullptr, nullptr) == 1;
-                if (rc == HX_OK && c->use_small_step && (rc = dev_alloc(c, &c->order_perm, H)) == HX_OK)
+                    c->use_run = launch(hx::fused_args_of(c), hx::RunClosure{}, c->rho, c->ua, c->ub, c->dt, c->order, 1,
+                                        c->gbar, c->sm_count, c->stream, true, nullptr, nullptr, hx::StepWait{}) == 1;
+                if (rc == HX_OK && c->use_run && (rc = dev_alloc(c, &c->order_perm, H)) == HX_OK)
                     hx::launch_run_order(c->ent_count, c->H, c->order_perm, c->stream);
             }
             // single-precision copies of the operators for the mixed band kernel
@@ -1181,7 +1187,7 @@ int hx_ctx_info(const hx_ctx* c, hx_info* info)
     int per_stage = (c->use_flip || c->use_csr || (c->use_fused && c->up_slots > 0)) ? 2 : 1;
     if (c->use_large) per_stage = 1 + (c->up_slots > 0 ? 1 : 0) + (c->mixed ? 1 : 0) + (c->dense ? 2 : 0);
     info->kernels_per_step = static_cast<uint32_t>(c->order) * per_stage;
-    if (runs_whole_steps(c)) info->kernels_per_step = 1;
+    if (c->use_run) info->kernels_per_step = 1;
     info->stage_path = c->dense     ? HX_PATH_DENSE
                        : c->use_csr ? HX_PATH_CSR
                        : c->use_flip ? HX_PATH_FLIP
@@ -1202,7 +1208,7 @@ int hx_ctx_counters(const hx_ctx* c, hx_counters* out)
 int hx_ctx_step(hx_ctx* c, uint64_t nsteps)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    if (runs_whole_steps(c)) enqueue_run(c, nsteps, nullptr, nullptr);
+    if (c->use_run) enqueue_run(c, nsteps, nullptr, nullptr);
     else
         for (uint64_t s = 0; s < nsteps; ++s) enqueue_step(c);
     return check_launch("stage kernel launch");
@@ -1220,7 +1226,7 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
     // chunk of steps buffered on the device: at most 256 steps and 64 MB of rho_0 copies
     const uint64_t by_bytes = std::max<uint64_t>(1, (uint64_t(64) << 20) / (c->slab * sizeof(double2)));
     const int cap = static_cast<int>(std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(nsteps, 1), 256), by_bytes));
-    const bool whole = runs_whole_steps(c);
+    const bool whole = c->use_run;
     if (c->trace_cap < cap || (!whole && !c->trace_buf)) {
         if (c->trace_buf) cudaFree(c->trace_buf);
         if (c->energy_buf) cudaFree(c->energy_buf);
@@ -1246,7 +1252,7 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
             // the run writes its records straight into the pinned staging
             enqueue_run(c, chunk, rho0_trace ? reinterpret_cast<double2*>(pin_rho) : nullptr,
                         energy_trace ? pin_en : nullptr);
-            c->counters.d2h_bytes += chunk * ((rho0_trace ? c->slab * sizeof(double2) : 0) +
+            c->counters.d2h_bytes += chunk * ((rho0_trace ? c->slab_store * sizeof(double2) : 0) +
                                               (energy_trace ? 3 * sizeof(double) : 0));
         }
         for (int t = 0; !whole && t < chunk; ++t) {
@@ -1605,7 +1611,7 @@ int hx_ctx_state_device_ptr(hx_ctx* c, void** ptr)
 int hx_ctx_inject_wait_timeout(hx_ctx* c)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    if (!runs_whole_steps(c) || !c->use_small)
+    if (!c->use_run || !c->use_small)
         return fail(HX_ERR_UNSUPPORTED_EXECUTION, "no grid-barrier waits in this context's steps");
     c->stall_next_step = true;
     return HX_OK;
@@ -1656,8 +1662,9 @@ int hx_ctx_set_closure(hx_ctx* c, hx_closure* cl)
         if (!hx::closure_matches_hierarchy(cl, c->d, c->M, c->H))
             return fail(HX_ERR_INVALID_RUNTIME_OPTION, "the closure was made for another hierarchy");
     }
-    c->closure = cl;
-    return HX_OK;
+    const int rc = hx::closure_attach(cl, c);
+    c->closure = rc == HX_OK ? cl : nullptr;
+    return rc;
 }
 
 int hx_ctx_check_finite(hx_ctx* c)

@@ -196,15 +196,27 @@ struct StepWait {
     unsigned skew = 0;
     unsigned max_polls = 1u << 22;
 };
+// A learned closure's term in a run of whole steps: (coef x) added to the right-hand side of every ADO n with
+// slot[n] >= 0, coef = slab slot[n] of the context's closure coefficients (nullptrs: no closure).
+struct RunClosure {
+    const double2* coef = nullptr;  // [top-tier ADOs][stored slab]
+    const int32_t* slot = nullptr;  // [H]
+};
 // nsteps whole integrator steps of a small-slab hierarchy (d <= 16, diagonal couplings, order >= 2) in one
 // launch: in one CTA when the hierarchy is tiny, else cooperatively with the stages separated by grid
 // barriers on an arrival counter (*gcount, zeroed by the caller once; every launch leaves it at zero).
 // trace (nsteps x d*d) and obs (nsteps x 3: energy, trace), device or pinned host memory, receive rho_0 and
 // its observables after every step; either may be nullptr.  Returns 1 when launched (with dry, called once
 // at creation: when it would launch), 0 when the hierarchy does not fit the resident CTAs, -1 when refused.
-int launch_small_run(const FusedArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
+int launch_small_run(const FusedArgs& a, const RunClosure& cl, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
                      unsigned* gcount, int sms, cudaStream_t s, bool dry, double2* trace, double* obs,
                      StepWait w = StepWait{});
+// The same for d = 32, 64 on Hermitian-packed slabs (hx_herm_run.cu); trace holds packed slabs.
+// herm_run_fits: whether a context should run this way (every up neighbour then is in its entry lists).
+bool herm_run_fits(int logd, int M, int J, int pauli, long long H, int sms);
+int launch_herm_run(const FusedArgs& a, const RunClosure& cl, double2* rho, double2* ua, double2* ub, double dt,
+                    int order, int nsteps, unsigned* gcount, int sms, cudaStream_t s, bool dry, double2* trace,
+                    double* obs, StepWait w = StepWait{});
 // order[k] = the ADO with the k-th most neighbour entries (FusedArgs::order of launch_small_run).
 void launch_run_order(const int* ent_count, long long H, int32_t* order, cudaStream_t s);
 bool launch_small(const FusedArgs& a, const double2* u, const double2* rho, double2* out, double alpha,
@@ -300,9 +312,15 @@ void launch_vec_d2f(const double* in, float* out, long long n, cudaStream_t s);
 
 // Whether a closure was made for a hierarchy of this dimension, mode count and size (hx_mlp.cu)
 bool closure_matches_hierarchy(const ::hx_closure* cl, int d, int M, long long H);
-// Learned closure term of a stage: out_top += alpha * (dropped up coupling) (hx_mlp.cu)
-int closure_stage(::hx_closure* cl, const ::hx_ctx* c, const double2* u, double2* out, double alpha,
-                  cudaStream_t s);
+// The closure of a context (hx_mlp.cu).  The dropped up coupling of a top-tier ADO is elementwise and linear
+// in it, so it is one complex coefficient per element of each top-tier ADO, kept per context.
+// closure_attach: room for them and the slot of every ADO (cl = nullptr: give both back).
+int closure_attach(::hx_closure* cl, ::hx_ctx* c);
+// Bring the coefficients up to date with the network (on the context's stream); c->cl_on tells whether
+// there is a term to add.
+int closure_update(::hx_ctx* c);
+// out_top += alpha * coefficient * u_top, after a stage.
+void closure_stage(const ::hx_ctx* c, const double2* u, double2* out, double alpha);
 
 // Argument blocks of a context's fused and up-term kernels (hx_ctx.cu)
 FusedArgs fused_args_of(const ::hx_ctx* c);
@@ -406,6 +424,10 @@ struct hx_ctx {
     bool use_large = false;       // band kernels for 128 <= d <= 1024, diagonal V (hx_large.cu)
     bool mixed = false;           // complex64 hierarchy, ADO 0 in double precision
     hx_closure* closure = nullptr; // learned closure term added by every stage (hx_mlp.cu)
+    double2* cl_coef = nullptr;   // [top-tier ADOs][slab_store] its coefficients, of table build cl_build
+    int32_t* cl_slot = nullptr;   // [H] slab of an ADO in cl_coef, or -1
+    uint64_t cl_build = 0;
+    bool cl_on = false;           // the closure is trained (or has its scales): its term counts
     float2* rho32 = nullptr;      // mixed: complex64 state buffers (rho, ua, ub mirror them)
     float2* ua32 = nullptr;
     float2* ub32 = nullptr;
@@ -421,8 +443,8 @@ struct hx_ctx {
     // fused stage-kernel tables (d = 32, 64)
     bool use_fused = false;
     bool use_small = false;       // d <= 16 sigma_z stage kernel (hx_small.cu)
-    bool use_small_step = false;  // d <= 16: whole steps in one launch (small_run_kernel)
-    unsigned* gbar = nullptr;     // grid-barrier arrival counter of small_run_kernel
+    bool use_run = false;         // whole steps in one launch (small_run_kernel, herm_run_kernel)
+    unsigned* gbar = nullptr;     // their grid-barrier arrival counter
     bool stall_next_step = false; // hx_ctx_inject_wait_timeout: the next step's barriers cannot complete
     int sm_count = 0;
     int up_slots = 0;             // ADOs in tier L-1

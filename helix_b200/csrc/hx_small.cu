@@ -26,6 +26,7 @@
 #include <cstdint>
 
 #include "hx_internal.h"
+#include "hx_run.cuh"
 
 namespace hx {
 
@@ -150,69 +151,6 @@ void launch_small_t(const FusedArgs& a, const double2* u, const double2* rho, do
     small_kernel<LOGD><<<static_cast<unsigned>(a.H), threads, smem, s>>>(a, u, rho, out, alpha, base);
 }
 
-// Grid barrier of small_run_kernel: every CTA is resident (cooperative
-// launch).  One arrival counter, zero when a launch begins: barrier k of the
-// launch waits until it reaches (k + 1) G.  The block's writes are ordered
-// before thread 0's arrival by the block barrier and a GPU-scope fence; the
-// wait polls the counter with acquire loads, bounded.  The launch puts the
-// counter back to zero at its end, so no host-side count is involved (a
-// captured launch replays correctly).
-// Returns false when the wait ran out.
-__device__ __forceinline__ void grid_arrive(unsigned* count)
-{
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(count, 1u);
-    }
-}
-
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, unsigned max_polls)
-{
-    int late = 0;
-    grid_arrive(count);
-    if (threadIdx.x == 0) {
-        for (uint32_t it = 0;; ++it) {
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            if (static_cast<int>(v - target) >= 0) break;
-            if (it >= max_polls) {
-                late = 1;
-                break;
-            }
-        }
-    }
-    return __syncthreads_or(late) == 0;
-}
-
-// Energy and trace of rho_0 by one warp, in the summation order of
-// observables_kernel (hx_stage.cu); at(r, c) returns an element of rho_0.
-template <int LOGD, typename At>
-__device__ __forceinline__ void warp_observables(const FusedArgs& a, At at, double* out)
-{
-    constexpr int D = 1 << LOGD;
-    const int r = threadIdx.x & 31;
-    double en = 0.0, tr = 0.0, ti = 0.0;
-    if (r < D) {
-        const double2 dg = at(r, r);
-        en = fma(__ldg(a.hdiag + r), dg.x, en);
-        tr += dg.x;
-        ti += dg.y;
-#pragma unroll
-        for (int i = 0; i < LOGD; ++i) en = fma(__ldg(a.hflip + i), at(r ^ (1 << i), r).x, en);
-    }
-    for (int off = 16; off > 0; off >>= 1) {
-        en += __shfl_down_sync(0xffffffffu, en, off);
-        tr += __shfl_down_sync(0xffffffffu, tr, off);
-        ti += __shfl_down_sync(0xffffffffu, ti, off);
-    }
-    if (r == 0) {
-        out[0] = en;
-        out[1] = tr;
-        out[2] = ti;
-    }
-}
-
 // Elements of a slab that one thread of small_run_kernel owns, and threads per slab.
 template <int LOGD> struct RunShape {
     static constexpr int E = LOGD == 4 ? 2 : 1;
@@ -256,7 +194,7 @@ constexpr int kRunBatch = 4;  // staged entries read back side by side
 // and the diagonal term comes from the table a.diag.
 template <int LOGD, bool PAULI, bool SOLO>
 __global__ void __launch_bounds__(kRunThreads, 1)
-    small_run_kernel(FusedArgs a, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
+    small_run_kernel(FusedArgs a, RunClosure cl, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
                      int apc, int per, int cap, unsigned* gcount, StepWait w, double2* trace, double* obs)
 {
     constexpr int D = 1 << LOGD, D2 = D * D, E = RunShape<LOGD>::E, TA = RunShape<LOGD>::TA;
@@ -272,7 +210,8 @@ __global__ void __launch_bounds__(kRunThreads, 1)
     int2* sN = reinterpret_cast<int2*>(sV + (PAULI ? 2 * D : a.J * D));  // [NL][2M] neighbour's first element, spin or bath
     int* sQ = reinterpret_cast<int*>(sN + NL * M2);      // [NL]
     int* sA = sQ + NL;                                   // [NL] the ADO of each local slab, or -1
-    int* sO = sA + NL;                                   // [apc] first staging place of each group of TA threads
+    int* sK = sA + NL;                                   // [NL] its slab of closure coefficients, or -1
+    int* sO = sK + NL;                                   // [apc] first staging place of each group of TA threads
     int* sC = sO + apc;                                  // [apc] entries it stages at a time
 
     const int tid = threadIdx.x;
@@ -298,6 +237,7 @@ __global__ void __launch_bounds__(kRunThreads, 1)
             sA[l] = n;
             sQ[l] = n >= 0 ? a.ent_count[n] : 0;
             sG[l] = n >= 0 ? a.gsum[n] : 0.0;
+            sK[l] = n >= 0 && cl.slot ? cl.slot[n] : -1;
         }
         if (PAULI) {
             if (tid < D) {
@@ -406,16 +346,17 @@ __global__ void __launch_bounds__(kRunThreads, 1)
 #pragma unroll
                         for (int k = 0; k < E; ++k)
                             if (need(p, k))
-                                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                                                 mine32 + static_cast<uint32_t>((q - q0) * D2 + TA * k) * 16u),
-                                             "l"(ue + p.x + TA * k)
-                                             : "memory");
+                                cp_async16(mine32 + static_cast<uint32_t>((q - q0) * D2 + TA * k) * 16u, ue + p.x + TA * k);
                     }
                 };
                 if (!SOLO) ask(0);
-                double2 x[E], acc[E];
+                double2 x[E], acc[E], kc[E];
+                const int ks = sK[l];
 #pragma unroll
-                for (int k = 0; k < E; ++k) x[k] = xs[lg + TA * k];
+                for (int k = 0; k < E; ++k) {
+                    x[k] = xs[lg + TA * k];
+                    kc[k] = ks >= 0 ? __ldg(cl.coef + ks * D2 + lg + TA * k) : make_double2(0.0, 0.0);
+                }
 #pragma unroll
                 for (int k = 0; k < E; ++k) {
                     // flips of the rows that this thread owns too are in registers
@@ -428,12 +369,12 @@ __global__ void __launch_bounds__(kRunThreads, 1)
                         hr = fma(sH[b], rp.x - cp.x, hr);
                         hi = fma(sH[b], rp.y - cp.y, hi);
                     }
-                    acc[k] = diag_term(tr0[k] - g, ti[k], x[k], make_double2(hr, hi));
+                    acc[k] = diag_term(tr0[k] - g + kc[k].x, ti[k] + kc[k].y, x[k], make_double2(hr, hi));
                 }
                 for (int q0 = 0; q0 < Q; q0 += C) {
                     if (!SOLO) {
                         if (q0 > 0) ask(q0);
-                        asm volatile("cp.async.wait_all;" ::: "memory");
+                        cp_async_wait();
                     }
                     const int q1 = min(Q, q0 + C);
                     for (int qb = q0; qb < q1; qb += kRunBatch) {
@@ -511,13 +452,7 @@ __global__ void __launch_bounds__(kRunThreads, 1)
         }
         return;
     }
-    // the counter goes back to zero for the next launch: by the watcher, whose last wait saw every arrival,
-    // or by the last CTA to get here once every CTA has passed every barrier
-    if (watch) {
-        if (watcher && tid == 0) atomicExch(gcount, 0u);
-    } else if (tid == 0 && atomicAdd(gcount, 1u) == static_cast<unsigned>(nsteps * order) * G - 1u) {
-        atomicExch(gcount, 0u);
-    }
+    grid_reset(gcount, watch, watcher, static_cast<unsigned>(nsteps * order));
 }
 
 // order[k] = the ADO with the k-th most entries (ties by index): ranks by
@@ -553,7 +488,7 @@ size_t run_smem(int logd, int M, int J, bool pauli, int apc, int per)
 {
     const size_t D = size_t(1) << logd, NL = static_cast<size_t>(apc) * per;
     return 3 * NL * D * D * sizeof(double2) + NL * 2 * M * (sizeof(double2) + sizeof(int2)) +
-           sizeof(double) * (NL + logd + (pauli ? 2 * D : J * D)) + sizeof(int) * 2 * (NL + apc);
+           sizeof(double) * (NL + logd + (pauli ? 2 * D : J * D)) + sizeof(int) * (3 * NL + 2 * apc);
 }
 
 bool plan_run(int logd, int M, int J, bool pauli, long long H, int sms, bool solo, RunPlan& p)
@@ -589,13 +524,14 @@ bool plan_run(int logd, int M, int J, bool pauli, long long H, int sms, bool sol
 }
 
 template <int LOGD, bool PAULI, bool SOLO>
-int launch_run_t(const RunPlan& p, const FusedArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order,
+int launch_run_t(const RunPlan& p, const FusedArgs& a, const RunClosure& cl, double2* rho, double2* ua, double2* ub, double dt, int order,
                  int nsteps, unsigned* gcount, StepWait w, double2* trace, double* obs, cudaStream_t s)
 {
     auto* kernel = small_run_kernel<LOGD, PAULI, SOLO>;
     FusedArgs args = a;
+    RunClosure clo = cl;
     int apc = p.apc, per = p.per, cap = p.cap;
-    void* params[] = {&args, &rho, &ua, &ub, &dt, &order, &nsteps, &apc, &per, &cap, &gcount, &w, &trace, &obs};
+    void* params[] = {&args, &clo, &rho, &ua, &ub, &dt, &order, &nsteps, &apc, &per, &cap, &gcount, &w, &trace, &obs};
     const dim3 grid(static_cast<unsigned>(p.grid + (!SOLO && (trace || obs) ? 1 : 0))), block(static_cast<unsigned>(p.threads));
     const cudaError_t e = SOLO ? cudaLaunchKernel(reinterpret_cast<void*>(kernel), grid, block, params, p.smem, s)
                                : cudaLaunchCooperativeKernel(reinterpret_cast<void*>(kernel), grid, block, params, p.smem, s);
@@ -603,7 +539,7 @@ int launch_run_t(const RunPlan& p, const FusedArgs& a, double2* rho, double2* ua
 }
 
 template <int LOGD>
-int launch_run_d(const RunPlan& p, const FusedArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order,
+int launch_run_d(const RunPlan& p, const FusedArgs& a, const RunClosure& cl, double2* rho, double2* ua, double2* ub, double dt, int order,
                  int nsteps, unsigned* gcount, StepWait w, double2* trace, double* obs, cudaStream_t s, bool dry)
 {
     if (dry) {  // creation: raise the shared-memory limits (function attributes, not to be set in a capture)
@@ -623,10 +559,10 @@ int launch_run_d(const RunPlan& p, const FusedArgs& a, double2* rho, double2* ua
         return ok ? 1 : -1;
     }
     if (a.pauli)
-        return p.solo ? launch_run_t<LOGD, true, true>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s)
-                      : launch_run_t<LOGD, true, false>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s);
-    return p.solo ? launch_run_t<LOGD, false, true>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s)
-                  : launch_run_t<LOGD, false, false>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s);
+        return p.solo ? launch_run_t<LOGD, true, true>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s)
+                      : launch_run_t<LOGD, true, false>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s);
+    return p.solo ? launch_run_t<LOGD, false, true>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s)
+                  : launch_run_t<LOGD, false, false>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s);
 }
 
 }  // namespace
@@ -639,7 +575,7 @@ size_t small_smem(int logd, int M)
 
 bool small_supported(int logd, int M, int pauli) { return pauli && logd >= 1 && logd <= 4 && small_smem(logd, M) <= 48 * 1024; }
 
-int launch_small_run(const FusedArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
+int launch_small_run(const FusedArgs& a, const RunClosure& cl, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
                      unsigned* gcount, int sms, cudaStream_t s, bool dry, double2* trace, double* obs, StepWait w)
 {
     RunPlan p;
@@ -647,10 +583,10 @@ int launch_small_run(const FusedArgs& a, double2* rho, double2* ua, double2* ub,
     // a wait that is to run out needs the grid barriers
     if (!plan_run(a.logd, a.M, a.J, a.pauli != 0, a.H, sms, w.skew == 0, p)) return 0;
     switch (a.logd) {
-    case 1: return launch_run_d<1>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
-    case 2: return launch_run_d<2>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
-    case 3: return launch_run_d<3>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
-    case 4: return launch_run_d<4>(p, a, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
+    case 1: return launch_run_d<1>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
+    case 2: return launch_run_d<2>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
+    case 3: return launch_run_d<3>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
+    case 4: return launch_run_d<4>(p, a, cl, rho, ua, ub, dt, order, nsteps, gcount, w, trace, obs, s, dry);
     default: return 0;
     }
 }

@@ -168,3 +168,42 @@ def test_whole_step_runs_match_oracle(n, baths, K, depth, collective):
         assert np.max(np.abs(a.state() - want)) <= TOL
     assert np.max(np.abs(rho - rho_ref)) <= TOL
     assert np.max(np.abs(en - en_ref)) <= TOL
+
+
+@pytest.mark.parametrize("n,baths,K,depth,order,collective", [
+    (5, 1, 0, 1, 4, False),   # 2 ADOs
+    (5, 5, 2, 2, 4, False),   # 136 ADOs: one per SM, kept in registers
+    (5, 4, 3, 2, 3, True),    # 153 ADOs: just more than one per SM
+    (5, 5, 1, 3, 2, False),   # 286 ADOs
+    (5, 3, 3, 3, 4, True),    # 455 ADOs, general diagonal couplings
+    (6, 6, 0, 1, 4, False),   # 7 ADOs at d = 64
+    (6, 4, 2, 2, 4, True),    # 91 ADOs
+    (6, 5, 2, 2, 4, False),   # 136 ADOs
+    (6, 6, 2, 2, 2, False),   # 190 ADOs: two per CTA
+])
+def test_packed_whole_step_runs_match_oracle(n, baths, K, depth, order, collective):
+    """Whole steps in one launch on Hermitian-packed slabs (d = 32, 64): the
+    trajectory against the oracle, the recorded run equal to the unrecorded
+    one, and to one step at a time."""
+    p = S.spin_glass(n, seed=90 + n, depth=depth, K=K, h=0.8, dt=0.005)
+    p.baths = p.baths[:baths]
+    if collective:
+        rng = np.random.default_rng(n)
+        for b in p.baths:
+            b.v_diag = rng.uniform(-0.7, 0.7, p.dim)
+    steps = 3
+    o = O.Oracle(p)
+    rho_ref, en_ref = o.run(steps, order=order, trace=True)
+    want = o.state()
+    o.close()
+    with capi.Context(p, order=order) as a, capi.Context(p, order=order) as b:
+        assert a.hermitian_packed and a.get_info().kernels_per_step == 1
+        rho, en = a.step_trace(steps)
+        for _ in range(steps):
+            b.step(1)
+        b.sync()
+        assert np.array_equal(a.state(), b.state())
+        assert np.max(np.abs(a.state() - want)) <= TOL
+        assert abs(a.observables()[0] - en[-1]) == 0.0
+    assert np.max(np.abs(rho - rho_ref)) <= TOL
+    assert np.max(np.abs(en - en_ref)) <= TOL
