@@ -58,7 +58,7 @@ void release(hx_ctx* c)
                     c->up_slab, c->up_bath, c->U, c->vflip, c->Bbuf, c->rho32, c->ua32, c->ub32,
                     c->U32, c->diag32, c->vdiag32, c->hflip32, c->diag_herm, c->vbit, c->csr_ptr, c->csr_col,
                     c->csr_val, c->pack_scale, c->pack_bad, c->dense_hr, c->dense_hr_lo, c->dense_y,
-                    c->dense_h64, c->dense_z0, c->gbar, c->cl_coef, c->cl_slot};
+                    c->dense_h64, c->dense_z0, c->gbar, c->cl_coef, c->cl_slot, c->xsum};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
@@ -185,6 +185,10 @@ hx::LargeArgs<double> large_args64(const hx_ctx* c)
     a.logd = c->logd;
     a.first_ado = 0;
     a.herm = c->herm ? 1 : 0;
+    a.pauli = c->vbit ? 1 : 0;
+    a.vbit = c->vbit;
+    a.hdiag = c->hdiag;
+    a.xsum = c->xsum;
     return a;
 }
 
@@ -209,6 +213,10 @@ hx::LargeArgs<float> large_args32(const hx_ctx* c)
     a.logd = c->logd;
     a.first_ado = 1;
     a.herm = c->herm ? 1 : 0;
+    a.pauli = c->vbit ? 1 : 0;
+    a.vbit = c->vbit;
+    a.hdiag = c->hdiag;
+    a.xsum = c->xsum;
     a.dense_y = c->dense ? c->dense_y : nullptr;
     return a;
 }
@@ -1058,6 +1066,13 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             bool all_pauli = true;
             for (int j = 0; j < J; ++j) all_pauli = all_pauli && (bits[j] = hx::pauli_spin(vd.data() + static_cast<size_t>(j) * d, c->d)) >= 0;
             if (rc == HX_OK && all_pauli && (rc = dev_alloc(c, &c->vbit, J)) == HX_OK) rc = upload(c, c->vbit, bits);
+            if (rc == HX_OK && all_pauli && c->use_large && (rc = dev_alloc(c, &c->xsum, d)) == HX_OK) {
+                std::vector<double> xs(d, 0.0);
+                for (uint32_t r = 0; r < d; ++r)
+                    for (int j = 0; j < J; ++j)
+                        if ((r >> bits[j]) & 1) xs[r] -= 4.0 * xi[j];
+                rc = upload(c, c->xsum, xs);
+            }
             const bool want_small = small_ok && all_pauli;
             // whole steps in one launch while the hierarchy fits the resident CTAs (d <= 16) and L2 (d = 32, 64)
             const char* step_env = std::getenv("HX_SMALL_STEP");

@@ -270,7 +270,11 @@ struct LargeArgs {
     long long H;
     int M, J, logd;
     int first_ado;           // 1 when ADO 0 runs in double precision (ado0_kernel)
-    int herm;                // 1: slabs, diag and U Hermitian-packed (herm_band_kernel)
+    int herm;                // 1: slabs, diag and U Hermitian-packed (herm_tile_kernel)
+    int pauli;               // 1: every coupling is the sigma_z of one spin, vbit[j]; then diagonal term =
+    const int* vbit;         // [J]  (xsum[r ^ c] + i (hdiag[c] - hdiag[r])) u
+    const double* hdiag;     // [d]
+    const double* xsum;      // [d] -4 sum_j xi_j over the j whose spin's bit is set
     // dense H on the tensor cores (HX_FLAG_DENSE_H, full slabs): Y_n = X_n H_off for every ADO (H_off: H
     // without its diagonal), in the state layout; X_n is Hermitian, so H_off X_n = Y_n^dagger and
     // -i[H_off, X_n]_rc = -i(conj(Y_cr) - Y_rc)
@@ -456,6 +460,7 @@ struct hx_ctx {
     double2* U = nullptr;         // [S][d*d]
     double2* diag_table = nullptr;
     double2* diag_herm = nullptr; // packed diagonal table (herm)
+    double* xsum = nullptr;       // [d] -4 sum_j xi_j over the j whose spin's bit is set (vbit != nullptr)
     int* vbit = nullptr;          // [J] sigma_z spin of each coupling operator, when every one is a sigma_z
     int* ent_count = nullptr;
     int32_t* ent_slab = nullptr;

@@ -267,167 +267,271 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 }
 
 // ---------------------------------------------------------------------------
-// Band kernel on Hermitian-packed slabs (layout in hx_internal.h).  A band is
-// G = 2048 / d packed rows: matrix rows s0 .. s0+G-1 and their mirror rows
-// d-1-s0-G+1 .. d-1-s0, so 2G full rows (4096 elements, as a full-slab band)
-// and G (d+1) packed outputs.  The CTA rebuilds those 2G rows in shared
-// memory: the upper parts from the band's own packed rows, the lower parts as
-// conjugates gathered from the other packed rows through L2.  Column flips
-// and the row flips of the low log2 G bits then read shared memory (mirror
-// rows flip with the same local index); flips of higher row bits read the
-// packed slab through L2.  Neighbours, the Horner base, U and the output
-// stream in packed order.  No device-side waits.
-// Threads per band: complex64 bands hide their L2 gathers with 512 threads
-// (5 elements each); double-precision ones need more registers: 384 (6 each).
-template <typename R> struct BandThreads { static constexpr int T = 384; };
-template <> struct BandThreads<float> { static constexpr int T = 512; };
+// Tile kernel on Hermitian-packed slabs (layout in hx_internal.h).  A CTA
+// computes one 64 x 64 tile (I, J), I <= J, of one ADO.  What bounds a stage
+// is the traffic between L2 and the SMs (64 bytes a cycle each): per element
+// its own value, the flip partners outside the tile, the neighbours, the base
+// and the result.  A square tile keeps the six low bits of row and column
+// inside, so 2 (log2 d - 6) partners come through L2 where bands of whole rows
+// needed log2 d - log2(2048 / d) and the scattered lower halves of the rows:
+//
+//  * the lanes of a warp are 4 rows x 8 columns, so a partner tile is read in
+//    pieces of 128 bytes directly and of 64 bytes where it lies below the
+//    diagonal (conjugates of the transposed tile): no load is scattered;
+//  * a thread owns 8 elements of one column, 8 rows apart, in NP passes: the
+//    flips of the rows of a pass are in registers, the other flips inside the
+//    tile in shared memory (element (r, c) at r 64 + (c ^ (r & 7)): free of
+//    bank conflicts for the mirrored writes of a diagonal tile too);
+//  * with sigma_z couplings the weights come from index bits and the diagonal
+//    term from two d-entry tables instead of a third slab-sized stream;
+//  * diagonal tiles compute their upper triangle only.
+//
+// MEASURED_TILE
+template <typename R, int LOGD> struct TileShape;
+template <int LOGD> struct TileShape<double, LOGD> { static constexpr int NP = 2, MINB = 2, LR = LOGD == 7 ? 1 : 4; };
+template <int LOGD> struct TileShape<float, LOGD> { static constexpr int NP = 1, MINB = 2, LR = 2; };
+constexpr int kTileT = 512;
 
-template <typename R, int LOGD>
-__global__ void __launch_bounds__(BandThreads<R>::T, 2)
-    herm_band_kernel(LargeArgs<R> a, const C2<R>* __restrict__ u, const C2<R>* rho, C2<R>* out, double alpha_d,
+// Element (r, c), r <= c, of a packed slab is at packed_row(r) + c.
+template <int LOGD>
+__device__ __forceinline__ int packed_row(int r)
+{
+    constexpr int D = 1 << LOGD;
+    return r < D / 2 ? r * D : (D - 1 - r) * (D + 1) + 1;
+}
+
+// acc += (weight at the k-th row) y for one neighbour entry with a sigma_z
+// coupling.  Where the spin's bits of row and column agree only -{V, y} wa
+// counts, else only -i [V, y] wc (twice the weights are given).  T: the bit of
+// k that the spin's row bit is, or -1 when all the rows of the pass share it.
+template <typename R, int E, int T>
+__device__ __forceinline__ void tile_entry(C2<R>* acc, const C2<R>* src, int step, const bool* on, int k0, int br0,
+                                           int bc, R wc, R wa)
+{
+    C2<R> y[E];
+    const bool same0 = br0 == bc;  // at rows whose bit is br0
+    const R wr0 = same0 ? (br0 ? -wa : wa) : R(0), wi0 = same0 ? R(0) : (br0 ? -wc : wc);
+    const R wr1 = same0 ? R(0) : (br0 ? wa : -wa), wi1 = same0 ? (br0 ? wc : -wc) : R(0);  // at the others
+    const bool need0 = wr0 != R(0) || wi0 != R(0), need1 = wr1 != R(0) || wi1 != R(0);
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const bool other = T >= 0 && ((k >> (T < 0 ? 0 : T)) & 1);
+        y[k] = mk<R>(0, 0);
+        if (on[k] && (other ? need1 : need0)) y[k] = __ldg(src + k * step);
+    }
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        const bool other = T >= 0 && ((k >> (T < 0 ? 0 : T)) & 1);
+        const R wr = other ? wr1 : wr0, wi = other ? wi1 : wi0;
+        acc[k].x += wr * y[k].x - wi * y[k].y;
+        acc[k].y += wr * y[k].y + wi * y[k].x;
+    }
+}
+
+template <typename R, int LOGD, bool PAULI>
+__global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
+    herm_tile_kernel(LargeArgs<R> a, const C2<R>* __restrict__ u, const C2<R>* rho, C2<R>* out, double alpha_d,
                      int base_kind)
 {
     using C = C2<R>;
-    constexpr int D = 1 << LOGD, T = BandThreads<R>::T, G = 2048 / D, LOGG = 11 - LOGD;
-    constexpr int NE = G * (D + 1);  // packed elements of a band
-    constexpr int E = (NE + T - 1) / T;
+    constexpr int D = 1 << LOGD, NP = TileShape<R, LOGD>::NP, E = 8 / NP, NBK = D / 64, NT = NBK * (NBK + 1) / 2;
+    constexpr int LR = TileShape<R, LOGD>::LR, LC = 32 / LR;  // rows and columns of a warp's lanes
     constexpr long long P = static_cast<long long>(D / 2) * (D + 1);
-    constexpr int NB = (D / 2) / G;  // bands per slab
     extern __shared__ __align__(128) unsigned char smem[];
-    C* sx = reinterpret_cast<C*>(smem);                                   // [2G][D] rebuilt rows
-    double* sWc = reinterpret_cast<double*>(smem + 2 * G * D * sizeof(C));  // [2M]
-    double* sWa = sWc + 2 * a.M;                                          // [2M]
-    R* sV = reinterpret_cast<R*>(sWa + 2 * a.M);                          // [J][D]
-    R* sH = sV + a.J * D;                                                 // [LOGD]
-    int* sSlab = reinterpret_cast<int*>(sH + LOGD + 1);                   // [2M]
-    int* sBath = sSlab + 2 * a.M;                                         // [2M]
+    C* sx = reinterpret_cast<C*>(smem);                                // [64][64] the tile
+    double* sE = reinterpret_cast<double*>(smem + 4096 * sizeof(C));   // [D] E_r (PAULI)
+    R* sX = reinterpret_cast<R*>(sE + (PAULI ? D : 0));                // [D] -4 sum of xi over differing bits (PAULI)
+    R* sV = sX + (PAULI ? D : 0);                                      // [J][D] (general couplings)
+    R* sH = sV + (PAULI ? 0 : a.J * D);                                // [LOGD]
+    R* sWc = sH + LOGD;                                                // [2M] (twice the weights with PAULI)
+    R* sWa = sWc + 2 * a.M;                                            // [2M]
+    int* sSlab = reinterpret_cast<int*>(sWa + 2 * a.M);                // [2M]
+    int* sBit = sSlab + 2 * a.M;                                       // [2M] spin (PAULI) or bath
 
     const int tid = threadIdx.x;
-    const long long n = a.first_ado + static_cast<long long>(blockIdx.x) / NB;
-    const int s0 = static_cast<int>(blockIdx.x % NB) * G;
-    const int q0 = s0 * (D + 1);  // the band's first packed element
+    const long long n = a.first_ado + static_cast<long long>(blockIdx.x) / NT;
+    int J = 0, I = static_cast<int>(blockIdx.x % NT);
+    while (I > J) I -= ++J;  // tile (I, J) of the upper triangle, column by column
     const C* un = u + n * P;
-    const int Q = a.ent_count[n];
-    for (int i = tid; i < a.J * D; i += T) sV[i] = a.vdiag[i];
-    if (tid < LOGD) sH[tid] = a.hflip[tid];
-    for (int q = tid; q < Q; q += T) {
-        const long long src = n * 2 * a.M + q;
-        sSlab[q] = a.ent_slab[src];
-        sBath[q] = a.ent_bath[src] & 0xffff;
-        sWc[q] = a.ent_wc[src];
-        sWa[q] = a.ent_wa[src];
+    const int warp = tid >> 5, lane = tid & 31;
+    const int r0 = lane / LC + LR * (warp / (2 * LR));  // rows r0 + 8 k of the tile
+    // the second half of the rows is stored shifted by -r mod 8 elements: shifting the columns of a thread
+    // the other way keeps eight lanes on one 128-byte line
+    const int c = (lane % LC + LC * (warp % (2 * LR)) + (I * 64 < D / 2 ? 0 : r0)) & 63;
+    const bool diag = I == J;
+    const int gc = J * 64 + c, gr0 = I * 64 + r0;
+    const int own = packed_row<LOGD>(gr0) + gc;     // packed position of element k: own + k * step
+    const int step = I * 64 < D / 2 ? 8 * D : -8 * (D + 1);
+
+    // ---- the tile (both triangles of a diagonal one)
+    {
+        C x[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (!diag || r0 + 8 * k <= c) x[k] = __ldg(un + own + k * step);
+        const int Q = a.ent_count[n];
+        for (int q = tid; q < Q; q += kTileT) {
+            const long long src = n * 2 * a.M + q;
+            const int j = a.ent_bath[src] & 0xffff;
+            sSlab[q] = a.ent_slab[src];
+            sBit[q] = PAULI ? a.vbit[j] : j;
+            sWc[q] = static_cast<R>(PAULI ? 2.0 * a.ent_wc[src] : a.ent_wc[src]);
+            sWa[q] = static_cast<R>(PAULI ? 2.0 * a.ent_wa[src] : a.ent_wa[src]);
+        }
+        if (PAULI) {
+            for (int i = tid; i < D; i += kTileT) {
+                sE[i] = a.hdiag[i];
+                sX[i] = static_cast<R>(a.xsum[i]);
+            }
+        } else {
+            for (int i = tid; i < a.J * D; i += kTileT) sV[i] = a.vdiag[i];
+        }
+        if (tid < LOGD) sH[tid] = a.hflip[tid];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int r = r0 + 8 * k;
+            if (diag && r > c) continue;
+            sx[r * 64 + (c ^ (r & 7))] = x[k];
+            if (diag && r < c) sx[c * 64 + (r ^ (c & 7))] = mk<R>(x[k].x, -x[k].y);
+        }
     }
+    const int Q = a.ent_count[n];
     const R g = static_cast<R>(a.gsum[n]);
     const int slot = a.slot ? a.slot[n] : -1;
     const R alpha = static_cast<R>(alpha_d);
-    // local row of matrix row r of the band
-    auto lrow = [&](int r) { return r < D / 2 ? r - s0 : G + (D - 1 - s0 - r); };
-
-    // ---- rebuild the band's 2G rows: upper parts from the band ...
-    int rc[E];
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int i = tid + T * k;
-        int r = 0, c = 0;
-        if (i < NE) {
-            herm_coords(q0 + i, LOGD, r, c);
-            sx[lrow(r) * D + c] = __ldg(un + q0 + i);
-        }
-        rc[k] = (r << 16) | c;
-    }
-    // ... lower parts (c < r) as conjugates of the elements (c, r) of other packed rows
-#pragma unroll 4
-    for (int t = tid; t < G * (D - 1); t += T) {
-        const int j = t / (D - 1), w = t - j * (D - 1);
-        const int ra = s0 + j;
-        int lr, r, c;
-        if (w < ra) {
-            lr = j;
-            r = ra;
-            c = w;
-        } else {
-            lr = G + j;
-            r = D - 1 - s0 - j;
-            c = w - ra;
-        }
-        const C v = __ldg(un + herm_index(c, r, LOGD));
-        sx[lr * D + c] = mk<R>(v.x, -v.y);
-    }
     __syncthreads();
 
-    // ---- diagonal table and transverse field
-    C acc[E];
+#pragma unroll 1
+    for (int k0 = 0; k0 < 8; k0 += E) {
+        if (diag && !__any_sync(0xffffffffu, r0 + 8 * k0 <= c)) break;  // the warp's rows are below its columns
+        C acc[E];
+        bool on[E];
+        const C* sp = sx + (r0 + 8 * k0) * 64;  // the pass's first row; + 512 per k
+        const int cs = c ^ (r0 & 7);
+        {
+            C x[E];
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int i = tid + T * k;
-        acc[k] = mk<R>(0, 0);
-        if (i >= NE) continue;
-        const int r = rc[k] >> 16, c = rc[k] & 0xffff, lr = lrow(r);
-        const C x = sx[lr * D + c];
-        const C t = __ldg(a.diag + q0 + i);
-        R hr = 0, hi = 0;
+            for (int k = 0; k < E; ++k) {
+                on[k] = !diag || r0 + 8 * (k0 + k) <= c;
+                x[k] = sp[cs + 512 * k];
+            }
+            // ---- diagonal term
 #pragma unroll
-        for (int b = 0; b < LOGD; ++b) {
-            C rowp;
-            if (b < LOGG) rowp = sx[(lr ^ (1 << b)) * D + c];
-            else rowp = packed_at(un, r ^ (1 << b), c, LOGD);
-            const C colp = sx[lr * D + (c ^ (1 << b))];
-            hr += sH[b] * (rowp.x - colp.x);
-            hi += sH[b] * (rowp.y - colp.y);
+            for (int k = 0; k < E; ++k) {
+                const int r = gr0 + 8 * (k0 + k);
+                R tr, ti;
+                if (PAULI) {
+                    tr = sX[r ^ gc];
+                    ti = static_cast<R>(sE[gc] - sE[r]);
+                } else {
+                    const C t = on[k] ? __ldg(a.diag + own + (k0 + k) * step) : mk<R>(0, 0);
+                    tr = t.x;
+                    ti = t.y;
+                }
+                tr -= g;
+                acc[k].x = tr * x[k].x - ti * x[k].y;
+                acc[k].y = tr * x[k].y + ti * x[k].x;
+            }
+            // ---- flips inside the tile: acc -= i h (row partner - column partner)
+#pragma unroll
+            for (int b = 0; b < 6; ++b) {
+                const R h = sH[b];
+                const C* rp = sx + (((r0 + 8 * k0) ^ (1 << b)) * 64);  // row partners not in registers (no bit of k)
+                const int rs = cs ^ (b < 3 ? (1 << b) : 0);
+#pragma unroll
+                for (int k = 0; k < E; ++k) {
+                    C rowp;
+                    if (b >= 3 && (1 << (b - 3)) < E) rowp = x[k ^ (1 << (b - 3))];
+                    else rowp = rp[rs + 512 * k];
+                    const C colp = sp[(cs ^ (1 << b)) + 512 * k];
+                    acc[k].x += h * (rowp.y - colp.y);
+                    acc[k].y -= h * (rowp.x - colp.x);
+                }
+            }
         }
-        const R tr = t.x - g;
-        acc[k].x = tr * x.x - t.y * x.y + hi;
-        acc[k].y = tr * x.y + t.y * x.x - hr;
-    }
-    // ---- neighbour entries, E loads in flight
-    for (int q = 0; q < Q; ++q) {
-        const int j = sBath[q];
-        const R wc = static_cast<R>(sWc[q]), wa = static_cast<R>(sWa[q]);
-        const C* src = u + static_cast<long long>(sSlab[q]) * P + q0 + tid;
+        // ---- flips of the higher bits: the same place in another tile, through L2
+#pragma unroll 1
+        for (int f = 0; f < 2 * (LOGD - 6); ++f) {
+            const int m = 1 << (f >> 1);
+            const R h = sH[6 + (f >> 1)];
+            const int A = f & 1 ? I : I ^ m, B = f & 1 ? J ^ m : J;  // the partner's tile
+            const R w = f & 1 ? -h : h;
+            C y[E];
+            if (A == B) {
+                const int rb = A * 64 + r0 + 8 * k0, cb = B * 64 + c;
+#pragma unroll
+                for (int k = 0; k < E; ++k) y[k] = on[k] ? packed_at(un, rb + 8 * k, cb, LOGD) : mk<R>(0, 0);
+            } else {
+                // above the diagonal directly, below it the transposed place
+                const int at = A < B ? packed_row<LOGD>(A * 64 + r0) + B * 64 + c : packed_row<LOGD>(B * 64 + c) + A * 64 + r0;
+                const int st = A < B ? (A * 64 < D / 2 ? 8 * D : -8 * (D + 1)) : 8;
+                const C* src = un + at + k0 * st;
+#pragma unroll
+                for (int k = 0; k < E; ++k) y[k] = on[k] ? __ldg(src + k * st) : mk<R>(0, 0);
+            }
+            const R wy = A > B ? -w : w;
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                acc[k].x += wy * y[k].y;
+                acc[k].y -= w * y[k].x;
+            }
+        }
+        // ---- neighbour entries, E loads in flight
+        const C* ub = u + own + k0 * step;
+#pragma unroll 1
+        for (int q = 0; q < Q; ++q) {
+            const C* src = ub + static_cast<long long>(sSlab[q]) * P;
+            const R wc = sWc[q], wa = sWa[q];
+            const int bit = sBit[q];
+            if (PAULI) {
+                const int br0 = ((gr0 + 8 * k0) >> bit) & 1, bc = (gc >> bit) & 1;
+                if (bit == 3 && E > 1) tile_entry<R, E, 0>(acc, src, step, on, k0, br0, bc, wc, wa);
+                else if (bit == 4 && E > 2) tile_entry<R, E, 1>(acc, src, step, on, k0, br0, bc, wc, wa);
+                else if (bit == 5 && E > 4) tile_entry<R, E, 2>(acc, src, step, on, k0, br0, bc, wc, wa);
+                else tile_entry<R, E, -1>(acc, src, step, on, k0, br0, bc, wc, wa);
+            } else {
+                const R* vj = sV + bit * D;
+                const R vc = vj[gc];
+                C y[E];
+#pragma unroll
+                for (int k = 0; k < E; ++k) {
+                    const R vr = vj[gr0 + 8 * (k0 + k)];
+                    y[k] = mk<R>(0, 0);
+                    if (on[k] && ((vr + vc) * wa != R(0) || (vr - vc) * wc != R(0))) y[k] = __ldg(src + k * step);
+                }
+#pragma unroll
+                for (int k = 0; k < E; ++k) {
+                    const R vr = vj[gr0 + 8 * (k0 + k)];
+                    const R ar = -(vr + vc) * wa, ai = -(vr - vc) * wc;
+                    acc[k].x += ar * y[k].x - ai * y[k].y;
+                    acc[k].y += ar * y[k].y + ai * y[k].x;
+                }
+            }
+        }
+        // ---- up term of tier L-1, summed by large_upterm_kernel
         C y[E];
+        if (slot >= 0) {
+            const C* Un = a.U + static_cast<long long>(slot) * P + own + k0 * step;
+#pragma unroll
+            for (int k = 0; k < E; ++k) y[k] = on[k] ? __ldcs(Un + k * step) : mk<R>(0, 0);
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                acc[k].x += y[k].x;
+                acc[k].y += y[k].y;
+            }
+        }
+        // ---- Horner epilogue
+        C* on_ = out + n * P + own + k0 * step;
+        const C* rn = rho + n * P + own + k0 * step;
 #pragma unroll
         for (int k = 0; k < E; ++k) {
-            const int r = rc[k] >> 16, c = rc[k] & 0xffff;
-            const R vr = sV[j * D + r], vc = sV[j * D + c];
             y[k] = mk<R>(0, 0);
-            if (tid + T * k < NE && ((vr + vc) * wa != R(0) || (vr - vc) * wc != R(0))) y[k] = __ldg(src + T * k);
+            if (base_kind == kBaseSelf) y[k] = sp[cs + 512 * k];
+            else if (base_kind == kBaseRho && on[k]) y[k] = __ldcs(rn + k * step);
         }
 #pragma unroll
-        for (int k = 0; k < E; ++k) {
-            const int r = rc[k] >> 16, c = rc[k] & 0xffff;
-            const R vr = sV[j * D + r], vc = sV[j * D + c];
-            const R ar = -(vr + vc) * wa, ai = -(vr - vc) * wc;
-            acc[k].x += ar * y[k].x - ai * y[k].y;
-            acc[k].y += ar * y[k].y + ai * y[k].x;
-        }
-    }
-    // ---- up term of tier L-1, summed by large_upterm_kernel
-    if (slot >= 0) {
-        const C* Un = a.U + static_cast<long long>(slot) * P + q0 + tid;
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-            if (tid + T * k >= NE) continue;
-            const C w = __ldcs(Un + T * k);
-            acc[k].x += w.x;
-            acc[k].y += w.y;
-        }
-    }
-    // ---- Horner epilogue
-    C* on = out + n * P + q0 + tid;
-    const C* rn = rho + n * P + q0 + tid;
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        if (tid + T * k >= NE) continue;
-        C b;
-        if (base_kind == kBaseSelf) {
-            const int r = rc[k] >> 16, c = rc[k] & 0xffff;
-            b = sx[lrow(r) * D + c];
-        } else if (base_kind == kBaseRho) {
-            b = __ldcs(rn + T * k);
-        } else {
-            b = mk<R>(0, 0);
-        }
-        __stcs(on + T * k, mk<R>(b.x + alpha * acc[k].x, b.y + alpha * acc[k].y));
+        for (int k = 0; k < E; ++k)
+            if (on[k]) __stcs(on_ + k * step, mk<R>(y[k].x + alpha * acc[k].x, y[k].y + alpha * acc[k].y));
     }
 }
 
@@ -455,24 +559,41 @@ __global__ void __launch_bounds__(kUpWarps * 32)
     }
     const C* ue = u + e;
     const int s0 = (blockIdx.x * kUpWarps + warp) * kUpSlots;
-    for (int s = s0; s < s0 + kUpSlots && s < a.S; ++s) {
-        const int32_t* slab = a.slab + static_cast<long long>(s) * a.M;
-        R re = 0, im = 0;
-        for (int j = 0; j < a.J; ++j) {
-            const R del = __ldg(a.vdiag + j * D + r) - __ldg(a.vdiag + j * D + c);
-            if (del == R(0)) continue;
-            const int m1 = __ldg(a.bath_off + j + 1);
-            R sr = 0, si = 0;
-            for (int m = __ldg(a.bath_off + j); m < m1; ++m) {
-                const C y = __ldg(ue + static_cast<long long>(__ldg(slab + m)) * D2);
-                sr += y.x;
-                si += y.y;
-            }
-            re += del * si;  // -i del S
-            im -= del * sr;
-        }
-        U[static_cast<long long>(s) * D2 + e] = mk<R>(re, im);
+    const int ns = min(a.S - s0, kUpSlots);
+    if (ns <= 0) return;
+    const int32_t* slab[kUpSlots];
+    R re[kUpSlots], im[kUpSlots];
+#pragma unroll
+    for (int t = 0; t < kUpSlots; ++t) {
+        slab[t] = a.slab + static_cast<long long>(s0 + min(t, ns - 1)) * a.M;
+        re[t] = im[t] = 0;
     }
+    for (int j = 0; j < a.J; ++j) {
+        const R del = __ldg(a.vdiag + j * D + r) - __ldg(a.vdiag + j * D + c);
+        if (del == R(0)) continue;
+        const int m1 = __ldg(a.bath_off + j + 1);
+        R sr[kUpSlots], si[kUpSlots];
+#pragma unroll
+        for (int t = 0; t < kUpSlots; ++t) sr[t] = si[t] = 0;
+        for (int m = __ldg(a.bath_off + j); m < m1; ++m) {
+            C y[kUpSlots];
+#pragma unroll
+            for (int t = 0; t < kUpSlots; ++t) y[t] = __ldg(ue + static_cast<long long>(__ldg(slab[t] + m)) * D2);
+#pragma unroll
+            for (int t = 0; t < kUpSlots; ++t) {
+                sr[t] += y[t].x;
+                si[t] += y[t].y;
+            }
+        }
+#pragma unroll
+        for (int t = 0; t < kUpSlots; ++t) {
+            re[t] += del * si[t];  // -i del S
+            im[t] -= del * sr[t];
+        }
+    }
+#pragma unroll
+    for (int t = 0; t < kUpSlots; ++t)
+        if (t < ns) U[static_cast<long long>(s0 + t) * D2 + e] = mk<R>(re[t], im[t]);
 }
 
 // Tier-0 ADO of the mixed-precision propagator in double precision: its own
@@ -595,6 +716,14 @@ __global__ void vec_d2f_kernel(const double* __restrict__ in, float* __restrict_
 }
 
 template <typename R, int LOGD>
+size_t tile_smem(int M, int J, bool pauli)
+{
+    const size_t D = size_t(1) << LOGD;
+    return 4096 * sizeof(C2<R>) + (pauli ? D * (sizeof(double) + sizeof(R)) : J * D * sizeof(R)) +
+           sizeof(R) * (LOGD + 4 * M) + sizeof(int) * 4 * M;
+}
+
+template <typename R, int LOGD>
 size_t large_smem(int M, int J, bool dense)
 {
     const size_t strip = dense ? sizeof(C2<R>) * (1 << LOGD) * (4096 / (1 << LOGD) + 1) + 16 : 0;
@@ -606,7 +735,8 @@ template <typename R, int LOGD>
 bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* out, double alpha, int base,
               cudaStream_t s, bool launch)
 {
-    const size_t smem = large_smem<R, LOGD>(a.M, a.J, a.dense_y != nullptr);
+    const size_t smem = a.herm ? tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0)
+                               : large_smem<R, LOGD>(a.M, a.J, a.dense_y != nullptr);
     if (smem > 227 * 1024) return false;
     static size_t configured[64] = {};
     int dev = 0;
@@ -614,17 +744,22 @@ bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* ou
     if (dev < 64 && configured[dev] < smem) {
         if (cudaFuncSetAttribute(large_kernel<R, LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)) != cudaSuccess ||
-            cudaFuncSetAttribute(herm_band_kernel<R, LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            cudaFuncSetAttribute(herm_tile_kernel<R, LOGD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 static_cast<int>(smem)) != cudaSuccess ||
+            cudaFuncSetAttribute(herm_tile_kernel<R, LOGD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(smem)) != cudaSuccess)
             return false;
         configured[dev] = smem;
     }
     if (!launch) return true;
-    // bands per slab: d^2 / 4096 full-slab bands, or (d / 2) / (2048 / d) = d^2 / 4096 packed bands
-    const long long nb = (a.H - a.first_ado) * ((1ll << (2 * LOGD)) / 4096);
+    // full slabs: d^2 / 4096 bands each; packed slabs: the tiles of the upper triangle
+    constexpr long long kBlocks = (1 << LOGD) / 64;
+    const long long nb = (a.H - a.first_ado) * (a.herm ? kBlocks * (kBlocks + 1) / 2 : (1ll << (2 * LOGD)) / 4096);
     if (nb <= 0) return true;
-    if (a.herm)
-        herm_band_kernel<R, LOGD><<<static_cast<unsigned>(nb), BandThreads<R>::T, smem, s>>>(a, u, rho, out, alpha, base);
+    if (a.herm && a.pauli)
+        herm_tile_kernel<R, LOGD, true><<<static_cast<unsigned>(nb), kTileT, smem, s>>>(a, u, rho, out, alpha, base);
+    else if (a.herm)
+        herm_tile_kernel<R, LOGD, false><<<static_cast<unsigned>(nb), kTileT, smem, s>>>(a, u, rho, out, alpha, base);
     else large_kernel<R, LOGD><<<static_cast<unsigned>(nb), LargeThreads<R>::T, smem, s>>>(a, u, rho, out, alpha, base);
     return true;
 }
