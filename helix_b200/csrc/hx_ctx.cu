@@ -218,13 +218,15 @@ hx::LargeArgs<float> large_args32(const hx_ctx* c)
     a.hdiag = c->hdiag;
     a.xsum = c->xsum;
     a.dense_y = c->dense ? c->dense_y : nullptr;
+    a.dense = c->dense ? 1 : 0;
     return a;
 }
 
 template <typename R>
 hx::LargeUpArgs<R> large_up_args(const hx_ctx* c, const R* vdiag)
 {
-    return hx::LargeUpArgs<R>{vdiag, c->up_slab, c->bath_off, c->up_slots, c->M, c->J, c->logd, c->herm ? 1 : 0};
+    return hx::LargeUpArgs<R>{vdiag, c->up_slab, c->bath_off, c->up_slots, c->M, c->J, c->logd, c->herm ? 1 : 0,
+                               c->dense ? 1 : 0};
 }
 
 hx::Ado0Args ado0_args(const hx_ctx* c)

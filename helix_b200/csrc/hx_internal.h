@@ -279,6 +279,7 @@ struct LargeArgs {
     // without its diagonal), in the state layout; X_n is Hermitian, so H_off X_n = Y_n^dagger and
     // -i[H_off, X_n]_rc = -i(conj(Y_cr) - Y_rc)
     const C2<R>* dense_y;
+    int dense;               // 1: a dense-H context (dense_tile_kernel)
 };
 template <typename R>
 struct LargeUpArgs {
@@ -287,6 +288,7 @@ struct LargeUpArgs {
     const int32_t* bath_off; // [J+1]
     int S, M, J, logd;
     int herm;                // 1: slabs and U Hermitian-packed
+    int upper;               // 1 (full slabs): the 64 x 64 tiles on and above the diagonal only
 };
 struct Ado0Args {
     const double2* diag;     // [d*d]

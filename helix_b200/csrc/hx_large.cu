@@ -23,7 +23,7 @@
 // the stage by the tensor-core GEMM (hx_tcgemm.cu) as one [H d x 2d] x
 // [2d x 2d] real product in 3-term TF32 split form.  Every ADO is Hermitian,
 // so H_off X_n = Y_n^dagger and -i[H_off, X_n]_rc = -i(conj(Y_cr) - Y_rc): one
-// product per ADO, not two.
+// product per ADO, not two (dense_tile_kernel).
 //
 // The reference has no precision other than the compiled one
 // (src/legacy_compile_options.h:6); the complex64 path is the
@@ -76,13 +76,10 @@ __global__ void __launch_bounds__(LargeThreads<R>::T, 2)
     R* sH = sV + a.J * D;                                     // [LOGD]
     int* sSlab = reinterpret_cast<int*>(sH + LOGD + 1);       // [2M]
     int* sBath = sSlab + 2 * a.M;                             // [2M]
-    constexpr int RB = BE / D, RBP = RB + 1;                  // rows of the band; padded strip row
-    C* sYT = reinterpret_cast<C*>((reinterpret_cast<uintptr_t>(sBath + 2 * a.M) + 15) & ~uintptr_t(15));  // [D][RBP]
 
     const int tid = threadIdx.x;
     const long long n = a.first_ado + static_cast<long long>(blockIdx.x) / NB;
     const long long be = static_cast<long long>(blockIdx.x % NB) * BE;  // band's first element in the slab
-    const int r0 = static_cast<int>(be >> LOGD);                        // band's first row
     const C* un = u + n * D2;
     if (tid == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(l_addr(bar)) : "memory");
@@ -108,22 +105,9 @@ __global__ void __launch_bounds__(LargeThreads<R>::T, 2)
         sWc[q] = a.ent_wc[src];
         sWa[q] = a.ent_wa[src];
     }
-    if (a.dense_y) {
-        // dense H: the strip Y_n[c][r0 .. r0 + RB) of every column c (coalesced row pieces, asynchronous
-        // 8-byte copies that overlap the table loads) for the transposed elements Y_cr of this band
-        const C* yn = a.dense_y + n * D2;
-#pragma unroll
-        for (int k = 0; k < BE / T; ++k) {
-            const int i = tid + k * T, cc = i / RB, j = i - cc * RB;
-            asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(l_addr(sYT + cc * RBP + j)),
-                         "l"(yn + (static_cast<long long>(cc) << LOGD) + r0 + j)
-                         : "memory");
-        }
-    }
     const R g = static_cast<R>(a.gsum[n]);
     const int slot = a.slot ? a.slot[n] : -1;
     const R alpha = static_cast<R>(alpha_d);
-    if (a.dense_y) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     bool ok = false;
     for (uint32_t it = 0; it < kLargeSpin && !ok; ++it) {
@@ -157,7 +141,7 @@ __global__ void __launch_bounds__(LargeThreads<R>::T, 2)
             R hr = 0, hi = 0;
 #pragma unroll
             for (int i = 0; i < LOGD; ++i) {
-                if (sH[i] == R(0)) continue;  // no field on this spin (every spin with a dense H): no gathers
+                if (sH[i] == R(0)) continue;  // no field on this spin: no gathers
                 constexpr long long one = 1;
                 const long long fb = static_cast<long long>(D) << i;  // row bit i of the element index
                 C rowp;
@@ -170,13 +154,6 @@ __global__ void __launch_bounds__(LargeThreads<R>::T, 2)
             const R tr = t[kk].x - g;
             acc[k0 + kk].x = tr * x[kk].x - t[kk].y * x[kk].y + hi;
             acc[k0 + kk].y = tr * x[kk].y + t[kk].y * x[kk].x - hr;
-            if (a.dense_y) {
-                // -i [H_off, X] = -i (conj(Y_cr) - Y_rc) from the tensor-core product Y = X H_off
-                const int r = static_cast<int>(ge >> LOGD), c = static_cast<int>(ge & (D - 1));
-                const C yrc = __ldg(a.dense_y + n * D2 + ge), ycr = sYT[c * RBP + (r - r0)];
-                acc[k0 + kk].x -= yrc.y + ycr.y;
-                acc[k0 + kk].y += yrc.x - ycr.x;
-            }
         }
     }
     // ---- neighbour entries, two at a time, CH elements per load batch
@@ -251,6 +228,149 @@ __global__ void __launch_bounds__(LargeThreads<R>::T, 2)
         else b = mk<R>(0, 0);
         __stcs(on + T * k, mk<R>(b.x + alpha * acc[k].x, b.y + alpha * acc[k].y));
     }
+}
+
+// ---------------------------------------------------------------------------
+// Stage of a dense H on full slabs (complex64): no flips, the commutator with
+// H_off comes from Y_n = X_n H_off.  The term at (r, c) needs Y_rc and Y_cr,
+// and the result is Hermitian, so a CTA takes a pair of 64 x 64 tiles (I, J)
+// and (J, I), I <= J: it reads both tiles of Y, but the slab, the neighbours,
+// the up terms and the base of the upper tile only, and writes the result and
+// its conjugate transpose.  The transposed tiles pass through shared memory
+// (element (r, c) at r 65 + c), so every access to memory is a run of columns.
+// Bound by HBM: 12 of the 16 slabs' bytes of the element by element form.
+// MEASURED_DENSE
+template <int LOGD, bool PAULI>
+__global__ void __launch_bounds__(512, 2)
+    dense_tile_kernel(LargeArgs<float> a, const float2* __restrict__ u, const float2* rho, float2* out, double alpha_d,
+                      int base_kind)
+{
+    constexpr int D = 1 << LOGD, NBK = D / 64, NT = NBK * (NBK + 1) / 2, E = 4;
+    constexpr long long D2 = static_cast<long long>(D) * D;
+    extern __shared__ __align__(128) unsigned char smem[];
+    float2* sT = reinterpret_cast<float2*>(smem);                            // [64][65] Y of tile (J, I), then the result
+    double* sE = reinterpret_cast<double*>(smem + 64 * 65 * sizeof(float2));  // [D] (PAULI)
+    float* sX = reinterpret_cast<float*>(sE + (PAULI ? D : 0));              // [D] (PAULI)
+    float* sV = sX + (PAULI ? D : 0);                                        // [J][D] (general couplings)
+    float* sWc = sV + (PAULI ? 0 : a.J * D);                                 // [2M] (twice the weights with PAULI)
+    float* sWa = sWc + 2 * a.M;                                              // [2M]
+    int* sSlab = reinterpret_cast<int*>(sWa + 2 * a.M);                      // [2M]
+    int* sBit = sSlab + 2 * a.M;                                             // [2M] spin (PAULI) or bath
+
+    const int tid = threadIdx.x;
+    const long long n = a.first_ado + static_cast<long long>(blockIdx.x) / NT;
+    int J = 0, I = static_cast<int>(blockIdx.x % NT);
+    while (I > J) I -= ++J;
+    const int c = tid & 63, r0 = tid >> 6;  // rows r0 + 8 k of the tile
+    const int gc = J * 64 + c, gr0 = I * 64 + r0;
+    const long long own = n * D2 + (static_cast<long long>(gr0) << LOGD) + gc;   // + 8 D k
+    const long long mir = n * D2 + (static_cast<long long>(J * 64 + r0) << LOGD) + I * 64 + c;  // the transposed tile
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sT[(r0 + 8 * k) * 65 + c] = __ldcs(a.dense_y + mir + 8ll * D * k);
+    const int Q = a.ent_count[n];
+    for (int q = tid; q < Q; q += 512) {
+        const long long e = n * 2 * a.M + q;
+        const int j = a.ent_bath[e] & 0xffff;
+        sSlab[q] = a.ent_slab[e];
+        sBit[q] = PAULI ? a.vbit[j] : j;
+        sWc[q] = static_cast<float>(PAULI ? 2.0 * a.ent_wc[e] : a.ent_wc[e]);
+        sWa[q] = static_cast<float>(PAULI ? 2.0 * a.ent_wa[e] : a.ent_wa[e]);
+    }
+    if (PAULI) {
+        for (int i = tid; i < D; i += 512) {
+            sE[i] = a.hdiag[i];
+            sX[i] = static_cast<float>(a.xsum[i]);
+        }
+    } else {
+        for (int i = tid; i < a.J * D; i += 512) sV[i] = a.vdiag[i];
+    }
+    const float g = static_cast<float>(a.gsum[n]);
+    const int slot = a.slot ? a.slot[n] : -1;
+    const float alpha = static_cast<float>(alpha_d);
+    __syncthreads();
+    float2 o[8];
+#pragma unroll
+    for (int k0 = 0; k0 < 8; k0 += E) {
+        float2 x[E], acc[E];
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            x[k] = __ldg(u + own + 8ll * D * (k0 + k));
+            acc[k] = __ldcs(a.dense_y + own + 8ll * D * (k0 + k));
+        }
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            const int r = gr0 + 8 * (k0 + k);
+            float tr, ti;
+            if (PAULI) {
+                tr = sX[r ^ gc];
+                ti = static_cast<float>(sE[gc] - sE[r]);
+            } else {
+                const float2 t = __ldg(a.diag + (static_cast<long long>(r) << LOGD) + gc);
+                tr = t.x;
+                ti = t.y;
+            }
+            tr -= g;
+            // -i [H_off, X] = -i (conj(Y_cr) - Y_rc)
+            const float2 yrc = acc[k], ycr = sT[c * 65 + r0 + 8 * (k0 + k)];
+            acc[k].x = tr * x[k].x - ti * x[k].y - (yrc.y + ycr.y);
+            acc[k].y = tr * x[k].y + ti * x[k].x + (yrc.x - ycr.x);
+        }
+        const float2* ub = u + own - n * D2 + 8ll * D * k0;
+#pragma unroll 1
+        for (int q = 0; q < Q; ++q) {
+            const float2* src = ub + sSlab[q] * D2;
+            const float wc = sWc[q], wa = sWa[q];
+            const int bit = sBit[q];
+            float2 y[E];
+            float wr[E], wi[E];
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                const int r = gr0 + 8 * (k0 + k);
+                if (PAULI) {
+                    // equal bits: only -{V, y} wa; different bits: only -i [V, y] wc
+                    const int br = (r >> bit) & 1;
+                    const bool same = br == ((gc >> bit) & 1);
+                    wr[k] = same ? (br ? -wa : wa) : 0.f;
+                    wi[k] = same ? 0.f : (br ? -wc : wc);
+                } else {
+                    const float vr = sV[bit * D + r], vc = sV[bit * D + gc];
+                    wr[k] = -(vr + vc) * wa;
+                    wi[k] = -(vr - vc) * wc;
+                }
+                y[k] = mk<float>(0.f, 0.f);
+                if (wr[k] != 0.f || wi[k] != 0.f) y[k] = __ldg(src + 8ll * D * k);
+            }
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                acc[k].x += wr[k] * y[k].x - wi[k] * y[k].y;
+                acc[k].y += wr[k] * y[k].y + wi[k] * y[k].x;
+            }
+        }
+        if (slot >= 0) {
+#pragma unroll
+            for (int k = 0; k < E; ++k) {
+                const float2 w = __ldcs(a.U + slot * D2 + own - n * D2 + 8ll * D * (k0 + k));
+                acc[k].x += w.x;
+                acc[k].y += w.y;
+            }
+        }
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            float2 b = mk<float>(0.f, 0.f);
+            if (base_kind == kBaseSelf) b = x[k];
+            else if (base_kind == kBaseRho) b = __ldcs(rho + own + 8ll * D * (k0 + k));
+            o[k0 + k] = mk<float>(b.x + alpha * acc[k].x, b.y + alpha * acc[k].y);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 8; ++k) __stcs(out + own + 8ll * D * k, o[k]);
+    if (I == J) return;
+    __syncthreads();  // every Y of the tile is read
+#pragma unroll
+    for (int k = 0; k < 8; ++k) sT[(r0 + 8 * k) * 65 + c] = mk<float>(o[k].x, -o[k].y);
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 8; ++k) __stcs(out + mir + 8ll * D * k, sT[c * 65 + r0 + 8 * k]);
 }
 
 // Element (r, c) of a Hermitian-packed slab, any r, c (one load, no branch
@@ -556,6 +676,7 @@ __global__ void __launch_bounds__(kUpWarps * 32)
     } else {
         r = static_cast<int>(e >> a.logd);
         c = static_cast<int>(e & (D - 1));
+        if (a.upper && (c >> 6) < (r >> 6)) return;  // a tile that nobody reads
     }
     const C* ue = u + e;
     const int s0 = (blockIdx.x * kUpWarps + warp) * kUpSlots;
@@ -724,11 +845,28 @@ size_t tile_smem(int M, int J, bool pauli)
 }
 
 template <typename R, int LOGD>
-size_t large_smem(int M, int J, bool dense)
+size_t large_smem(int M, int J)
 {
-    const size_t strip = dense ? sizeof(C2<R>) * (1 << LOGD) * (4096 / (1 << LOGD) + 1) + 16 : 0;
     return 4096 * sizeof(C2<R>) + 16 + sizeof(double) * 4 * M + sizeof(R) * (J * (1 << LOGD) + LOGD + 1) +
-           sizeof(int) * 4 * M + 16 + strip;
+           sizeof(int) * 4 * M + 16;
+}
+
+// Stage of a dense H; launch = false: raise the shared-memory limit only.
+template <int LOGD>
+bool launch_dense(const LargeArgs<float>& a, const float2* u, const float2* rho, float2* out, double alpha, int base,
+                  cudaStream_t s, bool launch)
+{
+    const size_t D = size_t(1) << LOGD;
+    const size_t smem = 64 * 65 * sizeof(float2) + (a.pauli ? D * (sizeof(double) + sizeof(float)) : a.J * D * sizeof(float)) +
+                        sizeof(float) * 4 * a.M + sizeof(int) * 4 * a.M;
+    if (smem > 227 * 1024) return false;
+    auto* kernel = a.pauli ? dense_tile_kernel<LOGD, true> : dense_tile_kernel<LOGD, false>;
+    if (!launch)
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
+    constexpr long long kBlocks = (1 << LOGD) / 64;
+    const long long nb = (a.H - a.first_ado) * (kBlocks * (kBlocks + 1) / 2);
+    if (nb > 0) kernel<<<static_cast<unsigned>(nb), 512, smem, s>>>(a, u, rho, out, alpha, base);
+    return true;
 }
 
 template <typename R, int LOGD>
@@ -736,7 +874,7 @@ bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* ou
               cudaStream_t s, bool launch)
 {
     const size_t smem = a.herm ? tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0)
-                               : large_smem<R, LOGD>(a.M, a.J, a.dense_y != nullptr);
+                               : large_smem<R, LOGD>(a.M, a.J);
     if (smem > 227 * 1024) return false;
     static size_t configured[64] = {};
     int dev = 0;
@@ -768,6 +906,16 @@ template <typename R>
 bool dispatch(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* out, double alpha, int base,
               cudaStream_t s, bool launch)
 {
+    if constexpr (sizeof(R) == sizeof(float))
+        if (a.dense) {
+            switch (a.logd) {
+            case 7: return launch_dense<7>(a, u, rho, out, alpha, base, s, launch);
+            case 8: return launch_dense<8>(a, u, rho, out, alpha, base, s, launch);
+            case 9: return launch_dense<9>(a, u, rho, out, alpha, base, s, launch);
+            case 10: return launch_dense<10>(a, u, rho, out, alpha, base, s, launch);
+            default: return false;
+            }
+        }
     switch (a.logd) {
     case 7: return launch_t<R, 7>(a, u, rho, out, alpha, base, s, launch);
     case 8: return launch_t<R, 8>(a, u, rho, out, alpha, base, s, launch);
