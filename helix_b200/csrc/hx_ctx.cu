@@ -58,7 +58,7 @@ void release(hx_ctx* c)
                     c->up_slab, c->up_bath, c->U, c->vflip, c->Bbuf, c->rho32, c->ua32, c->ub32,
                     c->U32, c->diag32, c->vdiag32, c->hflip32, c->diag_herm, c->vbit, c->csr_ptr, c->csr_col,
                     c->csr_val, c->pack_scale, c->pack_bad, c->dense_hr, c->dense_hr_lo, c->dense_y,
-                    c->dense_h64, c->dense_z0, c->gbar, c->cl_coef, c->cl_slot, c->xsum};
+                    c->dense_h64, c->dense_z0, c->gbar, c->cl_coef, c->cl_slot, c->xsum, c->obs_csr};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
@@ -397,7 +397,7 @@ int launch_obs(hx_ctx* c, double* out, double2* copy = nullptr)
     const bool csr = c->use_csr || c->dense;
     const bool fold = copy && !csr && c->logd <= hx::kMaxLogD;
     if (csr)
-        hx::launch_observables_csr(c->rho, c->logd, c->csr_ptr, c->csr_col, c->csr_val, out, c->stream);
+        hx::launch_observables_csr(c->rho, c->logd, c->csr_ptr, c->csr_col, c->csr_val, c->obs_csr, out, c->stream);
     else hx::launch_observables(c->rho, c->logd, c->herm, c->hdiag, c->hflip, fold ? copy : nullptr, out, c->stream);
     if (copy && !fold)
         HX_CUDA_TRY(cudaMemcpyAsync(copy, c->rho, c->slab_store * sizeof(double2), cudaMemcpyDeviceToDevice, c->stream));
@@ -910,6 +910,12 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     if ((rc = dev_alloc(c, &c->vflip, vf.size())) || (rc = upload(c, c->vflip, vf))) return bail(rc);
     // two-pass paths: [V_j, u_n] and {V_j, u_n} for every bath and ADO
     if ((c->use_flip || c->use_csr) && (rc = dev_alloc(c, &c->Bbuf, 2 * nstate * J))) return bail(rc);
+    if (c->use_csr || c->dense) {
+        const size_t n = hx::observables_csr_scratch();
+        if ((rc = dev_alloc(c, &c->obs_csr, n))) return bail(rc);
+        e = cudaMemsetAsync(c->obs_csr, 0, n * sizeof(double), c->stream);
+        if (e != cudaSuccess) return bail(hx::cuda_fail(e, "observables scratch"));
+    }
     if (c->use_csr) {
         std::vector<int32_t> ptr, col;
         std::vector<double2> val;

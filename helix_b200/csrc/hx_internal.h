@@ -371,9 +371,11 @@ struct CsrArgs {
 };
 void launch_csr_stage(const CsrArgs& a, const double2* u, double2* B, const double2* rho, double2* out, double alpha,
                       int base_kind, cudaStream_t s);
-// out[0] = Re Tr(H rho_0) with H in CSR (operator 0), out[1..2] = Tr rho_0.
+// out[0] = Re Tr(H rho_0) with H in CSR (operator 0), out[1..2] = Tr rho_0; scratch: that many doubles, zeroed
+// once by the caller (one per stream).
+size_t observables_csr_scratch();
 void launch_observables_csr(const double2* rho0, int logd, const int32_t* ptr, const int32_t* col,
-                            const double2* val, double* out, cudaStream_t s);
+                            const double2* val, double* scratch, double* out, cudaStream_t s);
 
 // Tables on the device (hx_tables.cu)
 int build_tables_device(int M, int D, long long H, int32_t* d_rows, int32_t* d_edges, cudaStream_t s);
@@ -472,6 +474,7 @@ struct hx_ctx {
     int32_t* order_perm = nullptr;
     int8_t* ado_keep = nullptr;
     double* obs = nullptr;        // [3] observables scratch
+    double* obs_csr = nullptr;    // partial sums of the CSR observables
     double2* trace_buf = nullptr; // per-step rho_0 chunk
     double* energy_buf = nullptr;
     int trace_cap = 0;

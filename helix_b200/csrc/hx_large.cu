@@ -8,8 +8,8 @@
 // for diagonal couplings V_j and H = diag(E) + sum_i h_i sigma_x(i).  A slab of
 // d = 256 is 1 MB in double precision, too large for shared memory, so:
 //
-//  * one CTA computes one band of 4096 elements (4096/d whole rows) of one
-//    ADO; the band arrives by one TMA bulk copy; consecutive CTAs take the
+//  * full slabs: one CTA computes one band of 4096 elements (4096/d whole rows)
+//    of one ADO (packed slabs: herm_tile_kernel below); the band arrives by one TMA bulk copy; consecutive CTAs take the
 //    bands of one ADO, so the rest of its slab is in L2 while they run;
 //  * column flips of the transverse field and row flips inside the band read
 //    shared memory; row flips across bands read the slab through L2;
@@ -239,7 +239,8 @@ __global__ void __launch_bounds__(LargeThreads<R>::T, 2)
 // its conjugate transpose.  The transposed tiles pass through shared memory
 // (element (r, c) at r 65 + c), so every access to memory is a run of columns.
 // Bound by HBM: 12 of the 16 slabs' bytes of the element by element form.
-// MEASURED_DENSE
+// d = 256, 969 ADOs: 384 us a stage, where bands that computed both triangles
+// took 635.
 template <int LOGD, bool PAULI>
 __global__ void __launch_bounds__(512, 2)
     dense_tile_kernel(LargeArgs<float> a, const float2* __restrict__ u, const float2* rho, float2* out, double alpha_d,
@@ -406,7 +407,9 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 //    term from two d-entry tables instead of a third slab-sized stream;
 //  * diagonal tiles compute their upper triangle only.
 //
-// MEASURED_TILE
+// d = 256, 969 ADOs: 0.70 ms a stage in double, 0.48 in complex64 (bands of
+// rows: 0.94 and 0.56).  The 64 registers of two CTAs per SM are the limit: one
+// pass of 8 rows in double spills or leaves one CTA (0.85 ms).
 template <typename R, int LOGD> struct TileShape;
 template <int LOGD> struct TileShape<double, LOGD> { static constexpr int NP = 2, MINB = 2, LR = LOGD == 7 ? 1 : 4; };
 template <int LOGD> struct TileShape<float, LOGD> { static constexpr int NP = 1, MINB = 2, LR = 2; };
@@ -780,46 +783,56 @@ __global__ void __launch_bounds__(256)
     out32[ge] = make_float2(static_cast<float>(o.x), static_cast<float>(o.y));
 }
 
-// Z = X H, d x d complex FP64 (ADO 0 of a dense-H stage): 32 x 32 output
-// tiles, K staged through shared memory 16 at a time; each thread keeps four
-// outputs of one column.  d^3 complex multiply-adds, a few microseconds at
-// d = 256.
+// Z = X H, d x d complex FP64 (ADO 0 of a dense-H stage): 32 x 16 output
+// tiles, two outputs of one row per thread, K staged through shared memory 32
+// at a time with the next block's loads under way.  d^3 complex multiply-adds
+// in d^2 / 512 CTAs (d = 256: 48 us with 64 CTAs of 16 x 4 outputs a warp,
+// ZGEMM us).
 __global__ void __launch_bounds__(256) zgemm_kernel(const double2* __restrict__ x, const double2* __restrict__ h,
                                                     double2* __restrict__ z, int logd)
 {
-    constexpr int TM = 32, TN = 32, TK = 16;
+    constexpr int TM = 32, TN = 16, TK = 32;
     __shared__ double2 sa[TM][TK + 1];
-    __shared__ double2 sb[TK][TN + 1];
+    __shared__ double2 sb[TK][TN];
     const int D = 1 << logd;
     const int m0 = blockIdx.y * TM, n0 = blockIdx.x * TN;
-    const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    double2 acc[4];
+    const int tid = threadIdx.x, col = tid & 7, row = tid >> 3;  // outputs (row, col) and (row, col + 8)
+    double2 ra[4], rb[2];
+    auto fetch = [&](int k0) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[j] = make_double2(0.0, 0.0);
+        for (int i = 0; i < 4; ++i) {
+            const int e = tid + 256 * i;
+            ra[i] = __ldg(x + (static_cast<long long>(m0 + (e >> 5)) << logd) + k0 + (e & 31));
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int e = tid + 256 * i;
+            rb[i] = __ldg(h + (static_cast<long long>(k0 + (e >> 4)) << logd) + n0 + (e & 15));
+        }
+    };
+    double2 acc[2] = {make_double2(0.0, 0.0), make_double2(0.0, 0.0)};
+    fetch(0);
     for (int k0 = 0; k0 < D; k0 += TK) {
-        for (int i = threadIdx.x; i < TM * TK; i += 256) {
-            const int rr = i / TK, kk = i - rr * TK;
-            sa[rr][kk] = x[(static_cast<long long>(m0 + rr) << logd) + k0 + kk];
-        }
-        for (int i = threadIdx.x; i < TK * TN; i += 256) {
-            const int kk = i / TN, cc = i - kk * TN;
-            sb[kk][cc] = h[(static_cast<long long>(k0 + kk) << logd) + n0 + cc];
-        }
         __syncthreads();
 #pragma unroll
-        for (int kk = 0; kk < TK; ++kk) {
-            const double2 b = sb[kk][tx];
+        for (int i = 0; i < 4; ++i) sa[(tid + 256 * i) >> 5][(tid + 256 * i) & 31] = ra[i];
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const double2 av = sa[ty + 8 * j][kk];
+        for (int i = 0; i < 2; ++i) sb[(tid + 256 * i) >> 4][(tid + 256 * i) & 15] = rb[i];
+        __syncthreads();
+        if (k0 + TK < D) fetch(k0 + TK);
+#pragma unroll 8
+        for (int kk = 0; kk < TK; ++kk) {
+            const double2 av = sa[row][kk];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const double2 b = sb[kk][col + 8 * j];
                 acc[j].x = fma(av.x, b.x, fma(-av.y, b.y, acc[j].x));
                 acc[j].y = fma(av.x, b.y, fma(av.y, b.x, acc[j].y));
             }
         }
-        __syncthreads();
     }
 #pragma unroll
-    for (int j = 0; j < 4; ++j) z[(static_cast<long long>(m0 + ty + 8 * j) << logd) + n0 + tx] = acc[j];
+    for (int j = 0; j < 2; ++j) z[(static_cast<long long>(m0 + row) << logd) + n0 + col + 8 * j] = acc[j];
 }
 
 __global__ void d2f_kernel(const double2* __restrict__ in, float2* __restrict__ out, long long n)
@@ -969,8 +982,7 @@ template void launch_large_upterm<float>(const LargeUpArgs<float>&, const float2
 
 void launch_zgemm(const double2* x, const double2* h, double2* z, int logd, cudaStream_t s)
 {
-    const unsigned nt = 1u << (logd - 5);
-    zgemm_kernel<<<dim3(nt, nt), 256, 0, s>>>(x, h, z, logd);
+    zgemm_kernel<<<dim3(1u << (logd - 4), 1u << (logd - 5)), 256, 0, s>>>(x, h, z, logd);
 }
 
 void launch_ado0(const Ado0Args& a, const double2* u0, const float2* u, const double2* rho0, double2* out0,
