@@ -164,6 +164,12 @@ hx::FlipArgs flip_args_of(const hx_ctx* c)
     return a;
 }
 
+hx::CsrArgs csr_args_of(const hx_ctx* c)
+{
+    return hx::CsrArgs{c->csr_ptr, c->csr_col, c->csr_val, c->edges, c->acoef, c->bcoef, c->gsum,
+                       c->xi,      c->counter, c->bath_off, c->H, c->M, c->J, c->logd};
+}
+
 hx::LargeArgs<double> large_args64(const hx_ctx* c)
 {
     hx::LargeArgs<double> a{};
@@ -311,10 +317,10 @@ int launch_stage_any(hx_ctx* c, const double2* u, const double2* rho, double2* o
 int launch_stage_core(hx_ctx* c, const double2* u, const double2* rho, double2* out, double alpha, int base)
 {
     if (c->use_large) return launch_large_stage(c, u, rho, out, alpha, base);
+    if (c->use_slab)
+        return hx::launch_slab_stage(csr_args_of(c), c->csr_nnz, u, c->Bbuf, rho, out, alpha, base, c->stream);
     if (c->use_csr) {
-        const hx::CsrArgs a{c->csr_ptr, c->csr_col, c->csr_val, c->edges, c->acoef, c->bcoef, c->gsum,
-                            c->xi,      c->counter, c->bath_off, c->H, c->M, c->J, c->logd};
-        hx::launch_csr_stage(a, u, c->Bbuf, rho, out, alpha, base, c->stream);
+        hx::launch_csr_stage(csr_args_of(c), u, c->Bbuf, rho, out, alpha, base, c->stream);
         return 2;
     }
     if (c->use_flip) {
@@ -351,9 +357,16 @@ void enqueue_run(hx_ctx* c, uint64_t nsteps, double2* trace, double* obs)
             w.max_polls = 1u << 12;
             c->stall_next_step = false;
         }
-        if (launch(hx::fused_args_of(c), cl, c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->sm_count, c->stream,
-                   false, trace ? trace + done * c->slab_store : nullptr, obs ? obs + 3 * done : nullptr, w) != 1)
+        double2* tr = trace ? trace + done * c->slab_store : nullptr;
+        double* ob = obs ? obs + 3 * done : nullptr;
+        if (c->use_slab) {
+            if (hx::launch_slab_run(csr_args_of(c), c->csr_nnz, c->slab_ctas, c->rho, c->ua, c->ub, c->dt, c->order, n,
+                                    c->gbar, c->error_flag, w, tr, ob, c->stream) != 1)
+                c->launch_failed = true;
+        } else if (launch(hx::fused_args_of(c), cl, c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->sm_count, c->stream,
+                   false, tr, ob, w) != 1) {
             c->launch_failed = true;
+        }
         c->counters.kernel_launches += 1;
         c->counters.stage_launches += static_cast<uint64_t>(c->order) * n;
         c->steps_done += n;
@@ -916,7 +929,14 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
         e = cudaMemsetAsync(c->obs_csr, 0, n * sizeof(double), c->stream);
         if (e != cudaSuccess) return bail(hx::cuda_fail(e, "observables scratch"));
     }
-    if (c->use_csr) {
+    const bool flip_slab = c->use_flip && logd <= hx::kMaxLogD;
+    if (flip_slab) {
+        ops.clear();
+        ops.push_back(flip_csr(p->h_diag, p->h_flip, static_cast<int>(d), logd));
+        for (int j = 0; j < J; ++j)
+            ops.push_back(flip_csr(p->baths[j].coupling_diag, p->baths[j].coupling_flip, static_cast<int>(d), logd));
+    }
+    if (c->use_csr || flip_slab) {
         std::vector<int32_t> ptr, col;
         std::vector<double2> val;
         for (const HostCsr& o : ops) {
@@ -929,6 +949,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             (rc = dev_alloc(c, &c->csr_val, val.size())) || (rc = upload(c, c->csr_ptr, ptr)) ||
             (rc = upload(c, c->csr_col, col)) || (rc = upload(c, c->csr_val, val)))
             return bail(rc);
+        c->csr_nnz = static_cast<int>(col.size());
     }
     // double-precision state: the whole hierarchy, or only ADO 0 in mixed precision
     const size_t n64 = c->mixed ? c->slab_store : nstate;
@@ -1164,6 +1185,20 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     cudaFree(dphi);
     cudaFree(dtc);
     cudaFree(dta);
+    // sparse operators at d <= 64: a slab per CTA when the operators fit beside it; couplings with flips run
+    // whole steps in one launch
+    if (rc == HX_OK && (c->use_csr || flip_slab) && logd <= hx::kMaxLogD && hx::prepare_slab(csr_args_of(c), c->csr_nnz)) {
+        c->use_slab = true;
+        if (flip_slab && c->order >= 2) {
+            cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
+            c->slab_ctas = hx::slab_run_ctas(csr_args_of(c), c->csr_nnz, c->sm_count);
+            if (c->slab_ctas > 0 && (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
+                e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
+                if (e != cudaSuccess) rc = hx::cuda_fail(e, "grid barrier counter");
+                else c->use_run = true;
+            }
+        }
+    }
     if (rc == HX_OK && c->use_large && (c->diag_table == nullptr || c->ent_count == nullptr))
         rc = fail(HX_ERR_UNSUPPORTED_EXECUTION, "band-kernel tables were not built");
     if (rc == HX_OK && c->use_large) {
@@ -1246,11 +1281,12 @@ int hx_ctx_sync(hx_ctx* c)
 int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* energy_trace)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    // chunk of steps buffered on the device: at most 256 steps and 64 MB of rho_0 copies
-    const uint64_t by_bytes = std::max<uint64_t>(1, (uint64_t(64) << 20) / (c->slab * sizeof(double2)));
+    // chunk of steps buffered at a time: at most 256, and 64 MB of rho_0 copies where those are asked for
+    const uint64_t by_bytes =
+        rho0_trace ? std::max<uint64_t>(1, (uint64_t(64) << 20) / (c->slab_store * sizeof(double2))) : 256;
     const int cap = static_cast<int>(std::min<uint64_t>(std::min<uint64_t>(std::max<uint64_t>(nsteps, 1), 256), by_bytes));
     const bool whole = c->use_run;
-    if (c->trace_cap < cap || (!whole && !c->trace_buf)) {
+    if (c->trace_cap < cap || (rho0_trace && !c->trace_rho) || (!whole && !c->energy_buf)) {
         if (c->trace_buf) cudaFree(c->trace_buf);
         if (c->energy_buf) cudaFree(c->energy_buf);
         if (c->pinned) cudaFreeHost(c->pinned);
@@ -1258,16 +1294,18 @@ int hx_ctx_step_trace(hx_ctx* c, uint64_t nsteps, double* rho0_trace, double* en
         c->energy_buf = nullptr;
         c->pinned = nullptr;
         c->trace_cap = 0;
+        const size_t rho_bytes = rho0_trace ? cap * c->slab_store * sizeof(double2) : 0;
         if (!whole) {
-            HX_CUDA_TRY(cudaMalloc(&c->trace_buf, cap * c->slab * sizeof(double2)));
+            if (rho0_trace) HX_CUDA_TRY(cudaMalloc(&c->trace_buf, rho_bytes));
             HX_CUDA_TRY(cudaMalloc(&c->energy_buf, cap * 3 * sizeof(double)));
         }
-        c->pinned_bytes = cap * (c->slab * sizeof(double2) + 3 * sizeof(double));
+        c->pinned_bytes = rho_bytes + cap * 3 * sizeof(double);
         HX_CUDA_TRY(cudaMallocHost(&c->pinned, c->pinned_bytes));
         c->trace_cap = cap;
+        c->trace_rho = rho0_trace != nullptr;
     }
     double* pin_rho = c->pinned;
-    double* pin_en = c->pinned + static_cast<size_t>(c->trace_cap) * c->slab * 2;
+    double* pin_en = c->pinned + (c->trace_rho ? static_cast<size_t>(c->trace_cap) * c->slab_store * 2 : 0);
     uint64_t done = 0;
     while (done < nsteps) {
         const int chunk = static_cast<int>(std::min<uint64_t>(nsteps - done, c->trace_cap));

@@ -371,6 +371,17 @@ struct CsrArgs {
 };
 void launch_csr_stage(const CsrArgs& a, const double2* u, double2* B, const double2* rho, double2* out, double alpha,
                       int base_kind, cudaStream_t s);
+// The same operators at d <= 64, a slab per CTA (hx_slab.cu); nnz entries in all operators.  prepare_slab: 1
+// when the operators fit in shared memory beside the slabs (raises the kernels' limits; before any capture).
+int prepare_slab(const CsrArgs& a, int nnz);
+// One stage: gather pass (G: 2 J H slabs) and products.  Kernels launched.
+int launch_slab_stage(const CsrArgs& a, int nnz, const double2* u, double2* G, const double2* rho, double2* out,
+                      double alpha, int base_kind, cudaStream_t s);
+// Whole steps in one cooperative launch on `ctas` CTAs (slab_run_ctas; 0: not possible) and a watching one;
+// the rest as in launch_small_run.
+int slab_run_ctas(const CsrArgs& a, int nnz, int sms);
+int launch_slab_run(const CsrArgs& a, int nnz, int ctas, double2* rho, double2* ua, double2* ub, double dt, int order,
+                    int nsteps, unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs, cudaStream_t s);
 // out[0] = Re Tr(H rho_0) with H in CSR (operator 0), out[1..2] = Tr rho_0; scratch: that many doubles, zeroed
 // once by the caller (one per stream).
 size_t observables_csr_scratch();
@@ -426,6 +437,8 @@ struct hx_ctx {
     double* vflip = nullptr;      // [J][log2 d]
     bool use_flip = false;        // two-pass flip path (flips in V, or d > 1024)
     bool use_csr = false;         // two-pass path for general sparse H / V_j (hx_csr.cu)
+    bool use_slab = false;        // ... or with flips, at d <= 64: a slab per CTA (hx_slab.cu)
+    int csr_nnz = 0, slab_ctas = 0;
     int32_t* csr_ptr = nullptr;   // [(J+1)(d+1)] operator 0 = H, 1 + j = V_j
     int32_t* csr_col = nullptr;
     double2* csr_val = nullptr;
@@ -477,7 +490,8 @@ struct hx_ctx {
     double* obs_csr = nullptr;    // partial sums of the CSR observables
     double2* trace_buf = nullptr; // per-step rho_0 chunk
     double* energy_buf = nullptr;
-    int trace_cap = 0;
+    int trace_cap = 0;            // steps the trace buffers hold
+    bool trace_rho = false;       // ... with rho_0 (or energies only)
     double* pinned = nullptr;     // pinned staging for traces
     int* flag_pin = nullptr;      // pinned copy of the error word
     size_t pinned_bytes = 0;

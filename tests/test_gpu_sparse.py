@@ -95,3 +95,44 @@ def test_flip_form_csr_operators_take_the_fast_paths(case):
     o.close()
     assert np.max(np.abs(rb - rho_ref)) <= TOL
     assert np.max(np.abs(eb - en_ref)) <= TOL
+
+
+@pytest.mark.parametrize("n,baths,K,depth,order", [
+    (1, 1, 1, 2, 4),   # 6 ADOs at d = 2, less than a warp
+    (3, 3, 0, 2, 3),   # 10 ADOs at d = 8
+    (5, 2, 1, 2, 4),   # 15 ADOs at d = 32: a warp per row
+    (6, 3, 1, 3, 4),   # 84 ADOs at d = 64: two elements per lane
+    (6, 1, 0, 1, 4),   # 2 ADOs at d = 64: the two-pass kernels
+])
+def test_slab_kernels_match_oracle(n, baths, K, depth, order):
+    """d <= 64: general sparse operators (a slab per CTA, one stage per two
+    launches) and couplings with flips (whole steps in one launch), with
+    random complex states, right-hand side and steps."""
+    p = S.sparse_problem(n, seed=700 + n, depth=depth, K=K, dt=0.005)
+    p.baths = p.baths[:baths]
+    f = S.spin_glass(n, seed=710 + n, depth=depth, K=K, h=0.6, dt=0.005)
+    f.baths = f.baths[:baths]
+    rng = np.random.default_rng(n)
+    for b in f.baths:
+        b.v_diag = rng.uniform(-0.5, 0.5, f.dim)
+        b.v_flip = rng.uniform(0.2, 0.6, n)
+    for q, path in ((p, "csr"), (f, "flip")):
+        o = O.Oracle(q)
+        x = rng.standard_normal((o.size, q.dim, q.dim)) + 1j * rng.standard_normal((o.size, q.dim, q.dim))
+        x *= 0.1
+        with capi.Context(q, order=order) as a, capi.Context(q, order=order) as b:
+            assert a.stage_path == path
+            a.set_state(x)
+            b.set_state(x)
+            want = o.rhs(x)
+            assert np.max(np.abs(a.rhs() - want)) <= 1e-12 * max(1.0, np.max(np.abs(want)))
+            o.set_state(x)
+            rho_ref, en_ref = o.run(3, order=order, trace=True)
+            rho, en = a.step_trace(3)
+            b.step(3)
+            b.sync()
+            assert np.array_equal(a.state(), b.state())
+            assert np.max(np.abs(a.state() - o.state())) <= TOL
+            assert abs(a.observables()[0] - en[-1]) <= 1e-13 * max(1.0, abs(en[-1]))
+        o.close()
+        assert np.max(np.abs(rho - rho_ref)) <= TOL
