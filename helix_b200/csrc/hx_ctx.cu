@@ -899,7 +899,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
                              "HX_FLAG_DENSE_H needs 128 <= d <= 1024 and diagonal coupling operators"));
         if (static_cast<long long>(H) * d > INT32_MAX)
             return bail(fail(HX_ERR_UNSUPPORTED_EXECUTION, "HX_FLAG_DENSE_H: H d exceeds the GEMM's row range"));
-        if (!hx::tc_gemm_ready(true))
+        if (!hx::tc_gemm_ready())
             return bail(fail(HX_ERR_UNSUPPORTED_EXECUTION, "HX_FLAG_DENSE_H: the tensor-core GEMM is unavailable"));
         for (const double2& v : dense_h.val)
             if (!std::isfinite(v.x) || !std::isfinite(v.y))

@@ -167,21 +167,11 @@ struct TcGemmOut {
     const float* aux;   // pre-activation Z for kTcEpiGeluBack
     int ldo;
 };
-bool tc_gemm_eligible(const void* A, int lda, const void* B, int ldb);
+// part (part_elems floats, may be nullptr): room for the sums of a split K (plain stores only).
 bool tc_gemm(int M, int N, int K, const void* A, int lda, const void* B, int ldb, const TcGemmOut& o, int* err,
-             cudaStream_t s);
-// Sum of up to three products A_p B_p^T in one accumulator, BF16 or FP32 operands (the latter on the TF32
-// path): the terms of a split-precision product.  Leading dimensions multiples of 16 bytes.
-struct TcPair {
-    const void* A;
-    int lda;
-    const void* B;
-    int ldb;
-};
-bool tc_gemm_sum(int M, int N, int K, int npairs, const TcPair* pairs, bool tf32, const TcGemmOut& o, int* err,
-                 cudaStream_t s);
-// The driver entry point and kernel attributes the tensor-core GEMM needs are available.
-bool tc_gemm_ready(bool tf32);
+             cudaStream_t s, float* part, size_t part_elems);
+// The driver entry point the tensor loads need is available.
+bool tc_gemm_ready();
 // C [M x N] = A_hi B_hi^T + A_hi B_lo^T + A_lo B_hi^T with the TF32 split of the FP32 operand A done in
 // shared memory (B_hi, B_lo exact TF32 values, N <= 256 per tile column); FP32 result, row length ldo.
 bool tc_split_gemm(int M, int N, int K, const float* A, int lda, const float* Bhi, const float* Blo, int ldb,

@@ -1,28 +1,30 @@
-// GEMM on the 5th-generation tensor cores: C = sum_p A_p B_p^T (one to three
-// operand pairs in one accumulator) with A_p [M x K] and B_p [N x K], both
-// row-major (K contiguous), BF16 (kind::f16) or TF32 (kind::tf32) operands and
-// FP32 accumulation in tensor memory.  Used by the learned closure's MLP
-// (hx_mlp.cu; BF16, one pair, fused bias / GELU epilogues) and by the dense-H
-// stage (hx_ctx.cu; TF32, the three pairs of a split product, plain store).
-// No counterpart in the reference.
+// GEMMs on the 5th-generation tensor cores.  tc_gemm: C = A B^T with A [M x K]
+// and B [N x K], both row-major (K contiguous), BF16 operands (kind::f16) and
+// FP32 accumulation in tensor memory: the learned closure's MLP (hx_mlp.cu),
+// fused bias / GELU epilogues.  tc_split_gemm: the dense-H stage's TF32 split
+// product (below).  No counterpart in the reference.
 //
-// One CTA of four warps computes a 128 x BN tile of C (BN = 256 when N >=
-// 256, else 128; 1-D grid, N tiles fastest):
+// One CTA of eight warps computes a 128 x BN tile of C (BN = 256 when that
+// still gives every SM a tile, else 128; N tiles fastest):
 //  * warp 0 allocates BN tensor-memory columns (the 128 x BN FP32
 //    accumulator, one lane per row) and its lane 0 streams the K blocks of
-//    every pair (128 bytes of each of the 128 rows of A and BN rows of B: 64
-//    BF16 or 32 TF32) into a 192 KB shared-memory ring (6 stages at BN = 128,
+//    its split (128 bytes, 64 values, of each of the 128 rows of A and BN rows
+//    of B) into a 192 KB shared-memory ring (6 stages at BN = 128,
 //    4 at 256) with TMA tensor loads in the 128-byte swizzled layout;
 //  * lane 0 of warp 1 issues tcgen05.mma (M = 128, N = BN, 32 bytes of K per
-//    instruction: K = 16 BF16 or 8 TF32; four per K block, the shared-memory
+//    instruction: K = 16; four per K block, the shared-memory
 //    descriptor advanced by 32 bytes inside the swizzle atom) and returns each
 //    stage to the producer with tcgen05.commit on that stage's mbarrier;
 //  * after the last block a commit signals the accumulator complete; every
-//    warp reads its 32 lanes with tcgen05.ld (16 columns at a time) into a
-//    padded shared-memory tile over the drained ring, and the CTA then stores
-//    row after row of C with consecutive threads on consecutive columns,
-//    applying the epilogue (bias + GELU keeping the pre-activation, bias,
-//    plain store, or GELU backward).
+//    warp reads its 32 lanes with tcgen05.ld (16 columns at a time; warps 4-7
+//    take the other half of the columns) and applies the epilogue in registers
+//    (bias + GELU keeping the pre-activation, bias, plain store, or GELU
+//    backward): a lane stores 64 bytes of one row, whole sectors.  Through
+//    shared memory with four warps the epilogue of a 4096 x 512 GELU layer took
+//    most of 85 us; now the layer takes 19;
+//  * blockIdx.y splits K where the tiles alone leave SMs idle (the weight
+//    gradients: 512 x 512 outputs, K = the batch): every split writes its FP32
+//    sums, tc_reduce_kernel adds them in order.
 // Out-of-range rows, columns and K are zero-filled by the tensor loads and
 // masked at the stores.  Every mbarrier wait is bounded: a wait that runs
 // out sets the error word, the kernel still waits (bounded) for its copies
@@ -33,6 +35,8 @@
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
 
+#include <algorithm>
+#include <atomic>
 #include <cstdint>
 
 #include "hx_internal.h"
@@ -54,7 +58,6 @@ struct TileCfg {
     static constexpr int kStages = BN == 128 ? 6 : 4;  // a 192 KB ring either way
     static constexpr uint32_t kRing = kStages * kStageBytes;
     static constexpr uint32_t kSmem = kRing + 1024 + 256;
-    static_assert(kBM * (BN + 1) * 4 <= kRing, "the epilogue tile reuses the ring");
     static_assert(kSmem <= 227 * 1024, "shared memory per CTA");
 };
 
@@ -64,13 +67,6 @@ __host__ __device__ constexpr uint32_t idesc_of(uint32_t fmt, int bn)
 {
     return (1u << 4) | (fmt << 7) | (fmt << 10) | (uint32_t(bn >> 3) << 17) | (uint32_t(kBM >> 4) << 24);
 }
-
-// Tensor maps of up to three operand pairs; the kernel accumulates the sum of
-// their products A_p B_p^T (the terms of a split-precision product).
-struct TcMaps {
-    CUtensorMap a[3];
-    CUtensorMap b[3];
-};
 
 __device__ __forceinline__ uint32_t saddr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
@@ -133,15 +129,16 @@ __device__ __forceinline__ float gelu_grad_f(float z)
     return cdf + z * pdf;
 }
 
-template <bool TF32, int BN>
-__global__ void __launch_bounds__(128, 1)
-    tc_gemm_kernel(const __grid_constant__ TcMaps maps, int M, int N, int K, int npairs, TcGemmOut o, int* err)
+template <int BN>
+__global__ void __launch_bounds__(256, 1)
+    tc_gemm_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, int M, int N,
+                   int K, TcGemmOut o, int* err)
 {
     using Cfg = TileCfg<BN>;
     constexpr int kStages = Cfg::kStages;
     constexpr uint32_t kStageBytes = Cfg::kStageBytes;
-    constexpr int kBK = TF32 ? 32 : 64;  // K elements per 128-byte row
-    constexpr uint32_t kIdesc = idesc_of(TF32 ? 2u : 1u, BN);
+    constexpr int kBK = 64;  // K elements per 128-byte row
+    constexpr uint32_t kIdesc = idesc_of(1u, BN);
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = saddr(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;  // swizzled tiles need 1024-byte alignment
@@ -156,8 +153,10 @@ __global__ void __launch_bounds__(128, 1)
     // 1-D grid, N tiles fastest: the CTAs that share a row block of A run together and read it once from HBM
     const int ntn = (N + BN - 1) / BN;
     const int m0 = static_cast<int>(blockIdx.x / ntn) * kBM, n0 = static_cast<int>(blockIdx.x % ntn) * BN;
-    const int nkp = (K + kBK - 1) / kBK;  // K blocks of one operand pair
-    const int nk = nkp * npairs;
+    // this split's K blocks (every split has at least one)
+    const int nkb = (K + kBK - 1) / kBK;
+    const int kb0 = static_cast<int>(static_cast<long long>(nkb) * blockIdx.y / gridDim.y);
+    const int nk = static_cast<int>(static_cast<long long>(nkb) * (blockIdx.y + 1) / gridDim.y) - kb0;
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) {
@@ -196,9 +195,9 @@ __global__ void __launch_bounds__(128, 1)
                 asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(full_bar(s)),
                              "r"(kStageBytes)
                              : "memory");
-                const int p = kb / nkp, x = (kb - p * nkp) * kBK;
-                tma_load_2d(a, &maps.a[p], x, m0, full_bar(s));
-                tma_load_2d(b, &maps.b[p], x, n0, full_bar(s));
+                const int x = (kb0 + kb) * kBK;
+                tma_load_2d(a, &map_a, x, m0, full_bar(s));
+                tma_load_2d(b, &map_b, x, n0, full_bar(s));
                 issued = kb + 1;
             }
         }
@@ -219,14 +218,7 @@ __global__ void __launch_bounds__(128, 1)
                 for (int k = 0; k < 4; ++k) {  // 32 bytes of K per instruction (16 BF16 or 8 TF32)
                     const uint64_t da = sw128_desc(a + 32u * k), db = sw128_desc(b + 32u * k);
                     const uint32_t accumulate = (kb > 0 || k > 0) ? 1u : 0u;
-                    if constexpr (TF32)
-                        asm volatile(
-                            "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-                            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
-                            "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate)
-                            : "memory");
-                    else
-                        asm volatile(
+                    asm volatile(
                             "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
                             "l"(da), "l"(db), "r"(kIdesc), "r"(accumulate)
@@ -240,9 +232,7 @@ __global__ void __launch_bounds__(128, 1)
         __syncwarp();
     }
 
-    // ---- epilogue: the accumulator goes through shared memory (the ring is
-    // free once every MMA has completed and every copy has landed) so that
-    // each row of C is stored by consecutive threads
+    // ---- epilogue, 16 columns of one row per lane at a time
     const bool done = mbar_wait(done_bar, 0);
     if (!done && threadIdx.x == 0) atomicExch(err, 1);
     if (warp == 0 && lane == 0) {
@@ -250,48 +240,74 @@ __global__ void __launch_bounds__(128, 1)
         asm volatile("ld.shared.u32 %0, [%1];" : "=r"(consumed) : "r"(cslot) : "memory");
         for (int kb = consumed; kb < issued; ++kb) mbar_wait(full_bar(kb % kStages), (kb / kStages) & 1);
     }
+    __syncwarp();
     tc_fence_after();
-    __syncthreads();
-    float* stile = reinterpret_cast<float*>(smem_raw + (base - raw));  // [128][BN + 1]
-    constexpr int kLd = BN + 1;
-    const int trow = warp * 32 + lane;
-    for (int c0 = 0; c0 < BN; c0 += 16) {
+    const int quad = warp & 3, half = warp >> 2;
+    const int row = m0 + quad * 32 + lane;
+    float* outf = o.outf ? o.outf + static_cast<long long>(blockIdx.y) * M * N : nullptr;  // (one split: the result)
+    const bool has_bias = o.kind == kTcEpiBiasGelu || o.kind == kTcEpiBias;
+    // 16-byte accesses need every row to start on a 16-byte boundary
+    const bool wide = o.ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(outf) | reinterpret_cast<uintptr_t>(o.outh) |
+                                         reinterpret_cast<uintptr_t>(o.aux)) % 16 == 0;
+    for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
         uint32_t v[16];
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
             "%14, %15}, [%16];"
             : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
               "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-            : "r"(tmem + (static_cast<uint32_t>(warp * 32) << 16) + static_cast<uint32_t>(c0)));
+            : "r"(tmem + (static_cast<uint32_t>(quad * 32) << 16) + static_cast<uint32_t>(c0)));
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        const int col = n0 + c0;
+        if (!done || row >= M || col >= N) continue;
+        const long long off = static_cast<long long>(row) * o.ldo + col;
+        const int cnt = min(16, N - col);
+        float f[16], h[16], x[16];
+        const bool vec = wide && cnt == 16;
+        if (o.kind == kTcEpiGeluBack) {
+            if (vec) {
 #pragma unroll
-        for (int jj = 0; jj < 16; ++jj) stile[trow * kLd + c0 + jj] = __uint_as_float(v[jj]);
-    }
-    __syncthreads();
-    if (done) {
-        for (int cc = static_cast<int>(threadIdx.x); cc < BN; cc += 128) {
-            const int col = n0 + cc;
-            if (col >= N) break;
-            const float bias = (o.kind == kTcEpiBiasGelu || o.kind == kTcEpiBias) ? o.bias[col] : 0.0f;
-            for (int rr = 0; rr < kBM; ++rr) {
-                const int row = m0 + rr;
-                if (row >= M) break;
-                const float val = stile[rr * kLd + cc];
-                const long long off = static_cast<long long>(row) * o.ldo + col;
-                if (o.kind == kTcEpiBiasGelu) {
-                    const float z = val + bias;
-                    o.outf[off] = z;
-                    static_cast<__nv_bfloat16*>(o.outh)[off] = __float2bfloat16(gelu_f(z));
-                } else if (o.kind == kTcEpiBias) {
-                    o.outf[off] = val + bias;
-                } else if (o.kind == kTcEpiStore) {
-                    o.outf[off] = val;
-                } else {
-                    const float g = val * gelu_grad_f(o.aux[off]);
-                    static_cast<__nv_bfloat16*>(o.outh)[off] = __float2bfloat16(g);
-                    if (o.outf) o.outf[off] = g;
+                for (int i = 0; i < 4; ++i) {
+                    const float4 t = *reinterpret_cast<const float4*>(o.aux + off + 4 * i);
+                    x[4 * i] = t.x;
+                    x[4 * i + 1] = t.y;
+                    x[4 * i + 2] = t.z;
+                    x[4 * i + 3] = t.w;
                 }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 16; ++i) x[i] = i < cnt ? o.aux[off + i] : 0.0f;
             }
+        }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+            f[i] = __uint_as_float(v[i]);
+            if (has_bias) f[i] += i < cnt ? __ldg(o.bias + col + i) : 0.0f;
+            if (o.kind == kTcEpiGeluBack) f[i] *= gelu_grad_f(x[i]);
+            h[i] = o.kind == kTcEpiBiasGelu ? gelu_f(f[i]) : f[i];
+        }
+        __nv_bfloat16* outh = static_cast<__nv_bfloat16*>(o.outh);
+        const bool with_h = o.kind == kTcEpiBiasGelu || o.kind == kTcEpiGeluBack;
+        if (vec) {
+            if (outf)
+#pragma unroll
+                for (int i = 0; i < 4; ++i)
+                    *reinterpret_cast<float4*>(outf + off + 4 * i) = make_float4(f[4 * i], f[4 * i + 1], f[4 * i + 2], f[4 * i + 3]);
+            if (with_h)
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    __align__(16) __nv_bfloat16 b[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) b[q] = __float2bfloat16(h[8 * i + q]);
+                    *reinterpret_cast<uint4*>(outh + off + 8 * i) = *reinterpret_cast<const uint4*>(b);
+                }
+        } else {
+#pragma unroll
+            for (int i = 0; i < 16; ++i)
+                if (i < cnt) {
+                    if (outf) outf[off + i] = f[i];
+                    if (with_h) outh[off + i] = __float2bfloat16(h[i]);
+                }
         }
     }
     tc_fence_before();
@@ -560,6 +576,17 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
     }
 }
 
+// out[m][n] = sum over the splits of part[split][m][n], in order.
+__global__ void tc_reduce_kernel(const float* __restrict__ part, int splits, long long mn, int N, int ldo, float* out)
+{
+    for (long long i = blockIdx.x * 256ll + threadIdx.x; i < mn; i += gridDim.x * 256ll) {
+        float t = 0.0f;
+#pragma unroll 8
+        for (int s = 0; s < splits; ++s) t += __ldg(part + s * mn + i);
+        out[i / N * ldo + i % N] = t;
+    }
+}
+
 // Row-major BF16 transpose: out[c][r] = in[r][c] for rows x cols.
 __global__ void transpose_bf16_kernel(const __nv_bfloat16* __restrict__ in, int rows, int cols, int ld_in,
                                       __nv_bfloat16* __restrict__ out, int ld_out)
@@ -607,27 +634,23 @@ bool make_map(CUtensorMap* map, const void* ptr, int rows, int cols, int ld, boo
               CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <bool TF32, int BN>
+template <int BN>
 bool configure()
 {
-    static bool configured[64] = {};
+    static std::atomic<bool> configured[64];
     int dev = 0;
     cudaGetDevice(&dev);
     if (dev < 0 || dev >= 64) return false;
-    if (!configured[dev]) {
-        if (cudaFuncSetAttribute(tc_gemm_kernel<TF32, BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (!configured[dev].load()) {
+        if (cudaFuncSetAttribute(tc_gemm_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  static_cast<int>(TileCfg<BN>::kSmem)) != cudaSuccess)
             return false;
-        configured[dev] = true;
+        configured[dev].store(true);
     }
     return true;
 }
 
-template <bool TF32>
-bool configure_all()
-{
-    return configure<TF32, 128>() && configure<TF32, 256>();
-}
+bool configure_all() { return configure<128>() && configure<256>(); }
 
 bool eligible(const void* A, int lda, const void* B, int ldb, int esize)
 {
@@ -638,41 +661,48 @@ bool eligible(const void* A, int lda, const void* B, int ldb, int esize)
 
 }  // namespace
 
-bool tc_gemm_eligible(const void* A, int lda, const void* B, int ldb) { return eligible(A, lda, B, ldb, 2); }
-
-bool tc_gemm_ready(bool tf32) { return encode_fn() != nullptr && (tf32 ? configure_all<true>() : configure_all<false>()); }
+bool tc_gemm_ready() { return encode_fn() != nullptr; }
 
 bool tc_gemm(int M, int N, int K, const void* A, int lda, const void* B, int ldb, const TcGemmOut& o, int* err,
-             cudaStream_t s)
+             cudaStream_t s, float* part, size_t part_elems)
 {
-    const TcPair pair{A, lda, B, ldb};
-    return tc_gemm_sum(M, N, K, 1, &pair, false, o, err, s);
-}
-
-bool tc_gemm_sum(int M, int N, int K, int npairs, const TcPair* pairs, bool tf32, const TcGemmOut& o, int* err,
-                 cudaStream_t s)
-{
-    if (M <= 0 || N <= 0 || K <= 0 || npairs < 1 || npairs > 3) return false;
-    for (int p = 0; p < npairs; ++p)
-        if (!eligible(pairs[p].A, pairs[p].lda, pairs[p].B, pairs[p].ldb, tf32 ? 4 : 2)) return false;
-    if (!(tf32 ? configure_all<true>() : configure_all<false>())) return false;
-    const int bn = N >= 256 ? 256 : 128;  // wide tiles halve the re-reads of A
-    TcMaps maps;
-    for (int p = 0; p < npairs; ++p)
-        if (!make_map(&maps.a[p], pairs[p].A, M, K, pairs[p].lda, tf32, kBM) ||
-            !make_map(&maps.b[p], pairs[p].B, N, K, pairs[p].ldb, tf32, bn))
-            return false;
-    const long long tiles = static_cast<long long>((N + bn - 1) / bn) * ((M + kBM - 1) / kBM);
+    if (M <= 0 || N <= 0 || K <= 0) return false;
+    if (!eligible(A, lda, B, ldb, 2) || !configure_all()) return false;
+    const int dev = [] {
+        int d = 0;
+        return cudaGetDevice(&d) == cudaSuccess && d >= 0 && d < 64 ? d : -1;
+    }();
+    static std::atomic<int> sm_count[64];
+    if (dev < 0) return false;
+    int sms = sm_count[dev].load();
+    if (sms == 0) {
+        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return false;
+        sm_count[dev].store(sms);
+    }
+    auto tiles_of = [&](int bn) { return static_cast<long long>((N + bn - 1) / bn) * ((M + kBM - 1) / kBM); };
+    const int bn = tiles_of(256) >= sms ? 256 : 128;  // wide tiles halve the re-reads of A, if every SM gets one
+    const long long tiles = tiles_of(bn);
     if (tiles > 0x7fffffffll) return false;
-    const dim3 grid(static_cast<unsigned>(tiles));
-    if (tf32 && bn == 256)
-        tc_gemm_kernel<true, 256><<<grid, 128, TileCfg<256>::kSmem, s>>>(maps, M, N, K, npairs, o, err);
-    else if (tf32)
-        tc_gemm_kernel<true, 128><<<grid, 128, TileCfg<128>::kSmem, s>>>(maps, M, N, K, npairs, o, err);
-    else if (bn == 256)
-        tc_gemm_kernel<false, 256><<<grid, 128, TileCfg<256>::kSmem, s>>>(maps, M, N, K, npairs, o, err);
-    else
-        tc_gemm_kernel<false, 128><<<grid, 128, TileCfg<128>::kSmem, s>>>(maps, M, N, K, npairs, o, err);
+    // plain sums over a long K: as many splits as fill the GPU, at least four K blocks each
+    long long splits = 1;
+    const size_t mn = static_cast<size_t>(M) * N;
+    if (o.kind == kTcEpiStore && part && o.outf) {
+        splits = std::min<long long>({sms / std::max<long long>(tiles, 1), K / 256, static_cast<long long>(part_elems / mn)});
+        splits = std::max<long long>(splits, 1);
+    }
+    CUtensorMap ma, mb;
+    if (!make_map(&ma, A, M, K, lda, false, kBM) || !make_map(&mb, B, N, K, ldb, false, bn)) return false;
+    const dim3 grid(static_cast<unsigned>(tiles), static_cast<unsigned>(splits));
+    TcGemmOut to = o;
+    if (splits > 1) {
+        to.outf = part;
+        to.ldo = N;
+    }
+    if (bn == 256) tc_gemm_kernel<256><<<grid, 256, TileCfg<256>::kSmem, s>>>(ma, mb, M, N, K, to, err);
+    else tc_gemm_kernel<128><<<grid, 256, TileCfg<128>::kSmem, s>>>(ma, mb, M, N, K, to, err);
+    if (splits > 1)
+        tc_reduce_kernel<<<static_cast<unsigned>(std::min<size_t>((mn + 255) / 256, 148 * 8)), 256, 0, s>>>(
+            part, static_cast<int>(splits), static_cast<long long>(mn), N, o.ldo, o.outf);
     return true;
 }
 

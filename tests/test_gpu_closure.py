@@ -264,3 +264,30 @@ def test_closure_at_the_c5_size():
     print(f"closure gains at the C5 size: {gains}")
     assert np.mean(gains) >= 2.0, gains
     cl.close()
+
+
+@pytest.mark.parametrize("rows,inp,hidden,out", [
+    (1, 8, 32, 2), (127, 21, 96, 2), (513, 40, 200, 7), (1024, 64, 256, 130), (4096, 21, 512, 2),
+])
+def test_mlp_gradients_over_tile_edges(rows, inp, hidden, out):
+    """Loss and gradients at ragged rows and widths (tiles, split sums of the
+    weight gradients, chunks of the bias gradients) against the FP64
+    restatement with the same BF16 rounding points; bar as in the other
+    gradient test."""
+    rng = np.random.default_rng(rows + out)
+    net = capi.MLP(inp, hidden, out, seed=3)
+    x = rng.uniform(-1, 1, (rows, inp)).astype(np.float32)
+    t = rng.uniform(-1, 1, (rows, out)).astype(np.float32)
+    loss, g = net.gradients(x, t)
+    again = net.gradients(x, t)
+    assert loss == again[0] and np.array_equal(g, again[1])  # fixed summation order
+    _, want_loss, want = MO.forward_backward(net.params().astype(np.float64), x.astype(np.float64), t.astype(np.float64),
+                                             inp, hidden, out, bf16=True)
+    assert abs(loss - want_loss) <= 1e-3 * want_loss
+    off = 0
+    for name, size in [("W1", hidden * inp), ("b1", hidden), ("W2", hidden * hidden), ("b2", hidden), ("W3", out * hidden),
+                       ("b3", out)]:
+        gg, rr = g[off:off + size], want[off:off + size]
+        assert np.max(np.abs(gg - rr)) <= 2e-2 * np.max(np.abs(rr)), name
+        off += size
+    net.close()
