@@ -518,34 +518,37 @@ __global__ void batch_gsum_kernel(const int32_t* rows, const int32_t* bath_off, 
 }
 
 // trace[*counter % cap] = sum over instances of Tr(sigma_z(spin) rho_0); then ++*counter.
-// One block of 256 threads; fixed summation order, so the result does not depend on timing.
+// One block, a warp per instance at a time (a thread per instance waited on its diagonal
+// elements one after the other: 23 us for 128 instances, OBSB with the lanes on the diagonal);
+// fixed summation order, so the result does not depend on timing.
 // logd[i] carries bit 8 when instance i keeps Hermitian-packed slabs.
-__global__ void batch_obs_kernel(const double2* const* rho0, const int* logd, int count, int spin, double* trace,
-                                 int* counter, int cap)
+constexpr int kObsWarps = 32;
+
+__global__ void __launch_bounds__(kObsWarps * 32)
+    batch_obs_kernel(const double2* const* rho0, const int* logd, int count, int spin, double* trace, int* counter,
+                     int cap)
 {
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     double s = 0.0;
-    for (int i = threadIdx.x; i < count; i += blockDim.x) {
-        const int lg = logd[i] & 0xff;
-        const bool herm = (logd[i] >> 8) & 1;
-        const int D = 1 << lg;
+#pragma unroll 2
+    for (int i = warp; i < count; i += kObsWarps) {
+        const int lg = __ldg(logd + i) & 0xff;
+        const bool herm = (__ldg(logd + i) >> 8) & 1;
         const double2* r0 = rho0[i];
-        double v = 0.0;
-        for (int r = 0; r < D; ++r) {
-            const double d = r0[herm ? herm_index(r, r, lg) : static_cast<long long>(r) * D + r].x;
-            v += ((r >> spin) & 1) ? d : -d;
+        for (int r = lane; r < (1 << lg); r += 32) {
+            const double d = r0[herm ? herm_index(r, r, lg) : (static_cast<long long>(r) << lg) + r].x;
+            s += ((r >> spin) & 1) ? d : -d;
         }
-        s += v;
     }
-    __shared__ double red[256];
-    red[threadIdx.x] = s;
+    for (int off = 16; off > 0; off >>= 1) s += __shfl_down_sync(0xffffffffu, s, off);
+    __shared__ double red[kObsWarps];
+    if (lane == 0) red[warp] = s;
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if (threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
     if (threadIdx.x == 0) {
+        double v = 0.0;
+        for (int w = 0; w < kObsWarps; ++w) v += red[w];
         const int t = *counter;
-        trace[t % cap] = red[0];
+        trace[t % cap] = v;
         *counter = t + 1;
     }
 }
@@ -626,7 +629,7 @@ struct hx_batch {
     double* trace = nullptr;
     int* trace_counter = nullptr;
     int trace_cap = 0;
-    double* pinned = nullptr;
+    double* pinned = nullptr;          // trace staging [kTraceCap], then the error word
     size_t device_bytes = 0;
     // instances with d >= 32 run as internal contexts through the fused and
     // up-term kernels on forked streams of the captured step
@@ -788,6 +791,19 @@ int set_tile_shape(hx_batch* b, int lg, int tile_elems, int variant)
     return HX_OK;
 }
 
+// The shape without the autotuner: the tile size the caller asks for, else one
+// element per thread and three CTAs per SM on tiles of 1024 elements (512 below
+// d = 16, whose ADOs are many and small).  ms per step of 128 instances with up
+// to 4 spins, tiles of 2048 elements with two elements per thread (one CTA of
+// nine warps per SM) against this: 2.20 and BATCH4; up to 3 spins: 0.46 and
+// BATCH3.
+int default_tile_shape(hx_batch* b, int lg, int tile_elems)
+{
+    if (tile_elems > 0) return set_tile_shape(b, lg, tile_elems, 1);
+    if (lg > 4) return set_tile_shape(b, lg, 2048, 1);
+    return set_tile_shape(b, lg, lg == 4 ? 1024 : 512, 2);
+}
+
 void launch_class_stage(hx_batch* b, int lg, const double2* u, double2* out, double alpha, int base, cudaStream_t s)
 {
     const hx_batch::Class& c = b->cls[lg];
@@ -856,7 +872,7 @@ void enqueue_batch_step(hx_batch* b, cudaStream_t s)
             in = out;
         }
     }
-    hx::batch_obs_kernel<<<1, 256, 0, s>>>(b->rho0_ptr, b->logd_arr, b->count, b->spin, b->trace, b->trace_counter,
+    hx::batch_obs_kernel<<<1, hx::kObsWarps * 32, 0, s>>>(b->rho0_ptr, b->logd_arr, b->count, b->spin, b->trace, b->trace_counter,
                                           b->trace_cap);
 }
 
@@ -872,16 +888,29 @@ int ensure_graph(hx_batch* b)
     return HX_OK;
 }
 
-int batch_check_flag(hx_batch* b)
+// Error word: its copy travels with a result's, batch_flag looks at it after the wait.
+int batch_enqueue_flag(hx_batch* b)
 {
-    int flag = 0;
-    HX_CUDA_TRY(cudaMemcpyAsync(&flag, b->error_flag, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
-    HX_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    HX_CUDA_TRY(cudaMemcpyAsync(b->pinned + kTraceCap, b->error_flag, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
+    return HX_OK;
+}
+
+int batch_flag(hx_batch* b)
+{
+    int flag;
+    std::memcpy(&flag, b->pinned + kTraceCap, sizeof(int));
     if (flag) {
         cudaMemsetAsync(b->error_flag, 0, sizeof(int), b->stream);
         return fail(HX_ERR_DEVICE_TIMEOUT, "a device-side wait ran out of its iteration budget");
     }
     return HX_OK;
+}
+
+int batch_check_flag(hx_batch* b)
+{
+    if (int rc = batch_enqueue_flag(b)) return rc;
+    HX_CUDA_TRY(cudaStreamSynchronize(b->stream));
+    return batch_flag(b);
 }
 
 // Streams of the context instances (groups balanced by state size, largest
@@ -1131,7 +1160,7 @@ int hx_batch_create(const hx_problem* problems, uint32_t count, const hx_batch_o
         (rc = balloc(b, &b->trace_counter, 1)) || (rc = balloc(b, &b->trace, kTraceCap)))
         return bail(rc);
     b->trace_cap = kTraceCap;
-    e = cudaMallocHost(&b->pinned, kTraceCap * sizeof(double));
+    e = cudaMallocHost(&b->pinned, (kTraceCap + 1) * sizeof(double));
     if (e == cudaSuccess) e = cudaMalloc(&ddsrc, dsrc.size() * sizeof(double));
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(b->blk, blk.data(), blk.size() * sizeof(double), cudaMemcpyHostToDevice, b->stream);
@@ -1215,7 +1244,7 @@ int hx_batch_create(const hx_problem* problems, uint32_t count, const hx_batch_o
     // streams and arguments of the context instances, and the observable's pointer table
     if ((rc = build_context_launches(b)) != HX_OK) return bail(rc);
     for (int lg = 1; lg <= hx::kMaxBatchLogD; ++lg)
-        if ((rc = set_tile_shape(b, lg, te, 1)) != HX_OK) return bail(rc);
+        if ((rc = default_tile_shape(b, lg, opt ? static_cast<int>(opt->tile_elems) : 0)) != HX_OK) return bail(rc);
     if (opt && opt->tune) {
         uint32_t a = 0, c = 0;
         if ((rc = hx_batch_tune(b, &a, &c)) != HX_OK) return bail(rc);
@@ -1322,6 +1351,7 @@ int hx_batch_step(hx_batch* b, uint64_t nsteps, double* sz_sum_trace)
         b->launches += static_cast<uint64_t>(chunk) * (b->order * kernels_per_stage(b) + 1);
         if (sz_sum_trace) {
             HX_CUDA_TRY(cudaMemcpyAsync(b->pinned, b->trace, chunk * sizeof(double), cudaMemcpyDeviceToHost, b->stream));
+            if ((rc = batch_enqueue_flag(b)) != HX_OK) return rc;
             HX_CUDA_TRY(cudaStreamSynchronize(b->stream));
             std::memcpy(sz_sum_trace + done, b->pinned, chunk * sizeof(double));
         }
@@ -1329,7 +1359,7 @@ int hx_batch_step(hx_batch* b, uint64_t nsteps, double* sz_sum_trace)
     }
     b->steps_done += nsteps;
     if (!sz_sum_trace) return HX_OK;
-    return batch_check_flag(b);
+    return nsteps > 0 ? batch_flag(b) : batch_check_flag(b);
 }
 
 int hx_batch_sync(hx_batch* b)
@@ -1351,12 +1381,11 @@ int hx_batch_read_rho0(hx_batch* b, uint32_t instance, double* out, uint64_t n)
     if (k >= 0 && b->ctxs[k]->herm) {
         std::vector<double2> pk(b->ctxs[k]->slab_store);
         HX_CUDA_TRY(cudaMemcpyAsync(pk.data(), src, pk.size() * sizeof(double2), cudaMemcpyDeviceToHost, b->stream));
-        HX_CUDA_TRY(cudaStreamSynchronize(b->stream));
+        const int rc = batch_check_flag(b);
         hx::unpack_herm_host(pk.data(), in.logd, out);
-        return batch_check_flag(b);
+        return rc;
     }
     HX_CUDA_TRY(cudaMemcpyAsync(out, src, d2 * sizeof(double2), cudaMemcpyDeviceToHost, b->stream));
-    HX_CUDA_TRY(cudaStreamSynchronize(b->stream));
     return batch_check_flag(b);
 }
 

@@ -309,7 +309,7 @@ typedef struct hx_batch hx_batch;
 typedef struct hx_batch_options {
     uint32_t observable_spin; /* spin whose <sigma_z> is averaged (bit index), default 0 */
     uint32_t tune;            /* 1 = run the tile-shape autotuner at creation */
-    uint32_t tile_elems;      /* elements per tile (power of two, 64..8192); 0 = 2048 */
+    uint32_t tile_elems;      /* elements per tile (power of two, 64..8192); 0 = by dimension */
     uint32_t threads;         /* threads per CTA (multiple of 32, 64..1024); 0 = 256 */
 } hx_batch_options;
 
