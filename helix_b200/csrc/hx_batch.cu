@@ -519,7 +519,7 @@ __global__ void batch_gsum_kernel(const int32_t* rows, const int32_t* bath_off, 
 
 // trace[*counter % cap] = sum over instances of Tr(sigma_z(spin) rho_0); then ++*counter.
 // One block, a warp per instance at a time (a thread per instance waited on its diagonal
-// elements one after the other: 23 us for 128 instances, OBSB with the lanes on the diagonal);
+// elements one after the other: 23 us for 128 instances, 7 with the lanes on the diagonal);
 // fixed summation order, so the result does not depend on timing.
 // logd[i] carries bit 8 when instance i keeps Hermitian-packed slabs.
 constexpr int kObsWarps = 32;
@@ -795,8 +795,8 @@ int set_tile_shape(hx_batch* b, int lg, int tile_elems, int variant)
 // element per thread and three CTAs per SM on tiles of 1024 elements (512 below
 // d = 16, whose ADOs are many and small).  ms per step of 128 instances with up
 // to 4 spins, tiles of 2048 elements with two elements per thread (one CTA of
-// nine warps per SM) against this: 2.20 and BATCH4; up to 3 spins: 0.46 and
-// BATCH3.
+// nine warps per SM) against this: 2.20 and 1.30; up to 3 spins: 0.46 and
+// 0.28.
 int default_tile_shape(hx_batch* b, int lg, int tile_elems)
 {
     if (tile_elems > 0) return set_tile_shape(b, lg, tile_elems, 1);

@@ -307,7 +307,10 @@ __global__ void __launch_bounds__(256, MINB)
 // operator is sigma_z of one spin: v_r = +1 or -1 from a bit of r, and of
 // [V, X] and {V, X} exactly one is nonzero at each element.
 template <int LOGD> struct HermShape;
-template <> struct HermShape<5> { static constexpr int T = 192, MINB = 4; };  // 528 elements: 3 per thread
+// 528 elements: 3 per thread.  The d = 32 kernel waits on latency rather than on a unit:
+// five CTAs per SM (64 registers) carry a batch of 128 instances in 4.08 ms per step, four
+// in 4.59, six (56 registers, spilling without PAULI) in 4.07.
+template <> struct HermShape<5> { static constexpr int T = 192, MINB = 5; };
 template <> struct HermShape<6> { static constexpr int T = 416, MINB = 2; };  // 2080 elements: 5 per thread
 
 constexpr unsigned kPrefetchAhead = 148;  // CTAs per resident wave per unit of HermShape::MINB
