@@ -298,6 +298,14 @@ __global__ void __launch_bounds__(256, MINB)
 //
 // The CTA unpacks its own slab into a full d x d copy in shared memory for
 // the transverse-field flips, element (r, c) in slot r d + (c ^ (r & 7)).
+// A thread loads its elements itself, writes them and their mirrors, and goes
+// on to the neighbour entries at once; the flips come last, behind the second
+// of two barriers, when every warp's part has long arrived.  (A bulk copy of
+// the packed slab that all warps waited for, flips first, needed a second
+// buffer in shared memory: 1374 us a step at d = 64, 7315 ADOs, against 1340
+// with the L1 cache the buffer leaves free, and 801 against 772 at d = 32,
+// 15504 ADOs.)  Bound by the load-store unit: 65% of its wavefronts, three
+// quarters of them shared memory, at 2.7 TB/s of DRAM traffic.
 // With that swizzle every flip is one XOR of the slot with a constant
 // (row bit b: d 2^b, plus 2^b when b < 3; column bit b: 2^b), and the
 // accesses stay free of bank conflicts: a run of consecutive columns of one
@@ -307,11 +315,12 @@ __global__ void __launch_bounds__(256, MINB)
 // operator is sigma_z of one spin: v_r = +1 or -1 from a bit of r, and of
 // [V, X] and {V, X} exactly one is nonzero at each element.
 template <int LOGD> struct HermShape;
-// 528 elements: 3 per thread.  The d = 32 kernel waits on latency rather than on a unit:
-// five CTAs per SM (64 registers) carry a batch of 128 instances in 4.08 ms per step, four
-// in 4.59, six (56 registers, spilling without PAULI) in 4.07.
-template <> struct HermShape<5> { static constexpr int T = 192, MINB = 5; };
-template <> struct HermShape<6> { static constexpr int T = 416, MINB = 2; };  // 2080 elements: 5 per thread
+// d = 32: 528 elements, d = 64: 2080.  E elements per thread.  At d = 32 six CTAs of 56 registers: a step of
+// a batch of 128 instances took 4.59 ms with four CTAs per SM, 4.08 with five or six; two elements in 288
+// threads 9% longer.  At d = 64 26 warps of 72 registers: 544 threads of 4 elements 2% longer, three CTAs of
+// 288 threads (two passes of 4) 8%.
+template <> struct HermShape<5> { static constexpr int T = 192, MINB = 6, E = 3; };
+template <> struct HermShape<6> { static constexpr int T = 416, MINB = 2, E = 5; };
 
 constexpr unsigned kPrefetchAhead = 148;  // CTAs per resident wave per unit of HermShape::MINB
 
@@ -326,13 +335,12 @@ __device__ __forceinline__ void herm_ado(const FusedArgs& a, long long n, const 
                                          const double2* rho, double2* out, double alpha, int base_kind)
 {
     constexpr int D = 1 << LOGD, HALF = D / 2, P = HALF * (D + 1);
-    constexpr int T = HermShape<LOGD>::T, E = (P + T - 1) / T;
-    constexpr bool kExact = (P % T) == 0;
+    constexpr int T = HermShape<LOGD>::T, E = HermShape<LOGD>::E;
+    constexpr bool kExact = P == T * E;
+    static_assert(P <= T * E);
     extern __shared__ __align__(128) unsigned char smem[];
-    double2* full = reinterpret_cast<double2*>(smem);  // [D * D] own slab, unpacked and swizzled
-    double2* pk = full + D * D;                         // [P] own packed slab, then the packed rho slab
-    uint64_t* bar = reinterpret_cast<uint64_t*>(pk + P);
-    double* sV = reinterpret_cast<double*>(bar + 2);   // [J][D] (general couplings)
+    double2* full = reinterpret_cast<double2*>(smem);       // [D * D] own slab, unpacked and swizzled
+    double* sV = reinterpret_cast<double*>(full + D * D);  // [J][D] (general couplings)
     double* sH = sV + a.J * D;                          // [LOGD]
     double* sWc = sH + LOGD;                            // [2M]
     double* sWa = sWc + 2 * a.M;                        // [2M]
@@ -342,79 +350,50 @@ __device__ __forceinline__ void herm_ado(const FusedArgs& a, long long n, const 
 
     const int tid = threadIdx.x;
     const uint64_t pkeep = pol_last(), pn = pol_normal();
-    // thread 0 alone owns the two mbarriers (init, copies, waits); the others
-    // learn of a completed copy from the block barrier that follows its wait
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s_addr(&bar[0])) : "memory");
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(s_addr(&bar[1])) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        bulk_g2s(pk, u + n * P, P * sizeof(double2), &bar[0], a.ado_keep[n] ? pkeep : pn);
-    }
+    double2 acc[E];
+    int rc[E];  // row << 8 | column
     const int Q = a.ent_count[n];
-    if (PAULI) {
-        if (tid < a.J) sBit[tid] = a.vbit[tid];
-    } else {
-        for (int i = tid; i < a.J * D; i += T) sV[i] = a.vdiag[i];
-    }
-    if (tid < LOGD) sH[tid] = a.hflip[tid];
-    for (int q = tid; q < Q; q += T) {
-        const long long src = n * 2 * a.M + q;
-        sSlab[q] = a.ent_slab[src];
-        sBath[q] = a.ent_bath[src];
-        sWc[q] = a.ent_wc[src];
-        sWa[q] = a.ent_wa[src];
-    }
     const double g = a.gsum[n];
     const int slot = a.slot ? a.slot[n] : -1;
-    // one barrier publishes the tables above and the arrival of the slab
-    if (__syncthreads_or(tid == 0 && !bar_wait(&bar[0], 0))) {
-        if (tid == 0) atomicExch(a.error_flag, 1);
-        return;
-    }
-
-    // ---- unpack the own slab: (r, c) and its mirror (c, r) = conj
-    int rc[E];
+    // ---- own elements: into shared memory with their mirrors, and the diagonal term
+    {
+        const uint64_t pol = a.ado_keep[n] ? pkeep : pn;
+        double2 x[E];
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int i = tid + T * k;
-        int r = 0, c = 0;
-        if (kExact || i < P) {
-            herm_coords(i, LOGD, r, c);
-            const double2 v = pk[i];
-            full[herm_slot<LOGD>(r, c)] = v;
-            if (r != c) full[herm_slot<LOGD>(c, r)] = make_double2(v.x, -v.y);
+        for (int k = 0; k < E; ++k)
+            if (kExact || tid + T * k < P) x[k] = ldg_hint(u + n * P + tid + T * k, pol);
+        if (PAULI) {
+            if (tid < a.J) sBit[tid] = a.vbit[tid];
+        } else {
+            for (int i = tid; i < a.J * D; i += T) sV[i] = a.vdiag[i];
         }
-        rc[k] = (r << 8) | c;
-    }
-    __syncthreads();
-    // the packed copy is still the stage-1 base; otherwise stream rho_n into it
-    if (base_kind == kBaseRho && tid == 0) bulk_g2s(pk, rho + n * P, P * sizeof(double2), &bar[1], pol_first());
-
-    // ---- step A: diagonal (packed table) and transverse field (unpacked slab)
-    double2 acc[E];
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const int i = tid + T * k;
-        acc[k] = make_double2(0.0, 0.0);
-        if (!kExact && i >= P) continue;
-        const int sl = herm_slot<LOGD>(rc[k] >> 8, rc[k] & 255);
-        const double2 x = full[sl];
-        const double2 t = __ldg(a.diag + i);
-        double hr = 0.0, hi = 0.0;
-#pragma unroll
-        for (int b = 0; b < LOGD; ++b) {
-            const double h = sH[b];
-            const double2 rowp = full[sl ^ ((1 << b) << LOGD) ^ (b < 3 ? (1 << b) : 0)];
-            const double2 colp = full[sl ^ (1 << b)];
-            hr += h * (rowp.x - colp.x);
-            hi += h * (rowp.y - colp.y);
+        if (tid < LOGD) sH[tid] = a.hflip[tid];
+        for (int q = tid; q < Q; q += T) {
+            const long long src = n * 2 * a.M + q;
+            sSlab[q] = a.ent_slab[src];
+            sBath[q] = a.ent_bath[src];
+            sWc[q] = a.ent_wc[src];
+            sWa[q] = a.ent_wa[src];
         }
-        const double tr = t.x - g;
-        acc[k].x = tr * x.x - t.y * x.y + hi;
-        acc[k].y = tr * x.y + t.y * x.x - hr;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            rc[k] = 0;
+            acc[k] = make_double2(0.0, 0.0);
+            if (!kExact && tid + T * k >= P) continue;
+            int r, c;
+            herm_coords(tid + T * k, LOGD, r, c);
+            rc[k] = (r << 8) | c;
+            full[herm_slot<LOGD>(r, c)] = x[k];
+            if (r != c) full[herm_slot<LOGD>(c, r)] = make_double2(x[k].x, -x[k].y);
+            const double2 t = __ldg(a.diag + tid + T * k);
+            const double tr = t.x - g;
+            acc[k].x = tr * x[k].x - t.y * x[k].y;
+            acc[k].y = tr * x[k].y + t.y * x[k].x;
+        }
     }
 
-    // ---- step B: neighbour entries, E loads in flight per thread
+    // ---- neighbour entries, E loads in flight per thread
     const double2* ubase = u + tid;
     for (int q = 0; q < Q; ++q) {
         const int jb = sBath[q];
@@ -477,17 +456,40 @@ __device__ __forceinline__ void herm_ado(const FusedArgs& a, long long n, const 
         }
     }
 
+    // ---- transverse field: flips in the unpacked slab
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        if (!kExact && tid + T * k >= P) continue;
+        const int sl = herm_slot<LOGD>(rc[k] >> 8, rc[k] & 255);
+        double hr = 0.0, hi = 0.0;
+#pragma unroll
+        for (int b = 0; b < LOGD; ++b) {
+            const double h = sH[b];
+            const double2 rowp = full[sl ^ ((1 << b) << LOGD) ^ (b < 3 ? (1 << b) : 0)];
+            const double2 colp = full[sl ^ (1 << b)];
+            hr += h * (rowp.x - colp.x);
+            hi += h * (rowp.y - colp.y);
+        }
+        acc[k].x += hi;
+        acc[k].y -= hr;
+    }
+
     // ---- Horner epilogue
-    if (base_kind == kBaseRho && __syncthreads_or(tid == 0 && !bar_wait(&bar[1], 0))) {
-        if (tid == 0) atomicExch(a.error_flag, 1);
-        return;
+    const double2* rho_n = rho + n * P + tid;
+    double2 bs[E];
+#pragma unroll
+    for (int k = 0; k < E; ++k) {
+        bs[k] = make_double2(0.0, 0.0);
+        if (!kExact && tid + T * k >= P) continue;
+        if (base_kind == kBaseSelf) bs[k] = full[herm_slot<LOGD>(rc[k] >> 8, rc[k] & 255)];
+        else if (base_kind == kBaseRho) bs[k] = ldg_stream(rho_n + T * k);
     }
     double2* out_n = out + n * P + tid;
 #pragma unroll
     for (int k = 0; k < E; ++k) {
         if (!kExact && tid + T * k >= P) continue;
-        const double2 b = (base_kind == kBaseZero) ? make_double2(0.0, 0.0) : pk[tid + T * k];
-        stg_stream(out_n + T * k, make_double2(b.x + alpha * acc[k].x, b.y + alpha * acc[k].y));
+        stg_stream(out_n + T * k, make_double2(bs[k].x + alpha * acc[k].x, bs[k].y + alpha * acc[k].y));
     }
 }
 
@@ -515,16 +517,15 @@ template <int LOGD>
 size_t herm_smem(int M, int J)
 {
     const size_t D = size_t(1) << LOGD;
-    const size_t P = (D / 2) * (D + 1);
-    return (D * D + P) * sizeof(double2) + 16 + sizeof(double) * (J * D + LOGD + 4 * M) +
-           sizeof(int) * (4 * M + J);
+    return D * D * sizeof(double2) + sizeof(double) * (J * D + LOGD + 4 * M) + sizeof(int) * (4 * M + J);
 }
 
 template <int LOGD, bool PAULI>
 bool prepare_herm_t(int M, int J)
 {
     const size_t smem = herm_smem<LOGD>(M, J);
-    if (smem > 227 * 1024) return false;
+    // a slab's bytes below the limit: the tables of (M, J) accepted do not depend on how the slab is staged
+    if (smem + static_cast<size_t>(herm_elems(LOGD)) * sizeof(double2) + 16 > 227 * 1024) return false;
     static size_t configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
