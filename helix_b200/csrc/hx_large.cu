@@ -396,9 +396,18 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 // inside, so 2 (log2 d - 6) partners come through L2 where bands of whole rows
 // needed log2 d - log2(2048 / d) and the scattered lower halves of the rows:
 //
-//  * the lanes of a warp are 4 rows x 8 columns, so a partner tile is read in
-//    pieces of 128 bytes directly and of 64 bytes where it lies below the
-//    diagonal (conjugates of the transposed tile): no load is scattered;
+//  * double: the lanes of a warp are 4 rows x 8 columns, so a partner tile is
+//    read in pieces of 128 bytes directly and of 64 bytes where it lies below
+//    the diagonal (conjugates of the transposed tile): no load is scattered;
+//  * complex64: the lanes are one row of 32 columns, and the partner tiles on
+//    and below the diagonal come through shared memory, two asked for at the
+//    start and used after everything else (64 x 65 buffers, so the transposed
+//    read is free of bank conflicts).  Read directly they were 33 of the 46
+//    wavefronts of global loads per 32 elements.  Not staged where the tables
+//    leave no room for the buffers at two CTAs per SM;
+//  * the sum is kept times i: then a flip and a commutator entry are one
+//    packed multiply-add in complex64, and an entry whose weight is zero on
+//    all of a warp's rows is left out (the kernel issues 67% of the time);
 //  * a thread owns 8 elements of one column, 8 rows apart, in NP passes: the
 //    flips of the rows of a pass are in registers, the other flips inside the
 //    tile in shared memory (element (r, c) at r 64 + (c ^ (r & 7)): free of
@@ -407,12 +416,14 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 //    term from two d-entry tables instead of a third slab-sized stream;
 //  * diagonal tiles compute their upper triangle only.
 //
-// d = 256, 969 ADOs: 0.70 ms a stage in double, 0.48 in complex64 (bands of
-// rows: 0.94 and 0.56).  The 64 registers of two CTAs per SM are the limit: one
+// d = 256, 969 ADOs: 0.69 ms a stage in double, 0.43 in complex64 (bands of
+// rows: 0.94 and 0.56; complex64 without staged tiles and packed arithmetic
+// 0.48).  Double is at 74% of the load-store unit's wavefronts and 7.4 TB/s
+// between L2 and the SMs.  The 64 registers of two CTAs per SM are the limit: one
 // pass of 8 rows in double spills or leaves one CTA (0.85 ms).
 template <typename R, int LOGD> struct TileShape;
 template <int LOGD> struct TileShape<double, LOGD> { static constexpr int NP = 2, MINB = 2, LR = LOGD == 7 ? 1 : 4; };
-template <int LOGD> struct TileShape<float, LOGD> { static constexpr int NP = 1, MINB = 2, LR = 2; };
+template <int LOGD> struct TileShape<float, LOGD> { static constexpr int NP = 1, MINB = 2, LR = 1; };
 constexpr int kTileT = 512;
 
 // Element (r, c), r <= c, of a packed slab is at packed_row(r) + c.
@@ -423,12 +434,46 @@ __device__ __forceinline__ int packed_row(int r)
     return r < D / 2 ? r * D : (D - 1 - r) * (D + 1) + 1;
 }
 
-// acc += (weight at the k-th row) y for one neighbour entry with a sigma_z
+// z += w y and x - y, elementwise: one packed instruction each in complex64 (the same roundings).
+__device__ __forceinline__ void add_scaled(double2& z, double w, const double2& y)
+{
+    z.x += w * y.x;
+    z.y += w * y.y;
+}
+__device__ __forceinline__ double2 minus(const double2& x, const double2& y) { return make_double2(x.x - y.x, x.y - y.y); }
+__device__ __forceinline__ uint64_t bits2(const float2& v)
+{
+    uint64_t b;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "f"(v.x), "f"(v.y));
+    return b;
+}
+__device__ __forceinline__ float2 fma2(const float2& a, const float2& b, const float2& c)
+{
+    uint64_t d;
+    float2 v;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(bits2(a)), "l"(bits2(b)), "l"(bits2(c)));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(v.x), "=f"(v.y) : "l"(d));
+    return v;
+}
+__device__ __forceinline__ void add_scaled(float2& z, float w, const float2& y) { z = fma2(make_float2(w, w), y, z); }
+// z += (wx y.x, wy y.y)
+__device__ __forceinline__ void add_scaled2(float2& z, float wx, float wy, const float2& y)
+{
+    z = fma2(make_float2(wx, wy), y, z);
+}
+__device__ __forceinline__ void add_scaled2(double2& z, double wx, double wy, const double2& y)
+{
+    z.x += wx * y.x;
+    z.y += wy * y.y;
+}
+__device__ __forceinline__ float2 minus(const float2& x, const float2& y) { return fma2(y, make_float2(-1.f, -1.f), x); }
+
+// z += i (weight at the k-th row) y for one neighbour entry with a sigma_z
 // coupling.  Where the spin's bits of row and column agree only -{V, y} wa
 // counts, else only -i [V, y] wc (twice the weights are given).  T: the bit of
 // k that the spin's row bit is, or -1 when all the rows of the pass share it.
 template <typename R, int E, int T>
-__device__ __forceinline__ void tile_entry(C2<R>* acc, const C2<R>* src, int step, const bool* on, int k0, int br0,
+__device__ __forceinline__ void tile_entry(C2<R>* z, const C2<R>* src, int step, const bool* on, int k0, int br0,
                                            int bc, R wc, R wa)
 {
     C2<R> y[E];
@@ -436,22 +481,67 @@ __device__ __forceinline__ void tile_entry(C2<R>* acc, const C2<R>* src, int ste
     const R wr0 = same0 ? (br0 ? -wa : wa) : R(0), wi0 = same0 ? R(0) : (br0 ? -wc : wc);
     const R wr1 = same0 ? R(0) : (br0 ? wa : -wa), wi1 = same0 ? (br0 ? wc : -wc) : R(0);  // at the others
     const bool need0 = wr0 != R(0) || wi0 != R(0), need1 = wr1 != R(0) || wi1 != R(0);
+    // 3% of a complex64 step; in double, where issue slots are not short, the branch costs 1.5%
+    if (sizeof(R) == sizeof(float) && !need0 && (T < 0 || !need1)) return;
 #pragma unroll
     for (int k = 0; k < E; ++k) {
         const bool other = T >= 0 && ((k >> (T < 0 ? 0 : T)) & 1);
         y[k] = mk<R>(0, 0);
         if (on[k] && (other ? need1 : need0)) y[k] = __ldg(src + k * step);
     }
+    if (same0) {
 #pragma unroll
-    for (int k = 0; k < E; ++k) {
-        const bool other = T >= 0 && ((k >> (T < 0 ? 0 : T)) & 1);
-        const R wr = other ? wr1 : wr0, wi = other ? wi1 : wi0;
-        acc[k].x += wr * y[k].x - wi * y[k].y;
-        acc[k].y += wr * y[k].y + wi * y[k].x;
+        for (int k = 0; k < E; ++k) {
+            if (T >= 0 && ((k >> (T < 0 ? 0 : T)) & 1)) {
+                add_scaled(z[k], -wi1, y[k]);
+            } else {
+                z[k].x -= wr0 * y[k].y;
+                z[k].y += wr0 * y[k].x;
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            if (T >= 0 && ((k >> (T < 0 ? 0 : T)) & 1)) {
+                z[k].x -= wr1 * y[k].y;
+                z[k].y += wr1 * y[k].x;
+            } else {
+                add_scaled(z[k], -wi0, y[k]);
+            }
+        }
     }
 }
 
-template <typename R, int LOGD, bool PAULI>
+// Flip f of tile (I, J), f = 2 i for bit 6 + i of the row and 2 i + 1 of the column: the partner's tile
+// (A, B), true when it is not stored as such (on or below the diagonal).
+__device__ __forceinline__ bool flip_tile(int f, int I, int J, int& A, int& B)
+{
+    const int m = 1 << (f >> 1);
+    A = f & 1 ? I : I ^ m;
+    B = f & 1 ? J ^ m : J;
+    return A >= B;
+}
+
+// Ask for the stored tile (B, A), B <= A, of a packed slab into the 64 x 65 buffer dst (the upper triangle
+// only when A == B).
+template <typename R, int LOGD>
+__device__ __forceinline__ void stage_tile(const C2<R>* __restrict__ un, int A, int B, C2<R>* dst)
+{
+    constexpr int D = 1 << LOGD;
+    const int j = threadIdx.x & 63, i0 = threadIdx.x >> 6;  // rows i0 + 8 k
+    const C2<R>* src = un + packed_row<LOGD>(B * 64 + i0) + A * 64 + j;
+    const int step = B * 64 < D / 2 ? 8 * D : -8 * (D + 1);
+    const uint32_t at = l_addr(dst + i0 * 65 + j);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+        if (A != B || i0 + 8 * k <= j)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(
+                             at + k * 8 * 65 * static_cast<uint32_t>(sizeof(C2<R>))),
+                         "l"(src + k * step), "n"(sizeof(C2<R>))
+                         : "memory");
+}
+
+template <typename R, int LOGD, bool PAULI, bool STAGED>
 __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
     herm_tile_kernel(LargeArgs<R> a, const C2<R>* __restrict__ u, const C2<R>* rho, C2<R>* out, double alpha_d,
                      int base_kind)
@@ -461,8 +551,10 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
     constexpr int LR = TileShape<R, LOGD>::LR, LC = 32 / LR;  // rows and columns of a warp's lanes
     constexpr long long P = static_cast<long long>(D / 2) * (D + 1);
     extern __shared__ __align__(128) unsigned char smem[];
+    constexpr int F = 2 * (LOGD - 6);
     C* sx = reinterpret_cast<C*>(smem);                                // [64][64] the tile
-    double* sE = reinterpret_cast<double*>(smem + 4096 * sizeof(C));   // [D] E_r (PAULI)
+    C* sT = sx + 4096;                                                 // [2][64][65] partner tiles, when staged
+    double* sE = reinterpret_cast<double*>(sT + (STAGED ? 2 * 64 * 65 : 0));  // [D] E_r (PAULI)
     R* sX = reinterpret_cast<R*>(sE + (PAULI ? D : 0));                // [D] -4 sum of xi over differing bits (PAULI)
     R* sV = sX + (PAULI ? D : 0);                                      // [J][D] (general couplings)
     R* sH = sV + (PAULI ? 0 : a.J * D);                                // [LOGD]
@@ -487,11 +579,22 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
     const int step = I * 64 < D / 2 ? 8 * D : -8 * (D + 1);
 
     // ---- the tile (both triangles of a diagonal one)
+    [[maybe_unused]] int fl = 0;  // the next flip to stage, or past the last one
     {
         C x[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k)
             if (!diag || r0 + 8 * k <= c) x[k] = __ldg(un + own + k * step);
+        if constexpr (STAGED) {
+#pragma unroll 1
+            for (int b = 0; b < 2; ++b) {
+                int A, B;
+                while (fl < F && !flip_tile(fl, I, J, A, B)) ++fl;
+                if (fl < F) stage_tile<R, LOGD>(un, A, B, sT + b * 64 * 65);
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                ++fl;
+            }
+        }
         const int Q = a.ent_count[n];
         for (int q = tid; q < Q; q += kTileT) {
             const long long src = n * 2 * a.M + q;
@@ -526,8 +629,8 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
 
 #pragma unroll 1
     for (int k0 = 0; k0 < 8; k0 += E) {
-        if (diag && !__any_sync(0xffffffffu, r0 + 8 * k0 <= c)) break;  // the warp's rows are below its columns
-        C acc[E];
+        if (NP > 1 && diag && !__any_sync(0xffffffffu, r0 + 8 * k0 <= c)) break;  // the warp's rows are below its columns
+        C z[E];  // i times the sum
         bool on[E];
         const C* sp = sx + (r0 + 8 * k0) * 64;  // the pass's first row; + 512 per k
         const int cs = c ^ (r0 & 7);
@@ -552,10 +655,10 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
                     ti = t.y;
                 }
                 tr -= g;
-                acc[k].x = tr * x[k].x - ti * x[k].y;
-                acc[k].y = tr * x[k].y + ti * x[k].x;
+                z[k].x = -(tr * x[k].y + ti * x[k].x);
+                z[k].y = tr * x[k].x - ti * x[k].y;
             }
-            // ---- flips inside the tile: acc -= i h (row partner - column partner)
+            // ---- flips inside the tile: z += h (row partner - column partner)
 #pragma unroll
             for (int b = 0; b < 6; ++b) {
                 const R h = sH[b];
@@ -567,17 +670,16 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
                     if (b >= 3 && (1 << (b - 3)) < E) rowp = x[k ^ (1 << (b - 3))];
                     else rowp = rp[rs + 512 * k];
                     const C colp = sp[(cs ^ (1 << b)) + 512 * k];
-                    acc[k].x += h * (rowp.y - colp.y);
-                    acc[k].y -= h * (rowp.x - colp.x);
+                    add_scaled(z[k], h, minus(rowp, colp));
                 }
             }
         }
         // ---- flips of the higher bits: the same place in another tile, through L2
 #pragma unroll 1
-        for (int f = 0; f < 2 * (LOGD - 6); ++f) {
-            const int m = 1 << (f >> 1);
+        for (int f = 0; f < F; ++f) {
+            int A, B;  // the partner's tile
+            if (flip_tile(f, I, J, A, B) && STAGED) continue;
             const R h = sH[6 + (f >> 1)];
-            const int A = f & 1 ? I : I ^ m, B = f & 1 ? J ^ m : J;  // the partner's tile
             const R w = f & 1 ? -h : h;
             C y[E];
             if (A == B) {
@@ -595,8 +697,8 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
             const R wy = A > B ? -w : w;
 #pragma unroll
             for (int k = 0; k < E; ++k) {
-                acc[k].x += wy * y[k].y;
-                acc[k].y -= w * y[k].x;
+                z[k].x += w * y[k].x;
+                z[k].y += wy * y[k].y;
             }
         }
         // ---- neighbour entries, E loads in flight
@@ -608,10 +710,10 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
             const int bit = sBit[q];
             if (PAULI) {
                 const int br0 = ((gr0 + 8 * k0) >> bit) & 1, bc = (gc >> bit) & 1;
-                if (bit == 3 && E > 1) tile_entry<R, E, 0>(acc, src, step, on, k0, br0, bc, wc, wa);
-                else if (bit == 4 && E > 2) tile_entry<R, E, 1>(acc, src, step, on, k0, br0, bc, wc, wa);
-                else if (bit == 5 && E > 4) tile_entry<R, E, 2>(acc, src, step, on, k0, br0, bc, wc, wa);
-                else tile_entry<R, E, -1>(acc, src, step, on, k0, br0, bc, wc, wa);
+                if (bit == 3 && E > 1) tile_entry<R, E, 0>(z, src, step, on, k0, br0, bc, wc, wa);
+                else if (bit == 4 && E > 2) tile_entry<R, E, 1>(z, src, step, on, k0, br0, bc, wc, wa);
+                else if (bit == 5 && E > 4) tile_entry<R, E, 2>(z, src, step, on, k0, br0, bc, wc, wa);
+                else tile_entry<R, E, -1>(z, src, step, on, k0, br0, bc, wc, wa);
             } else {
                 const R* vj = sV + bit * D;
                 const R vc = vj[gc];
@@ -626,9 +728,47 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
                 for (int k = 0; k < E; ++k) {
                     const R vr = vj[gr0 + 8 * (k0 + k)];
                     const R ar = -(vr + vc) * wa, ai = -(vr - vc) * wc;
-                    acc[k].x += ar * y[k].x - ai * y[k].y;
-                    acc[k].y += ar * y[k].y + ai * y[k].x;
+                    z[k].x -= ar * y[k].y + ai * y[k].x;
+                    z[k].y += ar * y[k].x - ai * y[k].y;
                 }
+            }
+        }
+        // ---- the flips from staged tiles: conjugates of the transposed place
+        if constexpr (STAGED) {
+            int buf = 0;
+#pragma unroll 1
+            for (int f = 0; f < F; ++f) {
+                int A, B;
+                if (!flip_tile(f, I, J, A, B)) continue;
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                __syncthreads();
+                const C* t = sT + buf * 64 * 65;
+                const R h = sH[6 + (f >> 1)];
+                const R w = f & 1 ? -h : h;
+                if (A != B) {
+#pragma unroll
+                    for (int k = 0; k < E; ++k) {
+                        const C y = t[c * 65 + r0 + 8 * k];
+                        add_scaled2(z[k], w, -w, y);
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < E; ++k) {
+                        const int r = r0 + 8 * k;
+                        const C y = t[r <= c ? r * 65 + c : c * 65 + r];
+                        z[k].x += w * y.x;
+                        z[k].y += r <= c ? w * y.y : -w * y.y;
+                    }
+                }
+                int A2, B2;
+                while (fl < F && !flip_tile(fl, I, J, A2, B2)) ++fl;
+                if (fl < F) {
+                    __syncthreads();  // every warp has read the buffer
+                    stage_tile<R, LOGD>(un, A2, B2, sT + buf * 64 * 65);
+                }
+                asm volatile("cp.async.commit_group;" ::: "memory");
+                ++fl;
+                buf ^= 1;
             }
         }
         // ---- up term of tier L-1, summed by large_upterm_kernel
@@ -639,8 +779,8 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
             for (int k = 0; k < E; ++k) y[k] = on[k] ? __ldcs(Un + k * step) : mk<R>(0, 0);
 #pragma unroll
             for (int k = 0; k < E; ++k) {
-                acc[k].x += y[k].x;
-                acc[k].y += y[k].y;
+                z[k].x -= y[k].y;
+                z[k].y += y[k].x;
             }
         }
         // ---- Horner epilogue
@@ -654,7 +794,7 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
         }
 #pragma unroll
         for (int k = 0; k < E; ++k)
-            if (on[k]) __stcs(on_ + k * step, mk<R>(y[k].x + alpha * acc[k].x, y[k].y + alpha * acc[k].y));
+            if (on[k]) __stcs(on_ + k * step, mk<R>(y[k].x + alpha * z[k].y, y[k].y - alpha * z[k].x));
     }
 }
 
@@ -850,10 +990,10 @@ __global__ void vec_d2f_kernel(const double* __restrict__ in, float* __restrict_
 }
 
 template <typename R, int LOGD>
-size_t tile_smem(int M, int J, bool pauli)
+size_t tile_smem(int M, int J, bool pauli, bool staged)
 {
     const size_t D = size_t(1) << LOGD;
-    return 4096 * sizeof(C2<R>) + (pauli ? D * (sizeof(double) + sizeof(R)) : J * D * sizeof(R)) +
+    return (4096 + (staged ? 2 * 64 * 65 : 0)) * sizeof(C2<R>) + (pauli ? D * (sizeof(double) + sizeof(R)) : J * D * sizeof(R)) +
            sizeof(R) * (LOGD + 4 * M) + sizeof(int) * 4 * M;
 }
 
@@ -886,32 +1026,26 @@ template <typename R, int LOGD>
 bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* out, double alpha, int base,
               cudaStream_t s, bool launch)
 {
-    const size_t smem = a.herm ? tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0)
-                               : large_smem<R, LOGD>(a.M, a.J);
-    if (smem > 227 * 1024) return false;
-    static size_t configured[64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 64 && configured[dev] < smem) {
-        if (cudaFuncSetAttribute(large_kernel<R, LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)) != cudaSuccess ||
-            cudaFuncSetAttribute(herm_tile_kernel<R, LOGD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)) != cudaSuccess ||
-            cudaFuncSetAttribute(herm_tile_kernel<R, LOGD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 static_cast<int>(smem)) != cudaSuccess)
-            return false;
-        configured[dev] = smem;
+    using Kernel = void (*)(LargeArgs<R>, const C2<R>*, const C2<R>*, C2<R>*, double, int);
+    // complex64: partner tiles are staged where two CTAs per SM still find room for the buffers
+    constexpr bool kStage = sizeof(R) == sizeof(float);
+    const bool staged = kStage && tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0, true) <= 113 * 1024;
+    Kernel kernel = large_kernel<R, LOGD>;
+    size_t smem = large_smem<R, LOGD>(a.M, a.J);
+    if (a.herm) {
+        smem = tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0, staged);
+        if (staged) kernel = a.pauli ? herm_tile_kernel<R, LOGD, true, kStage> : herm_tile_kernel<R, LOGD, false, kStage>;
+        else kernel = a.pauli ? herm_tile_kernel<R, LOGD, true, false> : herm_tile_kernel<R, LOGD, false, false>;
     }
-    if (!launch) return true;
+    if (smem > 227 * 1024) return false;
+    // the limit is raised when a context is made, outside any capture
+    if (!launch)
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
     // full slabs: d^2 / 4096 bands each; packed slabs: the tiles of the upper triangle
     constexpr long long kBlocks = (1 << LOGD) / 64;
     const long long nb = (a.H - a.first_ado) * (a.herm ? kBlocks * (kBlocks + 1) / 2 : (1ll << (2 * LOGD)) / 4096);
     if (nb <= 0) return true;
-    if (a.herm && a.pauli)
-        herm_tile_kernel<R, LOGD, true><<<static_cast<unsigned>(nb), kTileT, smem, s>>>(a, u, rho, out, alpha, base);
-    else if (a.herm)
-        herm_tile_kernel<R, LOGD, false><<<static_cast<unsigned>(nb), kTileT, smem, s>>>(a, u, rho, out, alpha, base);
-    else large_kernel<R, LOGD><<<static_cast<unsigned>(nb), LargeThreads<R>::T, smem, s>>>(a, u, rho, out, alpha, base);
+    kernel<<<static_cast<unsigned>(nb), a.herm ? kTileT : LargeThreads<R>::T, smem, s>>>(a, u, rho, out, alpha, base);
     return true;
 }
 

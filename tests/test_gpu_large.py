@@ -152,3 +152,33 @@ def test_mixed_precision_at_the_c3_shape():
     o.close()
     assert np.max(np.abs(r64[:2] - ro)) < TOL
     assert np.max(np.abs(e64[:2] - eo)) < TOL
+
+
+@pytest.mark.parametrize("n,baths,K,collective", [
+    (7, 7, 1, False),   # one bit outside a tile: diagonal tiles as partners
+    (8, 3, 1, False),   # two: up to three partner tiles below the diagonal
+    (8, 3, 1, True),
+    (9, 2, 0, False),
+    (10, 1, 0, False),  # four bits
+    (10, 4, 0, True),   # the operators' tables leave no room for partner tiles in shared memory
+])
+def test_mixed_precision_packed_rhs_at_every_tile_grid(n, baths, K, collective):
+    """complex64 tiles of packed slabs, a different field on every spin: the
+    right-hand side within 1e-5 of the oracle's largest element (some fifty
+    roundings of 6e-8 each)."""
+    p = S.spin_glass(n, seed=40 + n, depth=2, K=K, h=0.5, dt=0.005)
+    rng = np.random.default_rng(n)
+    p.h_flip = rng.uniform(0.2, 1.0, n)
+    p.baths = p.baths[:baths]
+    if collective:
+        for b in p.baths:
+            b.v_diag = rng.uniform(-0.7, 0.7, p.dim)
+    o = O.Oracle(p)
+    x = _hermitian((rng.standard_normal((o.size, p.dim, p.dim)) + 1j * rng.standard_normal((o.size, p.dim, p.dim))) * 0.05)
+    ref = o.rhs(x)
+    o.close()
+    with capi.Context(p, precision="mixed") as cm:
+        assert cm.hermitian_packed
+        cm.set_state(x)
+        r = cm.rhs()
+        assert np.max(np.abs(r - ref)) < 1e-5 * np.max(np.abs(ref))
