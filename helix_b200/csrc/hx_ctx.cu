@@ -129,15 +129,16 @@ hx::UpTermArgs hx::upterm_args_of(const hx_ctx* c)
 
 void hx::unpack_herm_host(const double2* pk, int logd, double* out)
 {
-    const int D = 1 << logd, P = hx::herm_elems(logd);
-    for (int i = 0; i < P; ++i) {
-        int r, c;
-        hx::herm_coords(i, logd, r, c);
-        const double2 v = pk[i];
-        out[2 * (static_cast<size_t>(r) * D + c)] = v.x;
-        out[2 * (static_cast<size_t>(r) * D + c) + 1] = v.y;
-        out[2 * (static_cast<size_t>(c) * D + r)] = v.x;
-        out[2 * (static_cast<size_t>(c) * D + r) + 1] = r == c ? v.y : -v.y;
+    const size_t D = size_t(1) << logd;
+    for (size_t r = 0; r < D; ++r) {
+        const double2* row = pk + hx::herm_index(static_cast<int>(r), static_cast<int>(r), logd) - r;
+        for (size_t c = r; c < D; ++c) {
+            const double2 v = row[c];
+            out[2 * (r * D + c)] = v.x;
+            out[2 * (r * D + c) + 1] = v.y;
+            out[2 * (c * D + r)] = v.x;
+            out[2 * (c * D + r) + 1] = r == c ? v.y : -v.y;
+        }
     }
 }
 
