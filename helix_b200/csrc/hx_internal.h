@@ -404,6 +404,8 @@ void launch_init_state(double2* rho, long long n, long long one, cudaStream_t s)
 struct hx_ctx {
     int device = 0;
     cudaStream_t own_stream = nullptr;
+    cudaStream_t side_stream = nullptr;  // ADO 0's kernels of a mixed-precision stage, beside the others
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     cudaStream_t stream = nullptr;
     int d = 0, logd = 0, M = 0, J = 0, order = 4;
     long long H = 0;
