@@ -848,8 +848,7 @@ def run_mixed(args, cfg: dict) -> None:
                      "peak_source": f"{peak_kind} hbm_gbs (MEASURED_PEAKS.json)" if peak_kind == "measured"
                      else "fallback 6650 GB/s",
                      "algorithmic_bytes_per_launch": per_stage,
-                     "kernel": ("herm_band_kernel<float,8>" if state32 < H * p.dim * p.dim * 8 else "large_kernel<float,8>")
-                     + " + large_upterm_kernel + ado0_kernel",
+                     "kernel": "tile_kernel<float,8> + large_upterm_kernel + ado0_kernel",
                      "launch_ms": stage_ms},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": H * p.dim * p.dim * 16 / args.steps,
                 "d2h_bytes_per_step": p.dim * p.dim * 16 + 24,

@@ -260,7 +260,7 @@ struct LargeArgs {
     long long H;
     int M, J, logd;
     int first_ado;           // 1 when ADO 0 runs in double precision (ado0_kernel)
-    int herm;                // 1: slabs, diag and U Hermitian-packed (herm_tile_kernel)
+    int herm;                // 1: slabs, diag and U Hermitian-packed
     int pauli;               // 1: every coupling is the sigma_z of one spin, vbit[j]; then diagonal term =
     const int* vbit;         // [J]  (xsum[r ^ c] + i (hdiag[c] - hdiag[r])) u
     const double* hdiag;     // [d]

@@ -8,14 +8,15 @@
 // for diagonal couplings V_j and H = diag(E) + sum_i h_i sigma_x(i).  A slab of
 // d = 256 is 1 MB in double precision, too large for shared memory, so:
 //
-//  * full slabs: one CTA computes one band of 4096 elements (4096/d whole rows)
-//    of one ADO (packed slabs: herm_tile_kernel below); the band arrives by one TMA bulk copy; consecutive CTAs take the
-//    bands of one ADO, so the rest of its slab is in L2 while they run;
-//  * column flips of the transverse field and row flips inside the band read
-//    shared memory; row flips across bands read the slab through L2;
-//  * neighbour terms are elementwise (diagonal V) and read through L2, two
-//    entries at a time; the up term of tier L-1 (neighbours in the top tier)
-//    comes from large_upterm_kernel, which walks the top tier tile by tile.
+//  * one CTA computes one 64 x 64 tile of one ADO, held in shared memory
+//    (tile_kernel; with packed slabs the tiles on and above the diagonal);
+//    consecutive CTAs take the tiles of one ADO, so the rest of its slab is in
+//    L2 while they run;
+//  * flips of the six low bits of row and column read shared memory or
+//    registers, flips of the higher bits another tile through L2;
+//  * neighbour terms are elementwise (diagonal V) and read through L2; the up
+//    term of tier L-1 (neighbours in the top tier) comes from
+//    large_upterm_kernel, which walks the top tier tile by tile.
 //
 // With a dense H (HX_FLAG_DENSE_H, complex64 path) the diagonal table keeps
 // the real diagonal of H and the commutator with the rest of H (no flip
@@ -41,8 +42,6 @@ namespace {
 
 __device__ __forceinline__ uint32_t l_addr(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
-constexpr uint32_t kLargeSpin = 1u << 20;
-
 template <typename R>
 __device__ __forceinline__ C2<R> mk(R x, R y)
 {
@@ -50,184 +49,6 @@ __device__ __forceinline__ C2<R> mk(R x, R y)
     v.x = x;
     v.y = y;
     return v;
-}
-
-// Threads of a full-slab band CTA: complex64 bands take twice the threads
-// (8 elements each instead of 16), so twice the warps per SM hide the
-// neighbour gathers' latency at the same shared memory per CTA.
-template <typename R> struct LargeThreads { static constexpr int T = 256; };
-template <> struct LargeThreads<float> { static constexpr int T = 512; };
-
-template <typename R, int LOGD>
-__global__ void __launch_bounds__(LargeThreads<R>::T, 2)
-    large_kernel(LargeArgs<R> a, const C2<R>* __restrict__ u, const C2<R>* rho, C2<R>* out, double alpha_d,
-                 int base_kind)
-{
-    using C = C2<R>;
-    constexpr int D = 1 << LOGD, T = LargeThreads<R>::T, BE = 4096, E = BE / T, CH = 4;
-    constexpr long long D2 = static_cast<long long>(D) * D;
-    constexpr int NB = static_cast<int>(D2 / BE);  // bands per slab
-    extern __shared__ __align__(128) unsigned char smem[];
-    C* sx = reinterpret_cast<C*>(smem);                       // [BE] the band
-    uint64_t* bar = reinterpret_cast<uint64_t*>(smem + BE * sizeof(C));
-    double* sWc = reinterpret_cast<double*>(bar + 2);         // [2M]
-    double* sWa = sWc + 2 * a.M;                              // [2M]
-    R* sV = reinterpret_cast<R*>(sWa + 2 * a.M);              // [J][D]
-    R* sH = sV + a.J * D;                                     // [LOGD]
-    int* sSlab = reinterpret_cast<int*>(sH + LOGD + 1);       // [2M]
-    int* sBath = sSlab + 2 * a.M;                             // [2M]
-
-    const int tid = threadIdx.x;
-    const long long n = a.first_ado + static_cast<long long>(blockIdx.x) / NB;
-    const long long be = static_cast<long long>(blockIdx.x % NB) * BE;  // band's first element in the slab
-    const C* un = u + n * D2;
-    if (tid == 0) {
-        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(l_addr(bar)) : "memory");
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (tid == 0) {
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(l_addr(bar)),
-                     "r"(static_cast<uint32_t>(BE * sizeof(C)))
-                     : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         l_addr(sx)),
-                     "l"(un + be), "r"(static_cast<uint32_t>(BE * sizeof(C))), "r"(l_addr(bar))
-                     : "memory");
-    }
-    const int Q = a.ent_count[n];
-    for (int i = tid; i < a.J * D; i += T) sV[i] = a.vdiag[i];
-    if (tid < LOGD) sH[tid] = a.hflip[tid];
-    for (int q = tid; q < Q; q += T) {
-        const long long src = n * 2 * a.M + q;
-        sSlab[q] = a.ent_slab[src];
-        sBath[q] = a.ent_bath[src] & 0xffff;
-        sWc[q] = a.ent_wc[src];
-        sWa[q] = a.ent_wa[src];
-    }
-    const R g = static_cast<R>(a.gsum[n]);
-    const int slot = a.slot ? a.slot[n] : -1;
-    const R alpha = static_cast<R>(alpha_d);
-    __syncthreads();
-    bool ok = false;
-    for (uint32_t it = 0; it < kLargeSpin && !ok; ++it) {
-        uint32_t done;
-        asm volatile(
-            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], 0;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-            : "=r"(done)
-            : "r"(l_addr(bar))
-            : "memory");
-        ok = done != 0;
-    }
-    if (__syncthreads_or(!ok)) {
-        if (tid == 0) atomicExch(a.error_flag, 1);
-        return;
-    }
-
-    C acc[E];
-    // ---- diagonal table and transverse field
-#pragma unroll
-    for (int k0 = 0; k0 < E; k0 += CH) {
-        C x[CH], t[CH];
-#pragma unroll
-        for (int kk = 0; kk < CH; ++kk) {
-            x[kk] = sx[tid + T * (k0 + kk)];
-            t[kk] = __ldg(a.diag + be + tid + T * (k0 + kk));
-        }
-#pragma unroll
-        for (int kk = 0; kk < CH; ++kk) {
-            const int e = tid + T * (k0 + kk);
-            const long long ge = be + e;
-            R hr = 0, hi = 0;
-#pragma unroll
-            for (int i = 0; i < LOGD; ++i) {
-                if (sH[i] == R(0)) continue;  // no field on this spin: no gathers
-                constexpr long long one = 1;
-                const long long fb = static_cast<long long>(D) << i;  // row bit i of the element index
-                C rowp;
-                if (fb < BE) rowp = sx[e ^ static_cast<int>(fb)];
-                else rowp = __ldg(un + (ge ^ fb));
-                const C colp = sx[e ^ static_cast<int>(one << i)];
-                hr += sH[i] * (rowp.x - colp.x);
-                hi += sH[i] * (rowp.y - colp.y);
-            }
-            const R tr = t[kk].x - g;
-            acc[k0 + kk].x = tr * x[kk].x - t[kk].y * x[kk].y + hi;
-            acc[k0 + kk].y = tr * x[kk].y + t[kk].y * x[kk].x - hr;
-        }
-    }
-    // ---- neighbour entries, two at a time, CH elements per load batch
-    const C* ub = u + be + tid;
-    int q = 0;
-    for (; q + 1 < Q; q += 2) {
-        const int j0 = sBath[q], j1 = sBath[q + 1];
-        const R wc0 = static_cast<R>(sWc[q]), wa0 = static_cast<R>(sWa[q]);
-        const R wc1 = static_cast<R>(sWc[q + 1]), wa1 = static_cast<R>(sWa[q + 1]);
-        const C* s0 = ub + static_cast<long long>(sSlab[q]) * D2;
-        const C* s1 = ub + static_cast<long long>(sSlab[q + 1]) * D2;
-#pragma unroll
-        for (int k0 = 0; k0 < E; k0 += CH) {
-            C y0[CH], y1[CH];
-            R ar0[CH], ai0[CH], ar1[CH], ai1[CH];
-#pragma unroll
-            for (int kk = 0; kk < CH; ++kk) {
-                const long long ge = be + tid + T * (k0 + kk);
-                const int r = static_cast<int>(ge >> LOGD), c = static_cast<int>(ge & (D - 1));
-                const R vr0 = sV[j0 * D + r], vc0 = sV[j0 * D + c];
-                const R vr1 = sV[j1 * D + r], vc1 = sV[j1 * D + c];
-                ar0[kk] = -(vr0 + vc0) * wa0;
-                ai0[kk] = -(vr0 - vc0) * wc0;
-                ar1[kk] = -(vr1 + vc1) * wa1;
-                ai1[kk] = -(vr1 - vc1) * wc1;
-                y0[kk] = mk<R>(0, 0);
-                y1[kk] = mk<R>(0, 0);
-                if (ar0[kk] != R(0) || ai0[kk] != R(0)) y0[kk] = __ldg(s0 + T * (k0 + kk));
-                if (ar1[kk] != R(0) || ai1[kk] != R(0)) y1[kk] = __ldg(s1 + T * (k0 + kk));
-            }
-#pragma unroll
-            for (int kk = 0; kk < CH; ++kk) {
-                acc[k0 + kk].x += ar0[kk] * y0[kk].x - ai0[kk] * y0[kk].y + ar1[kk] * y1[kk].x - ai1[kk] * y1[kk].y;
-                acc[k0 + kk].y += ar0[kk] * y0[kk].y + ai0[kk] * y0[kk].x + ar1[kk] * y1[kk].y + ai1[kk] * y1[kk].x;
-            }
-        }
-    }
-    if (q < Q) {
-        const int j0 = sBath[q];
-        const R wc0 = static_cast<R>(sWc[q]), wa0 = static_cast<R>(sWa[q]);
-        const C* s0 = ub + static_cast<long long>(sSlab[q]) * D2;
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-            const long long ge = be + tid + T * k;
-            const int r = static_cast<int>(ge >> LOGD), c = static_cast<int>(ge & (D - 1));
-            const R vr0 = sV[j0 * D + r], vc0 = sV[j0 * D + c];
-            const R ar = -(vr0 + vc0) * wa0, ai = -(vr0 - vc0) * wc0;
-            C y = mk<R>(0, 0);
-            if (ar != R(0) || ai != R(0)) y = __ldg(s0 + T * k);
-            acc[k].x += ar * y.x - ai * y.y;
-            acc[k].y += ar * y.y + ai * y.x;
-        }
-    }
-    // ---- up term of tier L-1 (neighbours in the top tier), summed by large_upterm_kernel
-    if (slot >= 0) {
-        const C* Un = a.U + static_cast<long long>(slot) * D2 + be + tid;
-#pragma unroll
-        for (int k = 0; k < E; ++k) {
-            const C w = __ldcs(Un + T * k);
-            acc[k].x += w.x;
-            acc[k].y += w.y;
-        }
-    }
-    // ---- Horner epilogue
-    C* on = out + n * D2 + be + tid;
-    const C* rn = rho + n * D2 + be + tid;
-#pragma unroll
-    for (int k = 0; k < E; ++k) {
-        C b;
-        if (base_kind == kBaseSelf) b = sx[tid + T * k];
-        else if (base_kind == kBaseRho) b = __ldcs(rn + T * k);
-        else b = mk<R>(0, 0);
-        __stcs(on + T * k, mk<R>(b.x + alpha * acc[k].x, b.y + alpha * acc[k].y));
-    }
 }
 
 // ---------------------------------------------------------------------------
@@ -388,8 +209,8 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 }
 
 // ---------------------------------------------------------------------------
-// Tile kernel on Hermitian-packed slabs (layout in hx_internal.h).  A CTA
-// computes one 64 x 64 tile (I, J), I <= J, of one ADO.  What bounds a stage
+// Tile kernel, on full slabs (FULL) or Hermitian-packed ones (layout in
+// hx_internal.h).  A CTA computes one 64 x 64 tile (I, J), packed I <= J, of one ADO.  What bounds a stage
 // is the traffic between L2 and the SMs (64 bytes a cycle each): per element
 // its own value, the flip partners outside the tile, the neighbours, the base
 // and the result.  A square tile keeps the six low bits of row and column
@@ -419,7 +240,9 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 // d = 256, 969 ADOs: 0.69 ms a stage in double, 0.43 in complex64 (bands of
 // rows: 0.94 and 0.56; complex64 without staged tiles and packed arithmetic
 // 0.48).  Double is at 74% of the load-store unit's wavefronts and 7.4 TB/s
-// between L2 and the SMs.  The 64 registers of two CTAs per SM are the limit: one
+// between L2 and the SMs.  Full slabs, us per step, bands of 4096 / d rows
+// against tiles: d = 256, 165 ADOs 1260 and 885 in double, 614 and 500 in
+// complex64; d = 128, 680 ADOs 1226 and 841; 604 and 475.  The 64 registers of two CTAs per SM are the limit: one
 // pass of 8 rows in double spills or leaves one CTA (0.85 ms).
 template <typename R, int LOGD> struct TileShape;
 template <int LOGD> struct TileShape<double, LOGD> { static constexpr int NP = 2, MINB = 2, LR = LOGD == 7 ? 1 : 4; };
@@ -432,6 +255,12 @@ __device__ __forceinline__ int packed_row(int r)
 {
     constexpr int D = 1 << LOGD;
     return r < D / 2 ? r * D : (D - 1 - r) * (D + 1) + 1;
+}
+
+template <int LOGD, bool FULL>
+__device__ __forceinline__ int row_at(int r)
+{
+    return FULL ? r << LOGD : packed_row<LOGD>(r);
 }
 
 // z += w y and x - y, elementwise: one packed instruction each in complex64 (the same roundings).
@@ -541,15 +370,16 @@ __device__ __forceinline__ void stage_tile(const C2<R>* __restrict__ un, int A, 
                          : "memory");
 }
 
-template <typename R, int LOGD, bool PAULI, bool STAGED>
+template <typename R, int LOGD, bool PAULI, bool STAGED, bool FULL>
 __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
-    herm_tile_kernel(LargeArgs<R> a, const C2<R>* __restrict__ u, const C2<R>* rho, C2<R>* out, double alpha_d,
+    tile_kernel(LargeArgs<R> a, const C2<R>* __restrict__ u, const C2<R>* rho, C2<R>* out, double alpha_d,
                      int base_kind)
 {
     using C = C2<R>;
-    constexpr int D = 1 << LOGD, NP = TileShape<R, LOGD>::NP, E = 8 / NP, NBK = D / 64, NT = NBK * (NBK + 1) / 2;
-    constexpr int LR = TileShape<R, LOGD>::LR, LC = 32 / LR;  // rows and columns of a warp's lanes
-    constexpr long long P = static_cast<long long>(D / 2) * (D + 1);
+    constexpr int D = 1 << LOGD, NP = TileShape<R, LOGD>::NP, E = 8 / NP, NBK = D / 64,
+                  NT = FULL ? NBK * NBK : NBK * (NBK + 1) / 2;
+    constexpr int LR = FULL ? 1 : TileShape<R, LOGD>::LR, LC = 32 / LR;  // rows and columns of a warp's lanes
+    constexpr long long P = FULL ? static_cast<long long>(D) * D : static_cast<long long>(D / 2) * (D + 1);
     extern __shared__ __align__(128) unsigned char smem[];
     constexpr int F = 2 * (LOGD - 6);
     C* sx = reinterpret_cast<C*>(smem);                                // [64][64] the tile
@@ -566,17 +396,22 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
     const int tid = threadIdx.x;
     const long long n = a.first_ado + static_cast<long long>(blockIdx.x) / NT;
     int J = 0, I = static_cast<int>(blockIdx.x % NT);
-    while (I > J) I -= ++J;  // tile (I, J) of the upper triangle, column by column
+    if constexpr (FULL) {
+        J = I % NBK;
+        I /= NBK;
+    } else {
+        while (I > J) I -= ++J;  // tile (I, J) of the upper triangle, column by column
+    }
     const C* un = u + n * P;
     const int warp = tid >> 5, lane = tid & 31;
     const int r0 = lane / LC + LR * (warp / (2 * LR));  // rows r0 + 8 k of the tile
     // the second half of the rows is stored shifted by -r mod 8 elements: shifting the columns of a thread
     // the other way keeps eight lanes on one 128-byte line
-    const int c = (lane % LC + LC * (warp % (2 * LR)) + (I * 64 < D / 2 ? 0 : r0)) & 63;
-    const bool diag = I == J;
+    const int c = (lane % LC + LC * (warp % (2 * LR)) + (FULL || I * 64 < D / 2 ? 0 : r0)) & 63;
+    const bool diag = !FULL && I == J;
     const int gc = J * 64 + c, gr0 = I * 64 + r0;
-    const int own = packed_row<LOGD>(gr0) + gc;     // packed position of element k: own + k * step
-    const int step = I * 64 < D / 2 ? 8 * D : -8 * (D + 1);
+    const int own = row_at<LOGD, FULL>(gr0) + gc;     // packed position of element k: own + k * step
+    const int step = FULL || I * 64 < D / 2 ? 8 * D : -8 * (D + 1);
 
     // ---- the tile (both triangles of a diagonal one)
     [[maybe_unused]] int fl = 0;  // the next flip to stage, or past the last one
@@ -682,19 +517,20 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
             const R h = sH[6 + (f >> 1)];
             const R w = f & 1 ? -h : h;
             C y[E];
-            if (A == B) {
+            if (!FULL && A == B) {
                 const int rb = A * 64 + r0 + 8 * k0, cb = B * 64 + c;
 #pragma unroll
                 for (int k = 0; k < E; ++k) y[k] = on[k] ? packed_at(un, rb + 8 * k, cb, LOGD) : mk<R>(0, 0);
             } else {
                 // above the diagonal directly, below it the transposed place
-                const int at = A < B ? packed_row<LOGD>(A * 64 + r0) + B * 64 + c : packed_row<LOGD>(B * 64 + c) + A * 64 + r0;
-                const int st = A < B ? (A * 64 < D / 2 ? 8 * D : -8 * (D + 1)) : 8;
+                const bool up = FULL || A < B;
+                const int at = up ? row_at<LOGD, FULL>(A * 64 + r0) + B * 64 + c : packed_row<LOGD>(B * 64 + c) + A * 64 + r0;
+                const int st = up ? (FULL || A * 64 < D / 2 ? 8 * D : -8 * (D + 1)) : 8;
                 const C* src = un + at + k0 * st;
 #pragma unroll
                 for (int k = 0; k < E; ++k) y[k] = on[k] ? __ldg(src + k * st) : mk<R>(0, 0);
             }
-            const R wy = A > B ? -w : w;
+            const R wy = !FULL && A > B ? -w : w;
 #pragma unroll
             for (int k = 0; k < E; ++k) {
                 z[k].x += w * y[k].x;
@@ -997,13 +833,6 @@ size_t tile_smem(int M, int J, bool pauli, bool staged)
            sizeof(R) * (LOGD + 4 * M) + sizeof(int) * 4 * M;
 }
 
-template <typename R, int LOGD>
-size_t large_smem(int M, int J)
-{
-    return 4096 * sizeof(C2<R>) + 16 + sizeof(double) * 4 * M + sizeof(R) * (J * (1 << LOGD) + LOGD + 1) +
-           sizeof(int) * 4 * M + 16;
-}
-
 // Stage of a dense H; launch = false: raise the shared-memory limit only.
 template <int LOGD>
 bool launch_dense(const LargeArgs<float>& a, const float2* u, const float2* rho, float2* out, double alpha, int base,
@@ -1029,23 +858,23 @@ bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* ou
     using Kernel = void (*)(LargeArgs<R>, const C2<R>*, const C2<R>*, C2<R>*, double, int);
     // complex64: partner tiles are staged where two CTAs per SM still find room for the buffers
     constexpr bool kStage = sizeof(R) == sizeof(float);
-    const bool staged = kStage && tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0, true) <= 113 * 1024;
-    Kernel kernel = large_kernel<R, LOGD>;
-    size_t smem = large_smem<R, LOGD>(a.M, a.J);
-    if (a.herm) {
-        smem = tile_smem<R, LOGD>(a.M, a.J, a.pauli != 0, staged);
-        if (staged) kernel = a.pauli ? herm_tile_kernel<R, LOGD, true, kStage> : herm_tile_kernel<R, LOGD, false, kStage>;
-        else kernel = a.pauli ? herm_tile_kernel<R, LOGD, true, false> : herm_tile_kernel<R, LOGD, false, false>;
-    }
+    // one coupling: the two tables of the sigma_z form are longer than the operator's, which may be what fits
+    const bool pauli = a.pauli && tile_smem<R, LOGD>(a.M, a.J, true, false) <= 227 * 1024;
+    const bool staged = kStage && a.herm && tile_smem<R, LOGD>(a.M, a.J, pauli, true) <= 113 * 1024;
+    const size_t smem = tile_smem<R, LOGD>(a.M, a.J, pauli, staged);
+    Kernel kernel;
+    if (!a.herm) kernel = pauli ? tile_kernel<R, LOGD, true, false, true> : tile_kernel<R, LOGD, false, false, true>;
+    else if (staged) kernel = pauli ? tile_kernel<R, LOGD, true, kStage, false> : tile_kernel<R, LOGD, false, kStage, false>;
+    else kernel = pauli ? tile_kernel<R, LOGD, true, false, false> : tile_kernel<R, LOGD, false, false, false>;
     if (smem > 227 * 1024) return false;
     // the limit is raised when a context is made, outside any capture
     if (!launch)
         return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) == cudaSuccess;
-    // full slabs: d^2 / 4096 bands each; packed slabs: the tiles of the upper triangle
+    // packed slabs: the tiles of the upper triangle
     constexpr long long kBlocks = (1 << LOGD) / 64;
-    const long long nb = (a.H - a.first_ado) * (a.herm ? kBlocks * (kBlocks + 1) / 2 : (1ll << (2 * LOGD)) / 4096);
+    const long long nb = (a.H - a.first_ado) * (a.herm ? kBlocks * (kBlocks + 1) / 2 : kBlocks * kBlocks);
     if (nb <= 0) return true;
-    kernel<<<static_cast<unsigned>(nb), a.herm ? kTileT : LargeThreads<R>::T, smem, s>>>(a, u, rho, out, alpha, base);
+    kernel<<<static_cast<unsigned>(nb), kTileT, smem, s>>>(a, u, rho, out, alpha, base);
     return true;
 }
 

@@ -182,3 +182,32 @@ def test_mixed_precision_packed_rhs_at_every_tile_grid(n, baths, K, collective):
         cm.set_state(x)
         r = cm.rhs()
         assert np.max(np.abs(r - ref)) < 1e-5 * np.max(np.abs(ref))
+
+
+@pytest.mark.parametrize("precision,tol", [("double", 1e-12), ("mixed", 1e-5)])
+@pytest.mark.parametrize("n,baths,K,collective", [
+    (7, 3, 1, True),
+    (8, 3, 1, False),
+    (9, 2, 0, False),
+    (10, 1, 0, True),   # four bits outside a tile
+])
+def test_full_slab_rhs_at_every_tile_grid(n, baths, K, collective, precision, tol):
+    """Tiles of full slabs (no Hermiticity used), a different field on every
+    spin: the right-hand side against the oracle, within the bounds of the
+    tests above."""
+    p = S.spin_glass(n, seed=60 + n, depth=2, K=K, h=0.5, dt=0.005)
+    rng = np.random.default_rng(n)
+    p.h_flip = rng.uniform(0.2, 1.0, n)
+    p.baths = p.baths[:baths]
+    if collective:
+        for b in p.baths:
+            b.v_diag = rng.uniform(-0.7, 0.7, p.dim)
+    o = O.Oracle(p)
+    x = (rng.standard_normal((o.size, p.dim, p.dim)) + 1j * rng.standard_normal((o.size, p.dim, p.dim))) * 0.05
+    ref = o.rhs(x)
+    o.close()
+    with capi.Context(p, precision=precision, full_state=True) as ctx:
+        assert not ctx.hermitian_packed
+        ctx.set_state(x)
+        r = ctx.rhs()
+        assert np.max(np.abs(r - ref)) < tol * max(1.0, np.max(np.abs(ref)))
