@@ -250,7 +250,7 @@ def stage_kernels_label(ctx, p, packed: bool, per_stage: int) -> str:
             (" (Hermitian-packed slabs)" if packed else "")
     if path == "small":
         if int(ctx.info.kernels_per_step) == 1:
-            return "small_run_kernel (d <= 16; whole steps in one launch, grid barriers between the stages)"
+            return "small_step_kernel per step (d <= 16; steps in one launch, grid barriers between the stages)"
         return "small_kernel per stage (d <= 16, batched neighbour gathers)"
     return "stage_kernel per stage (generic path)"
 
@@ -486,7 +486,7 @@ def run_ours(args, cfg: dict) -> None:
     stages = 4
     alg_bytes_per_step = (3 * stages - 1) * state_bytes
     # launches per step: one per stage, or one for the whole step (small_step_kernel)
-    step_launch = ctx.stage_path == "small" and int(ctx.info.kernels_per_step) == 1
+    step_launch = ctx.stage_path in ("small", "fused") and int(ctx.info.kernels_per_step) == 1
     launches_per_step = 1 if step_launch else stages
     per_launch_bytes = alg_bytes_per_step / launches_per_step
     launch_ms = ms / (args.steps * launches_per_step)
@@ -494,7 +494,7 @@ def run_ours(args, cfg: dict) -> None:
     peak, peak_kind = load_peaks()
     packed = bool(ctx.hermitian_packed)
     kernel = ("small_step_kernel" if step_launch else "small_kernel") if ctx.stage_path == "small" \
-        else ("herm_kernel" if packed else "fused_kernel")
+        else ("herm_run_kernel" if step_launch else "herm_kernel" if packed else "fused_kernel")
     # DRAM bytes of one stage: the stage kernel plus the up-term kernel (committed ncu summaries)
     traffic = profiled_traffic(args.config, kernel)
     traffic_files = [f"profiles/{kernel}_{args.config}_ncu.txt"]

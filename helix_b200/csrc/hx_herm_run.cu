@@ -18,7 +18,7 @@
 //    (herm_kernel's layout) while they are under way.  Up neighbours are
 //    entries like the others (they hit L2), so there is no up-term pass;
 //  * a barrier over the grid separates the stages, and the last CTA only
-//    watches (records rho_0 and the observables), as in small_run_kernel;
+//    watches (records rho_0 and the observables), as in small_step_kernel;
 //  * a closure's term is a second diagonal coefficient of the top-tier ADOs.
 //
 // us per step, a launch per pass against a run: 92 and 25 at d = 32, 136 ADOs

@@ -180,7 +180,7 @@ void launch_transpose_bf16(const void* in, int rows, int cols, int ld_in, void* 
 // d <= 16, full slabs, sigma_z couplings, every up term in the entry lists: batched gathers (hx_small.cu)
 size_t small_smem(int logd, int M);
 bool small_supported(int logd, int M, int pauli);
-// Grid-barrier waits of small_run_kernel: polls before giving up (and setting the error word), and an
+// Grid-barrier waits of small_step_kernel: polls before giving up (and setting the error word), and an
 // offset added to every barrier's arrival target (nonzero only to make the waits run out on purpose).
 struct StepWait {
     unsigned skew = 0;
@@ -456,7 +456,7 @@ struct hx_ctx {
     // fused stage-kernel tables (d = 32, 64)
     bool use_fused = false;
     bool use_small = false;       // d <= 16 sigma_z stage kernel (hx_small.cu)
-    bool use_run = false;         // whole steps in one launch (small_run_kernel, herm_run_kernel)
+    bool use_run = false;         // whole steps in one launch (small_step_kernel, herm_run_kernel)
     unsigned* gbar = nullptr;     // their grid-barrier arrival counter
     bool stall_next_step = false; // hx_ctx_inject_wait_timeout: the next step's barriers cannot complete
     int sm_count = 0;

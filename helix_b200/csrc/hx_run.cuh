@@ -1,5 +1,5 @@
 // What the kernels that run whole integrator steps in one launch share
-// (small_run_kernel in hx_small.cu, herm_run_kernel in hx_herm_run.cu): the
+// (small_step_kernel in hx_small.cu, herm_run_kernel in hx_herm_run.cu): the
 // barrier over the grid and the reduction of the observables by one warp.
 #ifndef HX_RUN_CUH
 #define HX_RUN_CUH

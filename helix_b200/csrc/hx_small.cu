@@ -1,4 +1,4 @@
-// Kernels for small slabs (d <= 16): small_run_kernel, whole integrator steps
+// Kernels for small slabs (d <= 16): small_step_kernel, whole integrator steps
 // in one launch, and small_kernel, one stage per launch with sigma_z couplings
 // (single right-hand sides, and hierarchies too large for the resident CTAs).
 //
@@ -151,7 +151,7 @@ void launch_small_t(const FusedArgs& a, const double2* u, const double2* rho, do
     small_kernel<LOGD><<<static_cast<unsigned>(a.H), threads, smem, s>>>(a, u, rho, out, alpha, base);
 }
 
-// Elements of a slab that one thread of small_run_kernel owns, and threads per slab.
+// Elements of a slab that one thread of small_step_kernel owns, and threads per slab.
 template <int LOGD> struct RunShape {
     static constexpr int E = LOGD == 4 ? 2 : 1;
     static constexpr int TA = (1 << (2 * LOGD)) / E;
@@ -194,7 +194,7 @@ constexpr int kRunBatch = 4;  // staged entries read back side by side
 // and the diagonal term comes from the table a.diag.
 template <int LOGD, bool PAULI, bool SOLO>
 __global__ void __launch_bounds__(kRunThreads, 1)
-    small_run_kernel(FusedArgs a, RunClosure cl, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
+    small_step_kernel(FusedArgs a, RunClosure cl, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
                      int apc, int per, int cap, unsigned* gcount, StepWait w, double2* trace, double* obs)
 {
     constexpr int D = 1 << LOGD, D2 = D * D, E = RunShape<LOGD>::E, TA = RunShape<LOGD>::TA;
@@ -527,7 +527,7 @@ template <int LOGD, bool PAULI, bool SOLO>
 int launch_run_t(const RunPlan& p, const FusedArgs& a, const RunClosure& cl, double2* rho, double2* ua, double2* ub, double dt, int order,
                  int nsteps, unsigned* gcount, StepWait w, double2* trace, double* obs, cudaStream_t s)
 {
-    auto* kernel = small_run_kernel<LOGD, PAULI, SOLO>;
+    auto* kernel = small_step_kernel<LOGD, PAULI, SOLO>;
     FusedArgs args = a;
     RunClosure clo = cl;
     int apc = p.apc, per = p.per, cap = p.cap;
@@ -551,10 +551,10 @@ int launch_run_d(const RunPlan& p, const FusedArgs& a, const RunClosure& cl, dou
             return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kRunSmem)) ==
                    cudaSuccess;
         };
-        const bool ok = a.pauli ? raise(reinterpret_cast<const void*>(small_run_kernel<LOGD, true, true>)) &&
-                                      raise(reinterpret_cast<const void*>(small_run_kernel<LOGD, true, false>))
-                                : raise(reinterpret_cast<const void*>(small_run_kernel<LOGD, false, true>)) &&
-                                      raise(reinterpret_cast<const void*>(small_run_kernel<LOGD, false, false>));
+        const bool ok = a.pauli ? raise(reinterpret_cast<const void*>(small_step_kernel<LOGD, true, true>)) &&
+                                      raise(reinterpret_cast<const void*>(small_step_kernel<LOGD, true, false>))
+                                : raise(reinterpret_cast<const void*>(small_step_kernel<LOGD, false, true>)) &&
+                                      raise(reinterpret_cast<const void*>(small_step_kernel<LOGD, false, false>));
         if (ok) raised[a.pauli ? 1 : 0][dev].store(true);
         return ok ? 1 : -1;
     }
