@@ -324,16 +324,20 @@ int launch_herm_run(const FusedArgs& a, const RunClosure& cl, double2* rho, doub
 #undef HX_RUN
 }
 
-// The line between a run and a launch per pass: while the three state buffers
-// fit L2 together the run is ahead (us per step, launches against run: d = 32,
-// 39 MiB of state 305 and 297, 31 MiB 245 and 234; d = 64, 26 MiB 210 and 197,
-// 16 MiB 148 and 146, but 42 MiB 304 and 342, 58 MiB 408 and 464, where one
-// CTA of 704 threads per SM hides less latency than herm_kernel's two).
+// The line between a run and a launch per pass: a run saves the launches and
+// the up-term pass, but its CTAs hide less latency than herm_kernel's.  us per
+// step, launches against run: d = 32, 1.1 MiB of state 91 and 23, 6.6 MiB 106
+// and 61, 13.8 MiB 120 and 105, 24 MiB 171 and 192, 31 MiB 226 and 235; d = 64,
+// 6 MiB 134 and 60, 14.4 MiB 142 and 107, 23 MiB 160 and 169, so the line lies
+// at 18 MiB for both.  (Runs of several contexts on several streams wait for
+// one another, their launches overlap: 24 contexts of 816 ADOs at d = 32 take
+// 59 us a step and context in runs and 37 without, of 136 ADOs 23 and 24;
+// HX_SMALL_STEP=0 leaves the runs out, and a batch never uses them.)
 bool herm_run_fits(int logd, int M, int J, int pauli, long long H, int sms)
 {
     HermRunPlan p;
     const long long state = H * herm_elems(logd) * static_cast<long long>(sizeof(double2));
-    return plan_herm_run(logd, M, J, pauli != 0, H, sms, p) && state <= (logd == 5 ? 40ll << 20 : 26ll << 20);
+    return plan_herm_run(logd, M, J, pauli != 0, H, sms, p) && state <= 18ll << 20;
 }
 
 }  // namespace hx

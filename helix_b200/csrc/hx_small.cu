@@ -520,7 +520,9 @@ bool plan_run(int logd, int M, int J, bool pauli, long long H, int sms, bool sol
     const size_t slab = static_cast<size_t>(d2) * sizeof(double2);
     p.cap = static_cast<int>(std::min<size_t>(static_cast<size_t>(p.apc) * 2 * M, (kRunSmem - p.smem) / slab));
     p.smem += p.cap * slab;
-    return p.cap >= p.apc;
+    // with less room than three entries per slab in hand the run waits on every entry by itself: d = 16, 12 modes,
+    // 1820 ADOs 120 us a step, 68 with a launch per stage; 1716 ADOs, where 18 entries fit, 47 and 67
+    return p.cap >= 3 * p.apc;
 }
 
 template <int LOGD, bool PAULI, bool SOLO>
