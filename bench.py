@@ -241,7 +241,7 @@ def stage_kernels_label(ctx, p, packed: bool, per_stage: int) -> str:
     if path == "csr":
         return "csr_comm_kernel + csr_combine_kernel per stage (general sparse operators)"
     if path == "band":
-        return "band kernels per stage" + (" (Hermitian-packed slabs)" if packed else "")
+        return "tile_kernel per stage" + (" (Hermitian-packed slabs)" if packed else "")
     if path == "fused" and int(ctx.info.kernels_per_step) == 1:
         return f"herm_run_kernel<{logd}> (whole steps in one cooperative launch, Hermitian-packed slabs)"
     if path == "fused":

@@ -249,7 +249,7 @@ hx::Ado0Args ado0_args(const hx_ctx* c)
 // Index of a state buffer of the context: 0 = rho, 1 = ua, 2 = ub.
 int buffer_id(const hx_ctx* c, const double2* p) { return p == c->rho ? 0 : (p == c->ua ? 1 : 2); }
 
-// Dense H: Y_n = X_n H_off (H without its diagonal, which the band kernels
+// Dense H: Y_n = X_n H_off (H without its diagonal, which the tile kernels
 // apply exactly) for every ADO of the complex64 stage input u32, as the real
 // product [H d x 2d] x [2d x 2d] (interleaved complex rows of X times the
 // real form of H_off) in 3-term TF32 split form, X_hi H_hi + X_hi H_lo +
@@ -265,8 +265,8 @@ int launch_dense_product(hx_ctx* c, const float2* u32)
     return 1;
 }
 
-// One stage of the band kernels (hx_large.cu): the up-term kernel of tier
-// L-1, the band kernel over the hierarchy and, in mixed precision, the
+// One stage of the tile kernels (hx_large.cu): the up-term kernel of tier
+// L-1, the tile kernel over the hierarchy and, in mixed precision, the
 // double-precision kernel of ADO 0 (with a dense H, the tensor-core product
 // first).  Returns kernels launched.
 int launch_large_stage(hx_ctx* c, const double2* u, const double2* rho, double2* out, double alpha, int base)
@@ -767,7 +767,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
         return fail(HX_ERR_INVALID_RUNTIME_OPTION, "unknown flags");
 
     const int J = static_cast<int>(p->n_baths);
-    // dense H on the tensor cores: the band kernels see only the diagonal of
+    // dense H on the tensor cores: the tile kernels see only the diagonal of
     // H, the rest is applied as matrix products before every stage
     const bool want_dense = (p->flags & HX_FLAG_DENSE_H) != 0;
     HostCsr dense_h;
@@ -783,7 +783,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
         } else {
             dense_h = flip_csr(p->h_diag, p->h_flip, static_cast<int>(d), logd);
         }
-        // the real diagonal of H stays exact in the band kernels' diagonal table; the
+        // the real diagonal of H stays exact in the tile kernels' diagonal table; the
         // products carry only the off-diagonal part (smaller terms, smaller rounding)
         dense_diag.assign(d, 0.0);
         for (uint32_t r = 0; r < d; ++r)
@@ -1175,7 +1175,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
                 if (rc == HX_OK && c->use_run && (rc = dev_alloc(c, &c->order_perm, H)) == HX_OK)
                     hx::launch_run_order(c->ent_count, c->H, c->order_perm, c->stream);
             }
-            // single-precision copies of the operators for the mixed band kernel
+            // single-precision copies of the operators for the mixed tile kernel
             if (rc == HX_OK && c->mixed) {
                 if ((rc = dev_alloc(c, &c->diag32, c->slab)) || (rc = dev_alloc(c, &c->vdiag32, static_cast<size_t>(J) * d)) ||
                     (rc = dev_alloc(c, &c->hflip32, logd))) {
@@ -1212,10 +1212,10 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
         }
     }
     if (rc == HX_OK && c->use_large && (c->diag_table == nullptr || c->ent_count == nullptr))
-        rc = fail(HX_ERR_UNSUPPORTED_EXECUTION, "band-kernel tables were not built");
+        rc = fail(HX_ERR_UNSUPPORTED_EXECUTION, "tile-kernel tables were not built");
     if (rc == HX_OK && c->use_large) {
         const bool ok = c->mixed ? hx::prepare_large<float>(large_args32(c)) : hx::prepare_large<double>(large_args64(c));
-        if (!ok) rc = fail(HX_ERR_UNSUPPORTED_EXECUTION, "band kernel does not fit in shared memory");
+        if (!ok) rc = fail(HX_ERR_UNSUPPORTED_EXECUTION, "tile kernel does not fit in shared memory");
     }
     if (rc == HX_OK && c->mixed) {
         e = cudaStreamCreateWithFlags(&c->side_stream, cudaStreamNonBlocking);

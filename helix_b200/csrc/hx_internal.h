@@ -434,7 +434,7 @@ struct hx_ctx {
     int32_t* csr_ptr = nullptr;   // [(J+1)(d+1)] operator 0 = H, 1 + j = V_j
     int32_t* csr_col = nullptr;
     double2* csr_val = nullptr;
-    bool use_large = false;       // band kernels for 128 <= d <= 1024, diagonal V (hx_large.cu)
+    bool use_large = false;       // tile kernels for 128 <= d <= 1024, diagonal V (hx_large.cu)
     bool mixed = false;           // complex64 hierarchy, ADO 0 in double precision
     hx_closure* closure = nullptr; // learned closure term added by every stage (hx_mlp.cu)
     double2* cl_coef = nullptr;   // [top-tier ADOs][slab_store] its coefficients, of table build cl_build
