@@ -510,6 +510,10 @@ bool plan_run(int logd, int M, int J, bool pauli, long long H, int sms, bool sol
     const long long each = std::max<long long>((H + ctas - 1) / ctas, std::max(1, 256 / d2));
     if (each > 64ll * most) return false;
     p.per = static_cast<int>((each + most - 1) / most);
+    // general couplings read their weights per element and entry, and one round of slabs is what a run gains on
+    // them: us a step, run against a launch per stage, d = 16, one bath, 495 ADOs 29 and 37, 715 (two rounds) 42
+    // and 37, 1716 71 and 59; d = 8 924 22 and 34, 3003 (three rounds) 45 and 42
+    if (!pauli && p.per > 1) return false;
     p.apc = static_cast<int>((each + p.per - 1) / p.per);
     p.solo = false;
     p.grid = static_cast<int>((H + static_cast<long long>(p.apc) * p.per - 1) / (static_cast<long long>(p.apc) * p.per));
