@@ -1198,16 +1198,16 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     cudaFree(dtc);
     cudaFree(dta);
     // sparse operators at d <= 64: a slab per CTA when the operators fit beside it; couplings with flips run
-    // whole steps in one launch
+    // whole steps in one launch where that is ahead, else the two-pass kernels
     if (rc == HX_OK && (c->use_csr || flip_slab) && logd <= hx::kMaxLogD && hx::prepare_slab(csr_args_of(c), c->csr_nnz)) {
-        c->use_slab = true;
+        c->use_slab = c->use_csr;
         if (flip_slab && c->order >= 2) {
             cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
             c->slab_ctas = hx::slab_run_ctas(csr_args_of(c), c->csr_nnz, c->sm_count);
-            if (c->slab_ctas > 0 && (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
+            if (c->slab_ctas >= c->H && (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
                 e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
                 if (e != cudaSuccess) rc = hx::cuda_fail(e, "grid barrier counter");
-                else c->use_run = true;
+                else c->use_slab = c->use_run = true;
             }
         }
     }

@@ -413,20 +413,24 @@ int launch_slab_run_t(const CsrArgs& a, int nnz, int ctas, double2* rho, double2
     default: return 0;            \
     }
 
-// At d = 64 a slab is two waves of work for one CTA, so the two-pass kernels,
-// which spread every ADO over the GPU, stay ahead for few ADOs and baths (us per
-// step, two passes against a slab per CTA, at ADOs x baths = 78: 240 and 373, 84:
-// 186 and 235, 126: 146 and 137, 165: 308 and 263, 546: 660 and 450).
+// At d = 64 the two-pass kernels, which spread every ADO over the GPU, stay ahead while most SMs would have no
+// slab: us per four steps, two passes against a slab per CTA, 28 ADOs of six baths 1066 and 1522, 35 of four 839
+// and 1123, 45 of four 1131 and 1102, 55 of three 1215 and 990, 91 of six 2588 and 1779; at d = 32 a slab per
+// CTA is ahead from 2 ADOs (299 and 297) on, 20 ADOs 531 and 436.
 int prepare_slab(const CsrArgs& a, int nnz)
 {
-    if (a.logd == 6 && a.H * a.J < 120) return 0;
+    if (a.logd == 6 && a.H < 45) return 0;
 #define HX_CALL(L) (prepare_slab_t<L>(a.J, nnz) ? 1 : 0)
     HX_SLAB_SWITCH(HX_CALL)
 #undef HX_CALL
 }
 
+// Couplings with flips run whole steps while every ADO has a CTA of its own (an SM of its own at d = 32); at
+// d = 64 two passes with four rows per thread are ahead at any count (us per four steps, two passes against a run:
+// 20 ADOs 275 and 517, 126 502 and 626; d = 32, 126 ADOs 290 and 204, 210 311 and 322, 495 474 and 590).
 int slab_run_ctas(const CsrArgs& a, int nnz, int sms)
 {
+    if (a.logd == 6 || (a.logd == 5 && a.H > sms - 1)) return 0;
 #define HX_CALL(L) run_ctas_t<L>(a, nnz, sms)
     HX_SLAB_SWITCH(HX_CALL)
 #undef HX_CALL
