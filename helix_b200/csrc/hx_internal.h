@@ -270,6 +270,7 @@ struct LargeArgs {
     // -i[H_off, X_n]_rc = -i(conj(Y_cr) - Y_rc)
     const C2<R>* dense_y;
     int dense;               // 1: a dense-H context (dense_tile_kernel)
+    int halves;              // 1: two CTAs per tile, one per half of its rows (set at the launch, tile_kernel)
 };
 template <typename R>
 struct LargeUpArgs {
