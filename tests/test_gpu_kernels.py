@@ -160,7 +160,9 @@ def test_whole_step_runs_match_oracle(n, baths, K, depth, collective):
     want = o.state()
     o.close()
     with capi.Context(p) as a, capi.Context(p) as b:
-        assert a.get_info().kernels_per_step == 1
+        # general couplings at d = 16: one round of four slabs in each of 147 CTAs, else a launch per stage
+        one = not (collective and n == 4 and a.size > 588)
+        assert a.get_info().kernels_per_step == (1 if one else 4)
         rho, en = a.step_trace(steps)
         b.step(steps)
         b.sync()

@@ -211,3 +211,36 @@ def test_full_slab_rhs_at_every_tile_grid(n, baths, K, collective, precision, to
         ctx.set_state(x)
         r = ctx.rhs()
         assert np.max(np.abs(r - ref)) < tol * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("n,baths,K,collective", [
+    (7, 3, 1, False),   # 28 ADOs, 84 tiles: two CTAs per tile
+    (7, 7, 0, True),    # 36 ADOs, 108 tiles
+    (8, 2, 0, False),   # 6 ADOs, 60 tiles
+    (8, 4, 0, True),    # 15 ADOs, 150 tiles: just more than 148, one CTA per tile
+])
+def test_few_packed_tiles_match_oracle(n, baths, K, collective):
+    """Packed double-precision tiles around the number of SMs: right-hand side
+    within 1e-12 of its largest element, two steps within 1e-10."""
+    p = S.spin_glass(n, seed=80 + n, depth=2, K=K, h=0.5, dt=0.005)
+    rng = np.random.default_rng(n)
+    p.h_flip = rng.uniform(0.2, 1.0, n)
+    p.baths = p.baths[:baths]
+    if collective:
+        for b in p.baths:
+            b.v_diag = rng.uniform(-0.7, 0.7, p.dim)
+    o = O.Oracle(p)
+    x = _hermitian((rng.standard_normal((o.size, p.dim, p.dim)) + 1j * rng.standard_normal((o.size, p.dim, p.dim))) * 0.05)
+    ref = o.rhs(x)
+    o.set_state(x)
+    o.run(2)
+    want = o.state()
+    o.close()
+    with capi.Context(p) as ctx:
+        assert ctx.hermitian_packed
+        ctx.set_state(x)
+        r = ctx.rhs()
+        assert np.max(np.abs(r - ref)) < 1e-12 * max(1.0, np.max(np.abs(ref)))
+        ctx.step(2)
+        ctx.sync()
+        assert np.max(np.abs(ctx.state() - want)) < TOL
