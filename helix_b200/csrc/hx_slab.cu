@@ -367,10 +367,11 @@ bool prepare_slab_t(int J, int nnz)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     if (raised[dev].load()) return true;
-    const bool ok = cudaFuncSetAttribute(slab_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(kSlabSmem)) == cudaSuccess &&
-                    cudaFuncSetAttribute(slab_run_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         static_cast<int>(kSlabSmem)) == cudaSuccess;
+    bool ok = cudaFuncSetAttribute(slab_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                   static_cast<int>(kSlabSmem)) == cudaSuccess;
+    if constexpr (LOGD < 6)
+        ok = ok && cudaFuncSetAttribute(slab_run_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                        static_cast<int>(kSlabSmem)) == cudaSuccess;
     if (ok) raised[dev].store(true);
     return ok;
 }
@@ -402,15 +403,15 @@ int launch_slab_run_t(const CsrArgs& a, int nnz, int ctas, double2* rho, double2
 
 }  // namespace
 
-#define HX_SLAB_SWITCH(CALL)      \
-    switch (a.logd) {             \
-    case 1: return CALL(1);       \
-    case 2: return CALL(2);       \
-    case 3: return CALL(3);       \
-    case 4: return CALL(4);       \
-    case 5: return CALL(5);       \
-    case 6: return CALL(6);       \
-    default: return 0;            \
+#define HX_SLAB_SWITCH(CALL, LAST) \
+    switch (a.logd) {              \
+    case 1: return CALL(1);        \
+    case 2: return CALL(2);        \
+    case 3: return CALL(3);        \
+    case 4: return CALL(4);        \
+    case 5: return CALL(5);        \
+    case 6: return LAST;           \
+    default: return 0;             \
     }
 
 // At d = 64 the two-pass kernels, which spread every ADO over the GPU, stay ahead while most SMs would have no
@@ -421,7 +422,7 @@ int prepare_slab(const CsrArgs& a, int nnz)
 {
     if (a.logd == 6 && a.H < 45) return 0;
 #define HX_CALL(L) (prepare_slab_t<L>(a.J, nnz) ? 1 : 0)
-    HX_SLAB_SWITCH(HX_CALL)
+    HX_SLAB_SWITCH(HX_CALL, HX_CALL(6))
 #undef HX_CALL
 }
 
@@ -432,7 +433,7 @@ int slab_run_ctas(const CsrArgs& a, int nnz, int sms)
 {
     if (a.logd == 6 || (a.logd == 5 && a.H > sms - 1)) return 0;
 #define HX_CALL(L) run_ctas_t<L>(a, nnz, sms)
-    HX_SLAB_SWITCH(HX_CALL)
+    HX_SLAB_SWITCH(HX_CALL, 0)
 #undef HX_CALL
 }
 
@@ -440,7 +441,7 @@ int launch_slab_run(const CsrArgs& a, int nnz, int ctas, double2* rho, double2* 
                     int nsteps, unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs, cudaStream_t s)
 {
 #define HX_CALL(L) launch_slab_run_t<L>(a, nnz, ctas, rho, ua, ub, dt, order, nsteps, gcount, error_flag, w, trace, obs, s)
-    HX_SLAB_SWITCH(HX_CALL)
+    HX_SLAB_SWITCH(HX_CALL, 0)
 #undef HX_CALL
 }
 
@@ -453,7 +454,7 @@ int launch_slab_stage(const CsrArgs& a, int nnz, const double2* u, double2* G, c
     (slab_kernel<L><<<static_cast<unsigned>(a.H), SlabShape<L>::T, slab_smem<L>(a.J, nnz), s>>>(a, nnz, u, G, rho, out, \
                                                                                                 alpha, base_kind),     \
      2)
-    HX_SLAB_SWITCH(HX_CALL)
+    HX_SLAB_SWITCH(HX_CALL, HX_CALL(6))
 #undef HX_CALL
 }
 
