@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(256, 1)
     }
 
     // ---- epilogue, 16 columns of one row per lane at a time
-    const bool done = mbar_wait(done_bar, 0);
+    const bool done = __all_sync(0xffffffffu, mbar_wait(done_bar, 0));  // the same for the whole warp
     if (!done && threadIdx.x == 0) atomicExch(err, 1);
     if (warp == 0 && lane == 0) {
         int consumed;
@@ -251,6 +251,7 @@ __global__ void __launch_bounds__(256, 1)
                                          reinterpret_cast<uintptr_t>(o.aux)) % 16 == 0;
     for (int c0 = half * (BN / 2); c0 < (half + 1) * (BN / 2); c0 += 16) {
         uint32_t v[16];
+        __syncwarp();  // the loads are .sync.aligned: lanes past the last row left the pass before early
         asm volatile(
             "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
             "%14, %15}, [%16];"
@@ -532,7 +533,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1)
             const int x = i & 1;
             int m0, n0;
             tile_of(i, m0, n0);
-            if (!mbar_wait(accf_bar(x), static_cast<uint32_t>((i >> 1) & 1))) {
+            if (!__all_sync(0xffffffffu, mbar_wait(accf_bar(x), static_cast<uint32_t>((i >> 1) & 1)))) {
                 atomicExch(err, 1);
                 break;
             }
