@@ -58,7 +58,7 @@ void release(hx_ctx* c)
                     c->up_slab, c->up_bath, c->U, c->vflip, c->Bbuf, c->rho32, c->ua32, c->ub32,
                     c->U32, c->diag32, c->vdiag32, c->hflip32, c->diag_herm, c->vbit, c->csr_ptr, c->csr_col,
                     c->csr_val, c->pack_scale, c->pack_bad, c->dense_hr, c->dense_hr_lo, c->dense_y,
-                    c->dense_h64, c->dense_z0, c->gbar, c->cl_coef, c->cl_slot, c->xsum, c->obs_csr};
+                    c->dense_h64, c->dense_z0, c->gbar, c->xsum, c->obs_csr};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);

@@ -310,11 +310,13 @@ void launch_vec_d2f(const double* in, float* out, long long n, cudaStream_t s);
 // Whether a closure was made for a hierarchy of this dimension, mode count and size (hx_mlp.cu)
 bool closure_matches_hierarchy(const ::hx_closure* cl, int d, int M, long long H);
 // The closure of a context (hx_mlp.cu).  The dropped up coupling of a top-tier ADO is elementwise and linear
-// in it, so it is one complex coefficient per element of each top-tier ADO, kept per context.
-// closure_attach: room for them and the slot of every ADO (cl = nullptr: give both back).
+// in it, so it is one complex coefficient per element of each top-tier ADO.  The closure owns them, in the slab
+// layout of the contexts it is attached to: they keep their place when the network is trained again or the
+// context takes another closure, so a captured step reads what an eager one does.
+// closure_attach: room for the coefficients and the slot of every ADO (cl = nullptr: detach).
 int closure_attach(::hx_closure* cl, ::hx_ctx* c);
-// Bring the coefficients up to date with the network (on the context's stream); c->cl_on tells whether
-// there is a term to add.
+// Bring the coefficients up to date with the network, complete on return; c->cl_on tells whether there is a
+// term to add.
 int closure_update(::hx_ctx* c);
 // out_top += alpha * coefficient * u_top, after a stage.
 void closure_stage(const ::hx_ctx* c, const double2* u, double2* out, double alpha);
@@ -438,9 +440,8 @@ struct hx_ctx {
     bool use_large = false;       // tile kernels for 128 <= d <= 1024, diagonal V (hx_large.cu)
     bool mixed = false;           // complex64 hierarchy, ADO 0 in double precision
     hx_closure* closure = nullptr; // learned closure term added by every stage (hx_mlp.cu)
-    double2* cl_coef = nullptr;   // [top-tier ADOs][slab_store] its coefficients, of table build cl_build
-    int32_t* cl_slot = nullptr;   // [H] slab of an ADO in cl_coef, or -1
-    uint64_t cl_build = 0;
+    const double2* cl_coef = nullptr;  // [top-tier ADOs][slab_store] its coefficients (the closure's)
+    const int32_t* cl_slot = nullptr;  // [H] slab of an ADO in cl_coef, or -1
     bool cl_on = false;           // the closure is trained (or has its scales): its term counts
     float2* rho32 = nullptr;      // mixed: complex64 state buffers (rho, ua, ub mirror them)
     float2* ua32 = nullptr;

@@ -23,7 +23,6 @@
 #include <mma.h>
 
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
@@ -789,7 +788,9 @@ struct hx_closure {
     float2* raw = nullptr;       // [M][maxd][d2] network output A
     double2* coef = nullptr;     // [M][maxd][d2] Hermitian part of A times s_out / s_in
     uint64_t table_version = ~0ull;  // network version the table was built from
-    uint64_t table_build = 0;    // number of the build among all closures' (contexts keep sums of the table)
+    int32_t* slot = nullptr;     // [H] of the coarse hierarchy: place among the top-tier ADOs, or -1
+    double2* sum[2] = {};        // [n_top][slab] coefficients of full / Hermitian-packed slabs (once attached to)
+    bool sum_current[2] = {};    // ... summed from the table as it is
     int cap = 0, n_snap = 0;
     double s_in = 1.0, s_out = 1.0;  // RMS scales of inputs and targets
     bool scaled = false;
@@ -803,7 +804,7 @@ void closure_release(hx_closure* c)
     if (!c) return;
     if (c->stream) cudaStreamSynchronize(c->stream);
     void* p[] = {c->top_coarse, c->top_fine, c->up_fine, c->up_local, c->mode_bath_d, c->din, c->dout,
-                 c->top_occ, c->vdiag, c->hdiag, c->xin, c->tgt, c->raw, c->coef};
+                 c->top_occ, c->vdiag, c->hdiag, c->xin, c->tgt, c->raw, c->coef, c->slot, c->sum[0], c->sum[1]};
     for (void* q : p)
         if (q) cudaFree(q);
     if (c->net) mlp_release(c->net);
@@ -839,9 +840,10 @@ namespace {
 
 // Evaluate the network on every (k, n_k, r, c) and store the Hermitian part
 // of A, times s_out / s_in, in the coefficient table.
-int build_table(hx_closure* cl, cudaStream_t s)
+int build_table(hx_closure* cl)
 {
     hx_mlp* n = cl->net;
+    cudaStream_t s = n->stream;
     const long long rows = static_cast<long long>(cl->M) * cl->maxd * cl->d2;
     const int chunk = 8192;
     int rc = mlp_reserve(n, chunk);
@@ -857,9 +859,41 @@ int build_table(hx_closure* cl, cudaStream_t s)
                                                                                cl->s_out / cl->s_in, cl->coef);
     HX_CUDA_TRY(cudaGetLastError());
     cl->table_version = n->version;
-    static std::atomic<uint64_t> builds{0};
-    cl->table_build = ++builds;
+    cl->sum_current[0] = cl->sum_current[1] = false;
     return HX_OK;
+}
+
+// A context's stream may be capturing its step.  What the closure does on its own stream is not part of the
+// captured step, and this lets the thread allocate and wait for it meanwhile.
+struct OutsideCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Table and coefficients of the network as it is, in place and complete on return (on the network's stream).
+int refresh(hx_closure* cl)
+{
+    const bool stale = cl->table_version != cl->net->version;
+    bool any = stale;
+    for (int h = 0; h < 2; ++h) any = any || (cl->sum[h] && !cl->sum_current[h]);
+    if (!any) return HX_OK;
+    OutsideCapture outside;
+    cudaStream_t s = cl->net->stream;
+    if (stale)
+        if (const int rc = build_table(cl)) return rc;
+    for (int h = 0; h < 2; ++h) {
+        if (!cl->sum[h] || cl->sum_current[h]) continue;
+        const int nel = h ? hx::herm_elems(cl->logd) : cl->d2;
+        hx::closure_sum_kernel<<<dim3((nel + 255) / 256, cl->n_top), 256, 0, s>>>(
+            cl->top_occ, cl->mode_bath_d, cl->vdiag, cl->coef, cl->M, cl->maxd, cl->logd, h, cl->sum[h]);
+        HX_CUDA_TRY(cudaGetLastError());
+        cl->sum_current[h] = true;
+    }
+    const cudaError_t e = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) return HX_OK;
+    cl->table_version = ~0ull;
+    return hx::cuda_fail(e, "closure coefficients");
 }
 
 }  // namespace
@@ -868,20 +902,23 @@ namespace hx {
 
 int closure_attach(hx_closure* cl, ::hx_ctx* c)
 {
-    // the stream may still read the coefficients of the closure before
-    if (c->cl_coef || c->cl_slot) HX_CUDA_TRY(cudaStreamSynchronize(c->stream));
-    cudaFree(c->cl_coef);
-    cudaFree(c->cl_slot);
+    OutsideCapture outside;
     c->cl_coef = nullptr;
     c->cl_slot = nullptr;
-    c->cl_build = 0;
     c->cl_on = false;
     if (!cl) return HX_OK;
-    HX_CUDA_TRY(cudaMalloc(&c->cl_coef, static_cast<size_t>(cl->n_top) * c->slab_store * sizeof(double2)));
-    HX_CUDA_TRY(cudaMalloc(&c->cl_slot, static_cast<size_t>(c->H) * sizeof(int32_t)));
-    HX_CUDA_TRY(cudaMemsetAsync(c->cl_slot, 0xff, static_cast<size_t>(c->H) * sizeof(int32_t), c->stream));
-    closure_slot_kernel<<<(cl->n_top + 255) / 256, 256, 0, c->stream>>>(cl->top_coarse, cl->n_top, c->cl_slot);
-    HX_CUDA_TRY(cudaGetLastError());
+    cudaStream_t s = cl->net->stream;
+    if (!cl->slot) {
+        HX_CUDA_TRY(cudaMalloc(&cl->slot, static_cast<size_t>(c->H) * sizeof(int32_t)));
+        HX_CUDA_TRY(cudaMemsetAsync(cl->slot, 0xff, static_cast<size_t>(c->H) * sizeof(int32_t), s));
+        closure_slot_kernel<<<(cl->n_top + 255) / 256, 256, 0, s>>>(cl->top_coarse, cl->n_top, cl->slot);
+        HX_CUDA_TRY(cudaGetLastError());
+        HX_CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    double2*& sum = cl->sum[c->herm ? 1 : 0];
+    if (!sum) HX_CUDA_TRY(cudaMalloc(&sum, static_cast<size_t>(cl->n_top) * c->slab_store * sizeof(double2)));
+    c->cl_coef = sum;
+    c->cl_slot = cl->slot;
     return HX_OK;
 }
 
@@ -890,17 +927,7 @@ int closure_update(::hx_ctx* c)
     hx_closure* cl = c->closure;
     c->cl_on = cl->scaled;
     if (!cl->scaled) return HX_OK;
-    if (cl->table_version != cl->net->version) {
-        const int rc = build_table(cl, c->stream);
-        if (rc != HX_OK) return rc;
-    }
-    if (c->cl_build == cl->table_build) return HX_OK;
-    const int herm = c->herm ? 1 : 0, nel = static_cast<int>(c->slab_store);
-    closure_sum_kernel<<<dim3((nel + 255) / 256, cl->n_top), 256, 0, c->stream>>>(
-        cl->top_occ, cl->mode_bath_d, cl->vdiag, cl->coef, cl->M, cl->maxd, cl->logd, herm, c->cl_coef);
-    HX_CUDA_TRY(cudaGetLastError());
-    c->cl_build = cl->table_build;
-    return HX_OK;
+    return refresh(cl);
 }
 
 void closure_stage(const ::hx_ctx* c, const double2* u, double2* out, double alpha)
@@ -1314,9 +1341,8 @@ int hx_closure_train(hx_closure* c, uint32_t iters, uint32_t batch, float lr, ui
         if (e != cudaSuccess) rc = hx::cuda_fail(e, "closure training");
     }
     if (rc != HX_OK) return rc;
-    if ((rc = build_table(c, n->stream)) != HX_OK) return rc;
-    HX_CUDA_TRY(cudaStreamSynchronize(n->stream));
-    return HX_OK;
+    c->table_version = ~0ull;  // the network may be the one of before (no iterations), the scales new
+    return refresh(c);
 }
 
 int hx_closure_set_scales(hx_closure* c, double s_in, double s_out)

@@ -318,3 +318,99 @@ def test_mlp_rows_that_fill_a_warp_in_part(rows):
         assert np.max(np.abs(gg - rr)) <= 2e-2 * np.max(np.abs(rr)), name
         off += size
     net.close()
+
+
+def _trained_closure(n, K=1, seed=31, hidden=32):
+    coarse = S.spin_glass(n, seed=seed, depth=2, K=K, h=1.0, dt=0.005)
+    fine = S.spin_glass(n, seed=seed, depth=3, K=K, h=1.0, dt=0.005)
+    cl = capi.Closure(coarse, fine_max_depth=4, hidden=hidden, capacity=3, seed=3)
+    with capi.Context(fine) as ctx:
+        for _ in range(3):
+            ctx.step(10)
+            cl.harvest(ctx)
+    cl.train(iters=30, batch=64, lr=1e-3, seed=5)
+    return coarse, cl
+
+
+def _start_state(ctx, seed):
+    """A Hermitian state that fills the top tier."""
+    rng = np.random.default_rng(seed)
+    x = rng.standard_normal((ctx.size, ctx.dim, ctx.dim)) + 1j * rng.standard_normal((ctx.size, ctx.dim, ctx.dim))
+    return 0.5 * (x + np.conj(np.transpose(x, (0, 2, 1))))
+
+
+@pytest.mark.parametrize("n,full", [(3, False), (5, False), (5, True)])
+def test_captured_closure_steps_follow_the_network(n, full):
+    """A step captured before any other use of the closure: an eager step that
+    comes before its first replay has the closure's term, and replays after the
+    network is trained again have the new network's, both bit for bit."""
+    import torch
+
+    coarse, cl = _trained_closure(n)
+    stream = torch.cuda.Stream()
+    with capi.Context(coarse, full_state=full) as ref, capi.Context(coarse, full_state=full) as ctx:
+        x = _start_state(ctx, n)
+
+        def eager(c):
+            c.set_state(x)
+            c.step(1)
+            c.sync()
+            return c.state()
+
+        plain = eager(ref)
+        ctx.set_stream(stream.cuda_stream)
+        cl.attach(ctx)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.step(1)
+        first = eager(ctx)
+        cl.attach(ref)
+        assert np.array_equal(first, eager(ref)) and np.max(np.abs(first - plain)) > 1e-9
+        for _ in range(2):
+            cl.train(iters=30, batch=64, lr=1e-2, seed=9)
+            ctx.set_state(x)
+            with torch.cuda.stream(stream):
+                graph.replay()
+            torch.cuda.synchronize()
+            got = ctx.state()
+            assert np.array_equal(got, eager(ref)) and not np.array_equal(got, first)
+        del graph
+    cl.close()
+
+
+def test_captured_closure_step_outlives_the_attachment():
+    """The coefficients belong to the closure: a step captured with one closure
+    keeps its term when the context takes another closure, or none."""
+    import torch
+
+    coarse, one = _trained_closure(5, seed=31)
+    _, two = _trained_closure(5, seed=32)
+    stream = torch.cuda.Stream()
+    with capi.Context(coarse) as ref, capi.Context(coarse) as ctx:
+        x = _start_state(ctx, 1)
+        one.attach(ref)
+        ref.set_state(x)
+        ref.step(1)
+        want = ref.state()
+        ctx.set_stream(stream.cuda_stream)
+        one.attach(ctx)
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            ctx.step(1)
+        for other in (two, None):
+            if other is None:
+                assert capi.lib().hx_ctx_set_closure(ctx._h, None) == 0
+            else:
+                other.attach(ctx)
+            ctx.set_state(x)
+            ctx.step(1)
+            ctx.sync()
+            assert not np.array_equal(ctx.state(), want)
+            ctx.set_state(x)
+            with torch.cuda.stream(stream):
+                graph.replay()
+            torch.cuda.synchronize()
+            assert np.array_equal(ctx.state(), want)
+        del graph
+    one.close()
+    two.close()
