@@ -59,6 +59,7 @@ void release(hx_ctx* c)
                     c->U32, c->diag32, c->vdiag32, c->hflip32, c->diag_herm, c->vbit, c->csr_ptr, c->csr_col,
                     c->csr_val, c->pack_scale, c->pack_bad, c->dense_hr, c->dense_hr_lo, c->dense_y,
                     c->dense_h64, c->dense_z0, c->gbar, c->xsum, c->obs_csr};
+    hx::closure_attach(nullptr, c);
     for (void* p : ptrs)
         if (p) cudaFree(p);
     if (c->pinned) cudaFreeHost(c->pinned);
@@ -1287,7 +1288,8 @@ int hx_ctx_step(hx_ctx* c, uint64_t nsteps)
     if (c->use_run) enqueue_run(c, nsteps, nullptr, nullptr);
     else
         for (uint64_t s = 0; s < nsteps; ++s) enqueue_step(c);
-    return check_launch("stage kernel launch");
+    const int rc = check_launch("stage kernel launch");
+    return rc == HX_OK && c->closure ? hx::closure_used(c) : rc;
 }
 
 int hx_ctx_sync(hx_ctx* c)

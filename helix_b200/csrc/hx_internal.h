@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 
 #include <cstdint>
+#include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -313,11 +315,18 @@ bool closure_matches_hierarchy(const ::hx_closure* cl, int d, int M, long long H
 // in it, so it is one complex coefficient per element of each top-tier ADO.  The closure owns them, in the slab
 // layout of the contexts it is attached to: they keep their place when the network is trained again or the
 // context takes another closure, so a captured step reads what an eager one does.
+// The contexts that read them: the event of each context's last enqueued steps, which a rebuild waits for.
+struct ClosureReaders {
+    std::mutex m;  // also held while the coefficients are rebuilt
+    std::vector<cudaEvent_t> used;
+};
 // closure_attach: room for the coefficients and the slot of every ADO (cl = nullptr: detach).
 int closure_attach(::hx_closure* cl, ::hx_ctx* c);
 // Bring the coefficients up to date with the network, complete on return; c->cl_on tells whether there is a
 // term to add.
 int closure_update(::hx_ctx* c);
+// The steps enqueued so far read the coefficients.
+int closure_used(::hx_ctx* c);
 // out_top += alpha * coefficient * u_top, after a stage.
 void closure_stage(const ::hx_ctx* c, const double2* u, double2* out, double alpha);
 
@@ -442,6 +451,8 @@ struct hx_ctx {
     hx_closure* closure = nullptr; // learned closure term added by every stage (hx_mlp.cu)
     const double2* cl_coef = nullptr;  // [top-tier ADOs][slab_store] its coefficients (the closure's)
     const int32_t* cl_slot = nullptr;  // [H] slab of an ADO in cl_coef, or -1
+    std::shared_ptr<hx::ClosureReaders> cl_readers;  // the closure's list that holds cl_used
+    cudaEvent_t cl_used = nullptr;
     bool cl_on = false;           // the closure is trained (or has its scales): its term counts
     float2* rho32 = nullptr;      // mixed: complex64 state buffers (rho, ua, ub mirror them)
     float2* ua32 = nullptr;

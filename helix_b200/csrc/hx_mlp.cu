@@ -791,6 +791,7 @@ struct hx_closure {
     int32_t* slot = nullptr;     // [H] of the coarse hierarchy: place among the top-tier ADOs, or -1
     double2* sum[2] = {};        // [n_top][slab] coefficients of full / Hermitian-packed slabs (once attached to)
     bool sum_current[2] = {};    // ... summed from the table as it is
+    std::shared_ptr<hx::ClosureReaders> readers = std::make_shared<hx::ClosureReaders>();
     int cap = 0, n_snap = 0;
     double s_in = 1.0, s_out = 1.0;  // RMS scales of inputs and targets
     bool scaled = false;
@@ -871,7 +872,8 @@ struct OutsideCapture {
     ~OutsideCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
 
-// Table and coefficients of the network as it is, in place and complete on return (on the network's stream).
+// Table and coefficients of the network as it is, in place and complete on return (cl->readers->m is held).
+// On the network's stream, behind every enqueued step that reads them, whatever stream that is on.
 int refresh(hx_closure* cl)
 {
     const bool stale = cl->table_version != cl->net->version;
@@ -880,6 +882,7 @@ int refresh(hx_closure* cl)
     if (!any) return HX_OK;
     OutsideCapture outside;
     cudaStream_t s = cl->net->stream;
+    for (cudaEvent_t ev : cl->readers->used) HX_CUDA_TRY(cudaStreamWaitEvent(s, ev, 0));
     if (stale)
         if (const int rc = build_table(cl)) return rc;
     for (int h = 0; h < 2; ++h) {
@@ -903,10 +906,20 @@ namespace hx {
 int closure_attach(hx_closure* cl, ::hx_ctx* c)
 {
     OutsideCapture outside;
+    if (c->cl_readers) {
+        std::lock_guard<std::mutex> lock(c->cl_readers->m);
+        cudaEventSynchronize(c->cl_used);  // a rebuild no longer waits for this context
+        auto& used = c->cl_readers->used;
+        used.erase(std::find(used.begin(), used.end(), c->cl_used));
+        cudaEventDestroy(c->cl_used);
+    }
+    c->cl_readers.reset();
+    c->cl_used = nullptr;
     c->cl_coef = nullptr;
     c->cl_slot = nullptr;
     c->cl_on = false;
     if (!cl) return HX_OK;
+    std::lock_guard<std::mutex> lock(cl->readers->m);
     cudaStream_t s = cl->net->stream;
     if (!cl->slot) {
         HX_CUDA_TRY(cudaMalloc(&cl->slot, static_cast<size_t>(c->H) * sizeof(int32_t)));
@@ -917,6 +930,9 @@ int closure_attach(hx_closure* cl, ::hx_ctx* c)
     }
     double2*& sum = cl->sum[c->herm ? 1 : 0];
     if (!sum) HX_CUDA_TRY(cudaMalloc(&sum, static_cast<size_t>(cl->n_top) * c->slab_store * sizeof(double2)));
+    HX_CUDA_TRY(cudaEventCreateWithFlags(&c->cl_used, cudaEventDisableTiming));
+    cl->readers->used.push_back(c->cl_used);
+    c->cl_readers = cl->readers;
     c->cl_coef = sum;
     c->cl_slot = cl->slot;
     return HX_OK;
@@ -927,7 +943,18 @@ int closure_update(::hx_ctx* c)
     hx_closure* cl = c->closure;
     c->cl_on = cl->scaled;
     if (!cl->scaled) return HX_OK;
+    std::lock_guard<std::mutex> lock(cl->readers->m);
     return refresh(cl);
+}
+
+int closure_used(::hx_ctx* c)
+{
+    if (!c->cl_on) return HX_OK;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    HX_CUDA_TRY(cudaStreamIsCapturing(c->stream, &capture));
+    // a graph's launches are ordered by whoever launches it
+    if (capture == cudaStreamCaptureStatusNone) HX_CUDA_TRY(cudaEventRecord(c->cl_used, c->stream));
+    return HX_OK;
 }
 
 void closure_stage(const ::hx_ctx* c, const double2* u, double2* out, double alpha)
@@ -1341,6 +1368,7 @@ int hx_closure_train(hx_closure* c, uint32_t iters, uint32_t batch, float lr, ui
         if (e != cudaSuccess) rc = hx::cuda_fail(e, "closure training");
     }
     if (rc != HX_OK) return rc;
+    std::lock_guard<std::mutex> lock(c->readers->m);
     c->table_version = ~0ull;  // the network may be the one of before (no iterations), the scales new
     return refresh(c);
 }

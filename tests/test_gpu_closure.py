@@ -378,6 +378,41 @@ def test_captured_closure_steps_follow_the_network(n, full):
     cl.close()
 
 
+def test_one_closure_in_contexts_on_several_streams():
+    """Contexts on streams of their own that share a closure, whose scales
+    change while their steps are under way and whose coefficients one of them
+    then brings up to date: every context ends where it does alone."""
+    coarse, cl = _trained_closure(5)
+    info = cl.info()
+    contexts = [capi.Context(coarse, full_state=k == 2) for k in range(4)]
+    x = _start_state(contexts[0], 5)
+    scales = [(info["s_in"], info["s_out"]), (info["s_in"], 2.0 * info["s_out"]), (2.0 * info["s_in"], info["s_out"])]
+
+    want = []
+    for c in contexts:
+        cl.attach(c)
+        c.set_state(x)
+        for a, b in scales:
+            cl.set_scales(a, b)
+            c.step(20)
+            c.sync()
+        want.append(c.state())
+    assert not np.array_equal(want[0], want[2])  # full slabs: other kernels
+    for _ in range(5):
+        for c in contexts:
+            c.set_state(x)
+        for a, b in scales:
+            cl.set_scales(a, b)
+            for c in contexts:
+                c.step(20)
+        for c, w in zip(contexts, want):
+            c.sync()
+            assert np.array_equal(c.state(), w)
+    for c in contexts:
+        c.close()
+    cl.close()
+
+
 def test_captured_closure_step_outlives_the_attachment():
     """The coefficients belong to the closure: a step captured with one closure
     keeps its term when the context takes another closure, or none."""
