@@ -449,3 +449,45 @@ def test_captured_closure_step_outlives_the_attachment():
         del graph
     one.close()
     two.close()
+
+
+@pytest.mark.parametrize("i,h,o", [(12, 248, 2), (13, 248, 2), (40, 320, 24)])
+def test_gradients_around_the_size_of_a_staging_piece(i, h, o):
+    """65474, 65722 and 123544 parameters: the gradients come back in one
+    piece of 65536 values, in two with a last one of 186, and in two. Bars as
+    in the other gradient tests."""
+    rows = 96
+    net, p = _net(i, h, o, 17)
+    rng = np.random.default_rng(h + i)
+    x = rng.uniform(-1, 1, (rows, i)).astype(np.float32)
+    t = rng.uniform(-1, 1, (rows, o)).astype(np.float32)
+    loss, g = net.gradients(x, t)
+    _, loss_ref, g_ref = MO.forward_backward(p.astype(np.float64), x.astype(np.float64), t.astype(np.float64), i, h, o,
+                                             bf16=True)
+    assert abs(loss - loss_ref) <= 1e-3 * loss_ref
+    off = 0
+    for name, size in [("W1", h * i), ("b1", h), ("W2", h * h), ("b2", h), ("W3", o * h), ("b3", o)]:
+        gg, rr = g[off:off + size], g_ref[off:off + size]
+        assert np.max(np.abs(gg - rr)) <= 2e-2 * np.max(np.abs(rr)), name
+        off += size
+    net.close()
+
+
+def test_first_gradients_of_a_network_take_no_page_locking():
+    """The first call of a new network makes room for its activations, which
+    is one allocation (0.3 ms, about one later call); page-locking room for
+    0.3 M gradients as well, and seventeen allocations, took 10 to 35."""
+    import time
+
+    rng = np.random.default_rng(0)
+    x = rng.uniform(-1, 1, (4096, 21)).astype(np.float32)
+    t = rng.uniform(-1, 1, (4096, 2)).astype(np.float32)
+    first, later = [], []
+    for seed in range(9):
+        net = capi.MLP(21, 512, 2, seed=seed)
+        for k in range(4):
+            t0 = time.perf_counter()
+            net.gradients(x, t)
+            (later if k else first).append(time.perf_counter() - t0)
+        net.close()
+    assert np.median(first) <= 6 * np.median(later)
