@@ -361,10 +361,14 @@ void enqueue_run(hx_ctx* c, uint64_t nsteps, double2* trace, double* obs)
     hx::RunClosure cl;
     if (c->closure && c->cl_on) cl = hx::RunClosure{c->cl_coef, c->cl_slot};
     auto* launch = c->herm ? hx::launch_herm_run : hx::launch_small_run;
+    // a graph's replays are not in steps_done, so neither are the steps that they lose
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaStreamIsCapturing(c->stream, &capture);
     constexpr uint64_t kMostSteps = 4096;  // of one launch
     for (uint64_t done = 0; done < nsteps;) {
         const int n = static_cast<int>(std::min(nsteps - done, kMostSteps));
         hx::StepWait w;
+        if (capture == cudaStreamCaptureStatusNone) w.lost = c->error_flag + 1;
         if (c->stall_next_step) {  // test hook: one arrival more than the CTAs make, a short wait
             w.skew = 1;
             w.max_polls = 1u << 12;
@@ -440,8 +444,8 @@ int check_launch(const char* what)
 // Enqueue the copy of the error word that flag_status reads after the next synchronisation.
 int enqueue_flag(hx_ctx* c)
 {
-    if (!c->flag_pin) HX_CUDA_TRY(cudaMallocHost(&c->flag_pin, sizeof(int)));
-    HX_CUDA_TRY(cudaMemcpyAsync(c->flag_pin, c->error_flag, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    if (!c->flag_pin) HX_CUDA_TRY(cudaMallocHost(&c->flag_pin, 2 * sizeof(int)));
+    HX_CUDA_TRY(cudaMemcpyAsync(c->flag_pin, c->error_flag, 2 * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
     return HX_OK;
 }
 
@@ -452,7 +456,9 @@ int flag_status(hx_ctx* c)
         return fail(HX_ERR_UNSUPPORTED_EXECUTION, "a kernel of a stage could not be enqueued");
     }
     if (*c->flag_pin != 0) {
-        cudaMemsetAsync(c->error_flag, 0, sizeof(int), c->stream);
+        // steps that a run did not come to; rho holds the ones before
+        c->steps_done -= std::min<uint64_t>(c->steps_done, static_cast<uint64_t>(std::max(0, c->flag_pin[1])));
+        cudaMemsetAsync(c->error_flag, 0, 2 * sizeof(int), c->stream);
         if (c->gbar) cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);  // a barrier that gave up
         return fail(HX_ERR_DEVICE_TIMEOUT, "a device-side wait ran out of its iteration budget");
     }
@@ -976,7 +982,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
         (rc = dev_alloc(c, &c->hdiag, d)) || (rc = dev_alloc(c, &c->hflip, logd)) ||
         (rc = dev_alloc(c, &c->vdiag, static_cast<size_t>(J) * d)) || (rc = dev_alloc(c, &c->xi, J)) ||
         (rc = dev_alloc(c, &c->counter, J)) || (rc = dev_alloc(c, &c->bath_off, J + 1)) ||
-        (rc = dev_alloc(c, &c->error_flag, 1)) || (rc = dev_alloc(c, &c->obs, 4)))
+        (rc = dev_alloc(c, &c->error_flag, 2)) || (rc = dev_alloc(c, &c->obs, 4)))
         return bail(rc);
 
     // host-side operator data (with sparse operators: the real parts of their diagonals)
@@ -1075,7 +1081,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     if (e == cudaSuccess) e = cudaMemcpyAsync(dphi, phi_m.data(), M * sizeof(double), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dtc, tc.data(), J * sizeof(double), cudaMemcpyHostToDevice, c->stream);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dta, ta.data(), J * sizeof(double), cudaMemcpyHostToDevice, c->stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(c->error_flag, 0, sizeof(int), c->stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(c->error_flag, 0, 2 * sizeof(int), c->stream);
     if (e != cudaSuccess) rc = hx::cuda_fail(e, "context setup");
     if (rc == HX_OK) rc = hx::build_tables_device(M, static_cast<int>(p->max_depth), c->H, c->rows, c->edges, c->stream);
     if (rc == HX_OK) {
@@ -1692,7 +1698,7 @@ int hx_ctx_state_device_ptr(hx_ctx* c, void** ptr)
 int hx_ctx_inject_wait_timeout(hx_ctx* c)
 {
     if (!c) return fail(HX_ERR_INVALID_RUNTIME_OPTION, "NULL context");
-    if (!c->use_run || !c->use_small)
+    if (!c->use_run)
         return fail(HX_ERR_UNSUPPORTED_EXECUTION, "no grid-barrier waits in this context's steps");
     c->stall_next_step = true;
     return HX_OK;

@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(TS, MINB)
                 break;
             }
             ++passed;
-            if (!grid_barrier(gcount, passed * G + w.skew, w.max_polls)) {
-                if (tid == 0) atomicExch(a.error_flag, 1);
+            if (!grid_barrier(gcount, passed, w)) {
+                run_gave_up(a.error_flag, w, nsteps, step, st == order);
                 return;
             }
             if (watcher && st == order) {

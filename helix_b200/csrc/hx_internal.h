@@ -182,11 +182,12 @@ void launch_transpose_bf16(const void* in, int rows, int cols, int ld_in, void* 
 // d <= 16, full slabs, sigma_z couplings, every up term in the entry lists: batched gathers (hx_small.cu)
 size_t small_smem(int logd, int M);
 bool small_supported(int logd, int M, int pauli);
-// Grid-barrier waits of small_step_kernel: polls before giving up (and setting the error word), and an
+// Grid-barrier waits of the kernels that run whole steps: polls before giving up (and setting the error word), and an
 // offset added to every barrier's arrival target (nonzero only to make the waits run out on purpose).
 struct StepWait {
     unsigned skew = 0;
     unsigned max_polls = 1u << 22;
+    int* lost = nullptr;  // += the steps of a launch that gave up which rho does not hold
 };
 // A learned closure's term in a run of whole steps: (coef x) added to the right-hand side of every ADO n with
 // slot[n] >= 0, coef = slab slot[n] of the context's closure coefficients (nullptrs: no closure).
@@ -465,7 +466,7 @@ struct hx_ctx {
     double* xi = nullptr;
     double* counter = nullptr;
     int32_t* bath_off = nullptr;
-    int* error_flag = nullptr;
+    int* error_flag = nullptr;    // [2] error word, steps that runs which gave up did not come to
     // fused stage-kernel tables (d = 32, 64)
     bool use_fused = false;
     bool use_small = false;       // d <= 16 sigma_z stage kernel (hx_small.cu)
@@ -498,7 +499,7 @@ struct hx_ctx {
     int trace_cap = 0;            // steps the trace buffers hold
     bool trace_rho = false;       // ... with rho_0 (or energies only)
     double* pinned = nullptr;     // pinned staging for traces
-    int* flag_pin = nullptr;      // pinned copy of the error word
+    int* flag_pin = nullptr;      // pinned copy of the two error words
     size_t pinned_bytes = 0;
     double2* state_pinned = nullptr; // pinned staging for packed whole-state transfers
     double* pack_scale = nullptr;    // [H] per-slab scale of the device-side packer (first use)

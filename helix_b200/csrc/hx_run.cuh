@@ -13,37 +13,64 @@
 namespace hx {
 
 // Grid barrier: every CTA is resident (cooperative launch).  One arrival
-// counter, zero when a launch begins: barrier k of the launch waits until it
-// reaches (k + 1) G.  The block's writes are ordered before thread 0's arrival
-// by the block barrier and a GPU-scope fence; the wait polls the counter with
-// acquire loads, bounded.  The launch puts the counter back to zero at its end,
-// so no host-side count is involved (a captured launch replays correctly).
-// Returns false when the wait ran out.
-__device__ __forceinline__ void grid_arrive(unsigned* count)
+// counter, zero when a launch begins: barrier k = 1, 2, ... of the launch waits
+// until it reaches k G.  The block's writes are ordered before thread 0's
+// arrival by the block barrier and a GPU-scope fence; the wait polls the
+// counter with acquire loads, bounded.  The launch puts the counter back to
+// zero at its end, so no host-side count is involved (a captured launch replays
+// correctly).
+//
+// A barrier is passed by every CTA or by none, so rho ends at the same step in
+// all slabs: the CTA that gives up at barrier k replaces the counter by
+// kRunAborted + k G, in one exchange that fails when the last arrival comes
+// first.  Who arrives later finds the mark and gives up at once, at the same
+// barrier; who still polls for an earlier one passes it.  (At most G - 1
+// arrivals follow a mark, so k stays readable.)  The mark stays until the host
+// has read the error word: launches already enqueued find it at their first
+// arrival and leave rho alone.
+constexpr unsigned kRunAborted = 1u << 31;
+
+// The counter before this CTA's arrival (thread 0).
+__device__ __forceinline__ unsigned grid_arrive(unsigned* count)
 {
     __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(count, 1u);
-    }
+    if (threadIdx.x != 0) return 0u;
+    __threadfence();
+    return atomicAdd(count, 1u);
 }
 
-__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned target, unsigned max_polls)
+// Barrier k (from 1); false when it was given up.
+__device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned k, const StepWait& w)
 {
+    const unsigned all = k * gridDim.x;
     int late = 0;
-    grid_arrive(count);
-    if (threadIdx.x == 0) {
+    if (grid_arrive(count) & kRunAborted) {
+        late = 1;
+    } else if (threadIdx.x == 0) {
         for (uint32_t it = 0;; ++it) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
-            if (static_cast<int>(v - target) >= 0) break;
-            if (it >= max_polls) {
+            if (v & kRunAborted) {
+                late = (v & ~kRunAborted) < all + gridDim.x;  // at this barrier, not at the next
+                break;
+            }
+            if (static_cast<int>(v - all - w.skew) >= 0) break;
+            if (it >= w.max_polls && atomicCAS(count, v, kRunAborted | all) == v) {
                 late = 1;
                 break;
             }
         }
     }
     return __syncthreads_or(late) == 0;
+}
+
+// A barrier that was not passed, after a stage of step `step` (its last one: the step is in rho): the error
+// word, and the steps of the launch that rho does not hold.
+__device__ __forceinline__ void run_gave_up(int* error_flag, const StepWait& w, int nsteps, int step, bool last_stage)
+{
+    if (threadIdx.x != 0) return;
+    if (blockIdx.x == 0 && w.lost) atomicAdd(w.lost, nsteps - step - (last_stage ? 1 : 0));
+    atomicExch(error_flag, 1);
 }
 
 // The counter goes back to zero for the next launch: by the watching CTA,

@@ -319,8 +319,8 @@ __global__ void __launch_bounds__(SlabShape<LOGD>::T)
                 break;
             }
             ++passed;
-            if (!grid_barrier(gcount, passed * G + w.skew, w.max_polls)) {
-                if (threadIdx.x == 0) atomicExch(error_flag, 1);
+            if (!grid_barrier(gcount, passed, w)) {
+                run_gave_up(error_flag, w, nsteps, step, st == order);
                 return;
             }
             if (watcher && st == order) {

@@ -283,14 +283,17 @@ int hx_ctx_rhs(hx_ctx* ctx, double* out, uint64_t n);
  * reference. */
 int hx_ctx_dense_product(hx_ctx* ctx, uint32_t count);
 
-/* Failure-detection test hook: the next step of a context whose steps run as
- * one cooperative launch (small slabs) waits at its first grid barrier for an
- * arrival that never comes, with a short poll limit.  The kernel gives up,
- * sets the device error word and returns before writing rho; the next
- * hx_ctx_sync reports HX_ERR_DEVICE_TIMEOUT, clears the error and the barrier
- * counter, and the context steps on from the state before the failed step.
- * HX_ERR_UNSUPPORTED_EXECUTION for other contexts.  No counterpart in the
- * reference. */
+/* Failure-detection test hook: the next steps of a context whose steps run in
+ * one cooperative launch (hx_info.kernels_per_step is 1) wait at their first
+ * grid barrier for an arrival that never comes, with a short poll limit.  The
+ * kernel gives up, sets the device error word and returns before writing rho,
+ * and steps enqueued behind it leave rho alone too; the next hx_ctx_sync
+ * reports HX_ERR_DEVICE_TIMEOUT, clears the error and the barrier counter, and
+ * the context steps on from the state before the failed step.  (A wait that
+ * runs out later in a run of steps leaves the last step that every CTA has
+ * completed.  hx_info.steps_done is the step that rho holds, once the error is
+ * reported.)  HX_ERR_UNSUPPORTED_EXECUTION for other contexts.  No counterpart
+ * in the reference. */
 int hx_ctx_inject_wait_timeout(hx_ctx* ctx);
 
 /* Device check that the state holds only finite values; returns

@@ -209,3 +209,55 @@ def test_packed_whole_step_runs_match_oracle(n, baths, K, depth, order, collecti
         assert abs(a.observables()[0] - en[-1]) == 0.0
     assert np.max(np.abs(rho - rho_ref)) <= TOL
     assert np.max(np.abs(en - en_ref)) <= TOL
+
+
+def _run_problem(kind, n, baths, K, depth):
+    p = S.spin_glass(n, seed=60 + n, depth=depth, K=K, h=0.8, dt=0.005)
+    p.baths = p.baths[:baths]
+    rng = np.random.default_rng(n)
+    for b in p.baths:
+        if kind != "spin":
+            b.v_diag = rng.uniform(-0.7, 0.7, p.dim)
+        if kind == "flip":
+            b.v_flip = rng.uniform(0.1, 0.4, n)
+    return p
+
+
+@pytest.mark.parametrize("kind,n,baths,K,depth", [
+    ("spin", 2, 2, 1, 2),         # 15 ADOs at d = 4: one CTA without barriers, unless a wait is to run out
+    ("collective", 1, 1, 1, 3),   # 10 ADOs at d = 2, the same with a general diagonal coupling
+    ("collective", 4, 2, 3, 4),   # 495 ADOs at d = 16
+    ("spin", 5, 5, 2, 2),         # 136 ADOs at d = 32, one per SM
+    ("spin", 5, 5, 1, 3),         # 286 ADOs at d = 32, two CTAs per SM
+    ("collective", 6, 4, 2, 2),   # 91 ADOs at d = 64
+    ("spin", 6, 6, 2, 2),         # 190 ADOs at d = 64, two per CTA
+    ("flip", 2, 1, 2, 3),         # 20 ADOs at d = 4, couplings with flips
+    ("flip", 5, 1, 2, 4),         # 35 ADOs at d = 32
+])
+def test_waits_of_every_run_kernel_are_reported_and_recovered_from(kind, n, baths, K, depth):
+    """A wait that runs out in any kernel of whole steps, in a run of several
+    steps and with more steps enqueued behind it: reported once, rho and the
+    count of steps are those of before, and the context goes on as one that
+    never failed."""
+    p = _run_problem(kind, n, baths, K, depth)
+    with capi.Context(p) as ref, capi.Context(p) as ctx:
+        assert ctx.get_info().kernels_per_step == 1
+        ref.step(2)
+        before = ref.state()
+        ctx.step(2)
+        for traced in (False, True):
+            assert np.array_equal(ctx.state(), before) and ctx.get_info().steps_done == 2
+            ctx.inject_wait_timeout()
+            with pytest.raises(capi.HxError) as e:
+                if traced:
+                    ctx.step_trace(3)
+                else:
+                    ctx.step(3)
+                    if n >= 4:  # (with one CTA there is no barrier for later steps to stop at)
+                        ctx.step(1)
+                    ctx.sync()
+            assert e.value.status == "DeviceWaitTimeout"
+        assert np.array_equal(ctx.state(), before) and ctx.get_info().steps_done == 2
+        rho, _ = ctx.step_trace(3)
+        assert np.array_equal(rho, ref.step_trace(3)[0])
+        assert np.array_equal(ctx.state(), ref.state()) and ctx.get_info().steps_done == 5
