@@ -936,6 +936,9 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     const bool small_ok = !c->use_flip && !c->use_large && !c->use_csr && logd <= 4 &&
                           hx::small_supported(logd, M, 1) && !(force_generic && force_generic[0] == '1') &&
                           !(small_env && small_env[0] == '0');
+    // whole steps in one launch: not at order 1 (the step writes rho while neighbours read it)
+    const char* step_env = std::getenv("HX_SMALL_STEP");
+    const bool runs_ok = c->order >= 2 && !(step_env && step_env[0] == '0');
     c->herm = (fused_ok || c->use_large) && want_herm;
     c->slab_store = c->herm ? static_cast<size_t>(hx::herm_elems(logd)) : c->slab;
     const size_t nstate = static_cast<size_t>(H) * c->slab_store;
@@ -1123,8 +1126,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             }
             const bool want_small = small_ok && all_pauli;
             // whole steps in one launch while the hierarchy fits the resident CTAs (d <= 16) and L2 (d = 32, 64)
-            const char* step_env = std::getenv("HX_SMALL_STEP");
-            const bool herm_run = c->herm && fused_ok && c->order >= 2 && !(step_env && step_env[0] == '0') &&
+            const bool herm_run = c->herm && fused_ok && runs_ok &&
                                   hx::herm_run_fits(logd, M, J, all_pauli ? 1 : 0, c->H, c->sm_count);
             // every up neighbour in the entry lists (no up-term pass)
             const bool all_up = small_ok || herm_run;
@@ -1171,7 +1173,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
             c->up_slots = S;
             c->use_fused = (rc == HX_OK) && fused_ok;
             c->use_small = (rc == HX_OK) && want_small;
-            if (rc == HX_OK && (herm_run || (small_ok && c->order >= 2 && !(step_env && step_env[0] == '0'))) &&
+            if (rc == HX_OK && (herm_run || (small_ok && runs_ok)) &&
                 (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
                 auto* launch = herm_run ? hx::launch_herm_run : hx::launch_small_run;
                 e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
@@ -1208,7 +1210,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     // whole steps in one launch where that is ahead, else the two-pass kernels
     if (rc == HX_OK && (c->use_csr || flip_slab) && logd <= hx::kMaxLogD && hx::prepare_slab(csr_args_of(c), c->csr_nnz)) {
         c->use_slab = c->use_csr;
-        if (flip_slab && c->order >= 2) {
+        if (flip_slab && runs_ok) {
             cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
             c->slab_ctas = hx::slab_run_ctas(csr_args_of(c), c->csr_nnz, c->sm_count);
             if (c->slab_ctas >= c->H && (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {

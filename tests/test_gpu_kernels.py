@@ -261,3 +261,23 @@ def test_waits_of_every_run_kernel_are_reported_and_recovered_from(kind, n, bath
         rho, _ = ctx.step_trace(3)
         assert np.array_equal(rho, ref.step_trace(3)[0])
         assert np.array_equal(ctx.state(), ref.state()) and ctx.get_info().steps_done == 5
+
+
+@pytest.mark.parametrize("kind,n,baths,K,depth,per_step", [
+    ("spin", 4, 2, 1, 3, 4), ("spin", 5, 5, 2, 2, 8), ("flip", 2, 1, 2, 3, 8), ("flip", 5, 1, 2, 4, 8),
+])
+def test_small_step_variable_leaves_every_run_out(monkeypatch, kind, n, baths, K, depth, per_step):
+    """HX_SMALL_STEP=0 when a context is made: a launch per pass of a stage,
+    for couplings with flips too, and the same trajectory."""
+    p = _run_problem(kind, n, baths, K, depth)
+    with capi.Context(p) as ctx:
+        assert ctx.get_info().kernels_per_step == 1
+        want, _ = ctx.step_trace(4)
+    monkeypatch.setenv("HX_SMALL_STEP", "0")
+    with capi.Context(p) as ctx:
+        assert ctx.get_info().kernels_per_step == per_step
+        got, _ = ctx.step_trace(4)
+        with pytest.raises(capi.HxError) as e:
+            ctx.inject_wait_timeout()
+        assert e.value.status == "UnsupportedExecution"
+    assert np.max(np.abs(got - want)) <= TOL
