@@ -376,9 +376,9 @@ void enqueue_run(hx_ctx* c, uint64_t nsteps, double2* trace, double* obs)
         }
         double2* tr = trace ? trace + done * c->slab_store : nullptr;
         double* ob = obs ? obs + 3 * done : nullptr;
-        if (c->use_slab) {
-            if (hx::launch_slab_run(csr_args_of(c), c->csr_nnz, c->slab_ctas, c->rho, c->ua, c->ub, c->dt, c->order, n,
-                                    c->gbar, c->error_flag, w, tr, ob, c->stream) != 1)
+        if (c->use_flip) {
+            if (hx::launch_flip_run(flip_args_of(c), c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->error_flag, w, tr,
+                                    ob, c->stream) != 1)
                 c->launch_failed = true;
         } else if (launch(hx::fused_args_of(c), cl, c->rho, c->ua, c->ub, c->dt, c->order, n, c->gbar, c->sm_count, c->stream,
                    false, tr, ob, w) != 1) {
@@ -951,14 +951,7 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
         e = cudaMemsetAsync(c->obs_csr, 0, n * sizeof(double), c->stream);
         if (e != cudaSuccess) return bail(hx::cuda_fail(e, "observables scratch"));
     }
-    const bool flip_slab = c->use_flip && logd <= hx::kMaxLogD;
-    if (flip_slab) {
-        ops.clear();
-        ops.push_back(flip_csr(p->h_diag, p->h_flip, static_cast<int>(d), logd));
-        for (int j = 0; j < J; ++j)
-            ops.push_back(flip_csr(p->baths[j].coupling_diag, p->baths[j].coupling_flip, static_cast<int>(d), logd));
-    }
-    if (c->use_csr || flip_slab) {
+    if (c->use_csr) {
         std::vector<int32_t> ptr, col;
         std::vector<double2> val;
         for (const HostCsr& o : ops) {
@@ -1206,18 +1199,15 @@ int hx_ctx_create(const hx_problem* p, hx_ctx** out)
     cudaFree(dphi);
     cudaFree(dtc);
     cudaFree(dta);
-    // sparse operators at d <= 64: a slab per CTA when the operators fit beside it; couplings with flips run
-    // whole steps in one launch where that is ahead, else the two-pass kernels
-    if (rc == HX_OK && (c->use_csr || flip_slab) && logd <= hx::kMaxLogD && hx::prepare_slab(csr_args_of(c), c->csr_nnz)) {
-        c->use_slab = c->use_csr;
-        if (flip_slab && runs_ok) {
-            cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
-            c->slab_ctas = hx::slab_run_ctas(csr_args_of(c), c->csr_nnz, c->sm_count);
-            if (c->slab_ctas >= c->H && (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
-                e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
-                if (e != cudaSuccess) rc = hx::cuda_fail(e, "grid barrier counter");
-                else c->use_slab = c->use_run = true;
-            }
+    // sparse operators at d <= 64: a slab per CTA where the operators fit beside it and that is ahead
+    if (rc == HX_OK && c->use_csr && logd <= hx::kMaxLogD) c->use_slab = hx::prepare_slab(csr_args_of(c), c->csr_nnz) == 1;
+    // couplings with flips: whole steps in one launch where that is ahead, else the two-pass kernels
+    if (rc == HX_OK && c->use_flip && runs_ok) {
+        cudaDeviceGetAttribute(&c->sm_count, cudaDevAttrMultiProcessorCount, c->device);
+        if (hx::prepare_flip_run(flip_args_of(c), c->sm_count) && (rc = dev_alloc(c, &c->gbar, 1)) == HX_OK) {
+            e = cudaMemsetAsync(c->gbar, 0, sizeof(unsigned), c->stream);
+            if (e != cudaSuccess) rc = hx::cuda_fail(e, "grid barrier counter");
+            else c->use_run = true;
         }
     }
     if (rc == HX_OK && c->use_large && (c->diag_table == nullptr || c->ent_count == nullptr))

@@ -247,7 +247,7 @@ __global__ void __launch_bounds__(TS, MINB)
                     for (int i = tid; i < P; i += TS) trace[static_cast<long long>(step) * P + i] = __ldcg(rho + i);
                 if (obs && tid < 32)
                     warp_observables<LOGD>(
-                        a, [&](int r, int c) { return __ldcg(rho + (r <= c ? herm_index(r, c, LOGD) : herm_index(c, r, LOGD))); },
+                        a.hdiag, a.hflip, [&](int r, int c) { return __ldcg(rho + (r <= c ? herm_index(r, c, LOGD) : herm_index(c, r, LOGD))); },
                         obs + 3 * step);
             }
         }

@@ -354,6 +354,11 @@ struct FlipArgs {
 // B (2 J H d*d complex) receives [V_j, u_n], then {V_j, u_n}; then out = base + alpha L(u).
 void launch_flip_stage(const FlipArgs& a, const double2* u, double2* B, const double2* rho, double2* out,
                        double alpha, int base_kind, cudaStream_t s);
+// Whole steps in one cooperative launch, a CTA per ADO and a watching one (d <= 32; trace / obs as in
+// launch_small_run).  prepare_flip_run: whether it fits and is ahead (raises the kernel's limit; before any capture).
+bool prepare_flip_run(const FlipArgs& a, int sms);
+int launch_flip_run(const FlipArgs& a, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
+                    unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs, cudaStream_t s);
 
 // Two-pass stage for general sparse Hermitian H and V_j (hx_csr.cu).
 // Operator k (0 = H, 1 + j = V_j) has row pointers ptr[k (d+1) .. k (d+1) + d]
@@ -380,11 +385,6 @@ int prepare_slab(const CsrArgs& a, int nnz);
 // One stage: gather pass (G: 2 J H slabs) and products.  Kernels launched.
 int launch_slab_stage(const CsrArgs& a, int nnz, const double2* u, double2* G, const double2* rho, double2* out,
                       double alpha, int base_kind, cudaStream_t s);
-// Whole steps in one cooperative launch on `ctas` CTAs (slab_run_ctas; 0: not possible) and a watching one;
-// the rest as in launch_small_run.
-int slab_run_ctas(const CsrArgs& a, int nnz, int sms);
-int launch_slab_run(const CsrArgs& a, int nnz, int ctas, double2* rho, double2* ua, double2* ub, double dt, int order,
-                    int nsteps, unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs, cudaStream_t s);
 // out[0] = Re Tr(H rho_0) with H in CSR (operator 0), out[1..2] = Tr rho_0; scratch: that many doubles, zeroed
 // once by the caller (one per stream).
 size_t observables_csr_scratch();
@@ -442,8 +442,8 @@ struct hx_ctx {
     double* vflip = nullptr;      // [J][log2 d]
     bool use_flip = false;        // two-pass flip path (flips in V, or d > 1024)
     bool use_csr = false;         // two-pass path for general sparse H / V_j (hx_csr.cu)
-    bool use_slab = false;        // ... or with flips, at d <= 64: a slab per CTA (hx_slab.cu)
-    int csr_nnz = 0, slab_ctas = 0;
+    bool use_slab = false;        // ... at d <= 64: a slab per CTA (hx_slab.cu)
+    int csr_nnz = 0;
     int32_t* csr_ptr = nullptr;   // [(J+1)(d+1)] operator 0 = H, 1 + j = V_j
     int32_t* csr_col = nullptr;
     double2* csr_val = nullptr;

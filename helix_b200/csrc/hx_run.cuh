@@ -89,7 +89,7 @@ __device__ __forceinline__ void grid_reset(unsigned* count, bool watch, bool wat
 // observables_kernel (hx_stage.cu); at(r, c) returns an element of rho_0 (the
 // real part alone counts off the diagonal).
 template <int LOGD, typename At>
-__device__ __forceinline__ void warp_observables(const FusedArgs& a, At at, double* out)
+__device__ __forceinline__ void warp_observables(const double* hdiag, const double* hflip, At at, double* out)
 {
     constexpr int D = 1 << LOGD;
     const int lane = threadIdx.x & 31;
@@ -100,11 +100,11 @@ __device__ __forceinline__ void warp_observables(const FusedArgs& a, At at, doub
         double en = 0.0, tr = 0.0, ti = 0.0;
         if (r < D) {
             const double2 dg = at(r, r);
-            en = fma(__ldg(a.hdiag + r), dg.x, en);
+            en = fma(__ldg(hdiag + r), dg.x, en);
             tr += dg.x;
             ti += dg.y;
 #pragma unroll
-            for (int i = 0; i < LOGD; ++i) en = fma(__ldg(a.hflip + i), at(r ^ (1 << i), r).x, en);
+            for (int i = 0; i < LOGD; ++i) en = fma(__ldg(hflip + i), at(r ^ (1 << i), r).x, en);
         }
         for (int off = 16; off > 0; off >>= 1) {
             en += __shfl_down_sync(0xffffffffu, en, off);

@@ -1,8 +1,7 @@
-// Stage kernels for sparse Hermitian operators (compressed rows, or diagonals
-// with spin flips written that way) at d <= 64, where a slab fits in shared
-// memory.
+// Stage kernels for sparse Hermitian operators (compressed rows) at d <= 64,
+// where a slab fits in shared memory.
 //
-// Same mathematics as the two-pass paths (hx_csr.cu, hx_flip.cu; reference
+// Same mathematics as the two-pass path (hx_csr.cu; reference
 // getdRhoSparse, src/liouville.cu:778-860), arranged so that no commutator of
 // an ADO leaves its CTA.  With C_j = [V_j, u_n], S_j the sum of the up
 // neighbours and of the down neighbours times a, and u_d the Drude mode's down
@@ -21,16 +20,12 @@
 //  * the two kinds of accumulators meet once per ADO, through shared memory;
 //  * the operators' entries stay in shared memory.
 //
-// Two forms: slab_kernel, one stage per launch after a gather pass
-// (slab_gather_kernel) has summed the neighbours, and slab_run_kernel, whole
-// integrator steps in one cooperative launch (grid barriers between the
-// stages, the last CTA records rho_0 and the observables).
+// slab_kernel runs one stage per launch, after a gather pass
+// (slab_gather_kernel) has summed the neighbours.
 //
 // Bound by shared memory (16 bytes per element and entry) and, for few ADOs,
-// by one CTA's time per ADO.  us per step, two passes against this: sparse
-// operators at d = 64, six baths, 91 ADOs 660 and 450; d = 32, four baths, 165
-// ADOs 285 and 183; couplings with flips at d = 32, 35 ADOs 60 and 45, at d = 4,
-// 10 ADOs 47 and 22.
+// by one CTA's time per ADO.  us per step, two passes against this: d = 64, six
+// baths, 91 ADOs 660 and 450; d = 32, four baths, 165 ADOs 285 and 183.
 
 #include <cuda_runtime.h>
 
@@ -39,7 +34,6 @@
 #include <cstdint>
 
 #include "hx_internal.h"
-#include "hx_run.cuh"
 
 namespace hx {
 
@@ -89,8 +83,7 @@ __device__ __forceinline__ void slab_product(const SlabOps& o, int op, const dou
     }
 }
 
-// One ADO: out_n = base_n + alpha L(u)_n.  gather != nullptr: S_j and u_d from
-// that buffer, else from the neighbours themselves (read through L2).
+// One ADO: out_n = base_n + alpha L(u)_n, S_j and b_j u_d from the gather buffer.
 template <int LOGD>
 __device__ __forceinline__ void slab_ado(const CsrArgs& a, const SlabOps& o, double2* X, double2* W, long long n,
                                          const double2* u, const double2* gather, const double2* base, double2* out,
@@ -130,7 +123,6 @@ __device__ __forceinline__ void slab_ado(const CsrArgs& a, const SlabOps& o, dou
             }
         }
     const long long HD2 = a.H * D2;
-    const int32_t* edges = a.edges + n * 2 * a.M;
     for (int j = 0; j < a.J; ++j) {
         // C_j: left part in registers, right part through W
         if (on)
@@ -151,37 +143,13 @@ __device__ __forceinline__ void slab_ado(const CsrArgs& a, const SlabOps& o, dou
         __syncthreads();
         // P_j into W, Q_j kept
         const double xi = a.xi[j], ka = a.counter[j];
-        const int m0 = a.bath_off[j], m1 = a.bath_off[j + 1];
-        const int dn0 = edges[a.M + m0];
-        const double b = dn0 < a.H ? a.bcoef[n * a.J + j] : 0.0;
         if (on)
 #pragma unroll
             for (int i = 0; i < NR; ++i)
 #pragma unroll
                 for (int k = 0; k < NC; ++k) {
                     const int r = line + S::GROUPS * i, c = lane + 32 * k, e = (r << LOGD) + c;
-                    double2 s = make_double2(0.0, 0.0), d = s;
-                    if (gather) {
-                        s = __ldcg(gather + j * HD2 + n * D2 + e);
-                        d = __ldcg(gather + (a.J + j) * HD2 + n * D2 + e);
-                    } else {
-#pragma unroll 2
-                        for (int m = m0; m < m1; ++m) {
-                            const int up = __ldg(edges + m), dn = __ldg(edges + a.M + m);
-                            if (up < a.H) {
-                                const double2 v = __ldcg(u + up * D2 + e);
-                                s.x += v.x;
-                                s.y += v.y;
-                            }
-                            if (dn < a.H) {
-                                const double2 v = __ldcg(u + dn * D2 + e);
-                                const double w = __ldg(a.acoef + n * a.M + m);
-                                s.x = fma(w, v.x, s.x);
-                                s.y = fma(w, v.y, s.y);
-                                if (m == m0) d = make_double2(b * v.x, b * v.y);
-                            }
-                        }
-                    }
+                    const double2 s = __ldcg(gather + j * HD2 + n * D2 + e), d = __ldcg(gather + (a.J + j) * HD2 + n * D2 + e);
                     const double2 q = W[slab_at<LOGD>(r, c)], l = y[i * NC + k];
                     const double cx = l.x - q.x, cy = l.y - q.y;
                     // P = -i S - b u_d - (xi + i kappa) C, Q = i S - b u_d + (xi - i kappa) C
@@ -289,67 +257,6 @@ __global__ void __launch_bounds__(256) slab_gather_kernel(CsrArgs a, const doubl
 }
 
 template <int LOGD>
-__global__ void __launch_bounds__(SlabShape<LOGD>::T)
-    slab_run_kernel(CsrArgs a, int nnz, double2* rho, double2* ua, double2* ub, double dt, int order, int nsteps,
-                    unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs)
-{
-    constexpr int D = 1 << LOGD, D2 = D * D, T = SlabShape<LOGD>::T;
-    extern __shared__ __align__(16) unsigned char smem[];
-    double2* X = reinterpret_cast<double2*>(smem);
-    const SlabOps o = slab_ops<LOGD>(a, nnz, smem + 2 * D2 * sizeof(double2));
-    const bool watch = trace != nullptr || obs != nullptr;
-    const int G = static_cast<int>(gridDim.x), GC = G - (watch ? 1 : 0);
-    const bool watcher = watch && static_cast<int>(blockIdx.x) == GC;
-    __syncthreads();
-    unsigned passed = 0;
-    double2* bufs[2] = {ua, ub};
-    const double2* in = rho;
-    for (int step = 0; step < nsteps; ++step) {
-        for (int st = 1; st <= order; ++st) {
-            const double alpha = dt / static_cast<double>(order - st + 1);
-            double2* out = (st == order) ? rho : bufs[(st - 1) & 1];
-            for (long long n = blockIdx.x; !watcher && n < a.H; n += GC) {
-                slab_ado<LOGD>(a, o, X, X + D2, n, in, nullptr, rho, out, alpha, st == 1 ? kBaseSelf : kBaseRho);
-                __syncthreads();
-            }
-            in = out;
-            const bool last = step + 1 == nsteps && st == order;
-            if (last && !watcher) {
-                if (watch) grid_arrive(gcount);  // the watcher waits for the last state; nobody else does
-                break;
-            }
-            ++passed;
-            if (!grid_barrier(gcount, passed, w)) {
-                run_gave_up(error_flag, w, nsteps, step, st == order);
-                return;
-            }
-            if (watcher && st == order) {
-                if (trace)
-                    for (int i = threadIdx.x; i < D2; i += T) trace[static_cast<long long>(step) * D2 + i] = __ldcg(rho + i);
-                if (obs && threadIdx.x < 32) {
-                    // Re Tr(H rho_0) along the rows of H (Hermitian), Tr rho_0
-                    double s[3] = {0.0, 0.0, 0.0};
-                    for (int r = threadIdx.x; r < D; r += 32) {
-                        const double2 dg = __ldcg(rho + (r << LOGD) + r);
-                        s[1] += dg.x;
-                        s[2] += dg.y;
-                        for (int p = o.ptr[r]; p < o.ptr[r + 1]; ++p) {
-                            const double2 y = __ldcg(rho + (r << LOGD) + o.col[p]), v = o.val[p];
-                            s[0] += v.x * y.x + v.y * y.y;
-                        }
-                    }
-                    for (int q = 0; q < 3; ++q) {
-                        for (int off = 16; off > 0; off >>= 1) s[q] += __shfl_down_sync(0xffffffffu, s[q], off);
-                        if (threadIdx.x == 0) obs[3 * step + q] = s[q];
-                    }
-                }
-            }
-        }
-    }
-    grid_reset(gcount, watch, watcher, static_cast<unsigned>(nsteps * order));
-}
-
-template <int LOGD>
 size_t slab_smem(int J, int nnz)
 {
     constexpr size_t D = size_t(1) << LOGD;
@@ -367,51 +274,24 @@ bool prepare_slab_t(int J, int nnz)
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
     if (raised[dev].load()) return true;
-    bool ok = cudaFuncSetAttribute(slab_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   static_cast<int>(kSlabSmem)) == cudaSuccess;
-    if constexpr (LOGD < 6)
-        ok = ok && cudaFuncSetAttribute(slab_run_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        static_cast<int>(kSlabSmem)) == cudaSuccess;
-    if (ok) raised[dev].store(true);
-    return ok;
-}
-
-template <int LOGD>
-int run_ctas_t(const CsrArgs& a, int nnz, int sms)
-{
-    int per_sm = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, slab_run_kernel<LOGD>, SlabShape<LOGD>::T,
-                                                      slab_smem<LOGD>(a.J, nnz)) != cudaSuccess)
-        return 0;
-    const long long room = static_cast<long long>(per_sm) * sms - 1;  // and the watcher
-    return static_cast<int>(std::min<long long>(a.H, room));
-}
-
-template <int LOGD>
-int launch_slab_run_t(const CsrArgs& a, int nnz, int ctas, double2* rho, double2* ua, double2* ub, double dt, int order,
-                      int nsteps, unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs,
-                      cudaStream_t s)
-{
-    CsrArgs args = a;
-    void* params[] = {&args, &nnz, &rho, &ua, &ub, &dt, &order, &nsteps, &gcount, &error_flag, &w, &trace, &obs};
-    return cudaLaunchCooperativeKernel(reinterpret_cast<void*>(slab_run_kernel<LOGD>),
-                                       dim3(static_cast<unsigned>(ctas + (trace || obs ? 1 : 0))),
-                                       dim3(SlabShape<LOGD>::T), params, slab_smem<LOGD>(a.J, nnz), s) == cudaSuccess
-               ? 1
-               : -1;
+    if (cudaFuncSetAttribute(slab_kernel<LOGD>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             static_cast<int>(kSlabSmem)) != cudaSuccess)
+        return false;
+    raised[dev].store(true);
+    return true;
 }
 
 }  // namespace
 
-#define HX_SLAB_SWITCH(CALL, LAST) \
-    switch (a.logd) {              \
-    case 1: return CALL(1);        \
-    case 2: return CALL(2);        \
-    case 3: return CALL(3);        \
-    case 4: return CALL(4);        \
-    case 5: return CALL(5);        \
-    case 6: return LAST;           \
-    default: return 0;             \
+#define HX_SLAB_SWITCH(CALL) \
+    switch (a.logd) {        \
+    case 1: return CALL(1);  \
+    case 2: return CALL(2);  \
+    case 3: return CALL(3);  \
+    case 4: return CALL(4);  \
+    case 5: return CALL(5);  \
+    case 6: return CALL(6);  \
+    default: return 0;       \
     }
 
 // At d = 64 the two-pass kernels, which spread every ADO over the GPU, stay ahead while most SMs would have no
@@ -422,26 +302,7 @@ int prepare_slab(const CsrArgs& a, int nnz)
 {
     if (a.logd == 6 && a.H < 45) return 0;
 #define HX_CALL(L) (prepare_slab_t<L>(a.J, nnz) ? 1 : 0)
-    HX_SLAB_SWITCH(HX_CALL, HX_CALL(6))
-#undef HX_CALL
-}
-
-// Couplings with flips run whole steps while every ADO has a CTA of its own (an SM of its own at d = 32); at
-// d = 64 two passes with four rows per thread are ahead at any count (us per four steps, two passes against a run:
-// 20 ADOs 275 and 517, 126 502 and 626; d = 32, 126 ADOs 290 and 204, 210 311 and 322, 495 474 and 590).
-int slab_run_ctas(const CsrArgs& a, int nnz, int sms)
-{
-    if (a.logd == 6 || (a.logd == 5 && a.H > sms - 1)) return 0;
-#define HX_CALL(L) run_ctas_t<L>(a, nnz, sms)
-    HX_SLAB_SWITCH(HX_CALL, 0)
-#undef HX_CALL
-}
-
-int launch_slab_run(const CsrArgs& a, int nnz, int ctas, double2* rho, double2* ua, double2* ub, double dt, int order,
-                    int nsteps, unsigned* gcount, int* error_flag, StepWait w, double2* trace, double* obs, cudaStream_t s)
-{
-#define HX_CALL(L) launch_slab_run_t<L>(a, nnz, ctas, rho, ua, ub, dt, order, nsteps, gcount, error_flag, w, trace, obs, s)
-    HX_SLAB_SWITCH(HX_CALL, 0)
+    HX_SLAB_SWITCH(HX_CALL)
 #undef HX_CALL
 }
 
@@ -454,7 +315,7 @@ int launch_slab_stage(const CsrArgs& a, int nnz, const double2* u, double2* G, c
     (slab_kernel<L><<<static_cast<unsigned>(a.H), SlabShape<L>::T, slab_smem<L>(a.J, nnz), s>>>(a, nnz, u, G, rho, out, \
                                                                                                 alpha, base_kind),     \
      2)
-    HX_SLAB_SWITCH(HX_CALL, HX_CALL(6))
+    HX_SLAB_SWITCH(HX_CALL)
 #undef HX_CALL
 }
 

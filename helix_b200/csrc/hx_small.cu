@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kRunThreads, 1)
                 // xin of this stage is the state after the step before
                 if (trace)
                     for (int i = tid & 31; i < D2; i += 32) trace[static_cast<long long>(step - 1) * D2 + i] = xin[i];
-                if (obs) warp_observables<LOGD>(a, [&](int r0, int c0) { return xin[(r0 << LOGD) + c0]; }, obs + 3 * (step - 1));
+                if (obs) warp_observables<LOGD>(a.hdiag, a.hflip, [&](int r0, int c0) { return xin[(r0 << LOGD) + c0]; }, obs + 3 * (step - 1));
             }
             for (int j = 0; active && j < per; ++j) {
                 const int l = j * apc + la;
@@ -438,7 +438,7 @@ __global__ void __launch_bounds__(kRunThreads, 1)
                 if (trace)
                     for (int i = tid; i < D2; i += blockDim.x) trace[static_cast<long long>(step) * D2 + i] = __ldcg(rho + i);
                 if (obs && tid < 32)
-                    warp_observables<LOGD>(a, [&](int r0, int c0) { return __ldcg(rho + (r0 << LOGD) + c0); }, obs + 3 * step);
+                    warp_observables<LOGD>(a.hdiag, a.hflip, [&](int r0, int c0) { return __ldcg(rho + (r0 << LOGD) + c0); }, obs + 3 * step);
             }
         }
     }
@@ -448,7 +448,7 @@ __global__ void __launch_bounds__(kRunThreads, 1)
         if (watcher) {
             if (trace)
                 for (int i = tid & 31; i < D2; i += 32) trace[static_cast<long long>(nsteps - 1) * D2 + i] = xs[i];
-            if (obs) warp_observables<LOGD>(a, [&](int r0, int c0) { return xs[(r0 << LOGD) + c0]; }, obs + 3 * (nsteps - 1));
+            if (obs) warp_observables<LOGD>(a.hdiag, a.hflip, [&](int r0, int c0) { return xs[(r0 << LOGD) + c0]; }, obs + 3 * (nsteps - 1));
         }
         return;
     }

@@ -281,3 +281,128 @@ def test_small_step_variable_leaves_every_run_out(monkeypatch, kind, n, baths, K
             ctx.inject_wait_timeout()
         assert e.value.status == "UnsupportedExecution"
     assert np.max(np.abs(got - want)) <= TOL
+
+
+# ---- rounding: against the same sums in long double
+
+
+def _rhs_sums(p, rows, edges, x, real, cplx):
+    """The right-hand side in the given precision: every operator's terms summed by themselves, then added."""
+    d, H, M, r = p.dim, len(rows), rows.shape[1], np.arange(p.dim)
+    ext = np.concatenate([x, np.zeros((1, d, d), x.dtype)])
+
+    def apply(op, y, sign):  # [op, y] or {op, y}
+        diag, flips, matrix = op
+        if matrix is None:
+            out = (diag[:, None] + sign * diag[None, :]).astype(real) * y
+            for i, w in enumerate(flips):
+                if w != 0.0:
+                    out = out + real(w) * (y[:, r ^ (1 << i), :] + sign * y[:, :, r ^ (1 << i)])
+            return out
+        left, right = np.zeros_like(y), np.zeros_like(y)
+        for i, k in zip(*np.nonzero(matrix)):
+            left[:, i, :] += cplx(matrix[i, k]) * y[:, k, :]
+            right[:, :, k] += y[:, :, i] * cplx(matrix[i, k])
+        return left + sign * right
+
+    def operator(diag, flips, csr):
+        if csr is None:
+            return np.asarray(diag, real), np.zeros(0) if flips is None else np.asarray(flips), None
+        ptr, col, val = csr
+        m = np.zeros((d, d), np.complex128)
+        for i in range(d):
+            np.add.at(m, (i, col[ptr[i]:ptr[i + 1]]), val[ptr[i]:ptr[i + 1]])
+        return None, None, m
+
+    ham = operator(p.h_diag, p.h_flip, p.h_csr_explicit)
+    plain = ham[2] is None and all(b.v_csr is None and b.v_flip is None for b in p.baths)
+    g = np.zeros(H, real)
+    table = np.zeros((d, d), np.clongdouble)  # every term that multiplies the element itself, rounded once
+    total, entries = np.zeros_like(x), np.zeros_like(x)
+    o = 0
+    for b in p.baths:
+        c = O.bath_coefficients(b.beta, b.gamma, b.zeta, b.K)
+        op = operator(b.v_diag, b.v_flip, b.v_csr)
+        n = rows[:, o:o + b.K + 1]
+        g += (n * c["nu"]).sum(axis=1).astype(real)
+        weight = (n * c["nu"] * np.array([c["ktheta_c_im"], *c["kphi_im"]])).astype(real)
+        up = [ext[np.minimum(edges[:, o + k], H)] for k in range(b.K + 1)]
+        down = [ext[np.minimum(edges[:, M + o + k], H)] for k in range(b.K + 1)]
+        theta = (n[:, 0] * c["nu"][0] * c["ktheta_a"]).astype(real)[:, None, None]
+        if plain:
+            v = np.asarray(b.v_diag, np.longdouble)
+            dv, sv = v[:, None] - v[None, :], v[:, None] + v[None, :]
+            table -= c["kxi"] * dv * dv + 1j * c["kxi_counter_im"] * sv * dv
+            for k in range(b.K + 1):
+                entries = entries - 1j * (dv.astype(real) * up[k])
+                w = -1j * weight[:, k, None, None] * dv.astype(real) - (theta * sv.astype(real) if k == 0 else 0)
+                entries = entries + w * down[k]
+        else:
+            s = np.zeros_like(x)
+            for k in range(b.K + 1):
+                s = s + up[k] + weight[:, k, None, None] * down[k]
+            comm = apply(op, x, -1)
+            t = -1j * s - real(c["kxi"]) * comm
+            a = -1j * real(c["kxi_counter_im"]) * comm - theta * down[0]
+            total = total + (apply(op, t, -1) + apply(op, a, 1))
+        o += b.K + 1
+    if plain:
+        e = np.asarray(p.h_diag, np.longdouble)
+        table -= 1j * (e[:, None] - e[None, :])
+        flips = apply((np.zeros(d, real), p.h_flip, None), x, -1)
+        return ((table.astype(cplx) - g[:, None, None]) * x - 1j * flips) + entries
+    return (-1j * apply(ham, x, -1) - g[:, None, None] * x) + total
+
+
+def _step_sums(rhs, x, dt, real):
+    """One step, F = x + dt/1 L(x + dt/2 L(x + dt/3 L(x + dt/4 L x)))."""
+    y = x
+    for k in (4, 3, 2, 1):
+        y = x + real(dt) / real(k) * rhs(y)
+    return y
+
+
+def _distance(a, b):
+    return float(np.sqrt((np.abs(a - b) ** 2).sum()))
+
+
+@pytest.mark.parametrize("kind,n,baths,K,depth", [
+    ("flip", 2, 1, 2, 3), ("flip", 3, 2, 1, 3), ("flip", 5, 3, 1, 2),  # whole steps in one launch
+    ("flip", 6, 2, 1, 3), ("flip", 7, 1, 2, 3),                        # two passes
+])
+def test_no_more_rounding_than_term_by_term_sums(kind, n, baths, K, depth):
+    """Right-hand side and one step of length 1/4 against long double, from a
+    random Hermitian state.  The measure is the error of plain double-precision
+    sums on the host, every operator's terms by themselves: the kernels have a
+    rounding fewer per product, and half as much again is left for the order in
+    which they add the parts."""
+    bar = 1.5
+    p = _rounding_problem(kind, n, baths, K, depth)
+    M = sum(b.K + 1 for b in p.baths)
+    rows, edges = capi.hierarchy_tables(M, p.max_depth)
+    rng = np.random.default_rng(17)
+    x = rng.standard_normal((len(rows), p.dim, p.dim)) + 1j * rng.standard_normal((len(rows), p.dim, p.dim))
+    x = x + x.conj().transpose(0, 2, 1)
+
+    def exact(y):
+        return _rhs_sums(p, rows, edges, y, np.longdouble, np.clongdouble)
+
+    def plain(y):
+        return _rhs_sums(p, rows, edges, y, np.float64, np.complex128)
+
+    with capi.Context(p) as ctx:
+        ctx.set_state(x)
+        rhs = ctx.rhs()
+        ctx.step(1)
+        state = ctx.state()
+    xl = x.astype(np.clongdouble)
+    want = exact(xl)
+    assert _distance(rhs, want) <= bar * _distance(plain(x), want)
+    want = _step_sums(exact, xl, p.dt, np.longdouble)
+    assert _distance(state, want) <= bar * _distance(_step_sums(plain, x, p.dt, np.float64), want)
+
+
+def _rounding_problem(kind, n, baths, K, depth):
+    p = S.sparse_problem(n, seed=70 + n, depth=depth, K=K, dt=0.25) if kind == "sparse" else _run_problem(kind, n, n, K, depth)
+    p.baths, p.dt = p.baths[:baths], 0.25
+    return p

@@ -96,3 +96,86 @@ def test_large_dim_diagonal_coupling_matches_oracle():
     assert np.max(np.abs(rho - rho_ref)) <= TOL
     assert np.max(np.abs(en - en_ref)) <= TOL
     o.close()
+
+
+def _flip_rhs_exact(u, rows, edges, nu, baths, shift):
+    """sum of -i [H, u_n] - g_n u_n - i sum_up [V, u_up] in long double, the operators' diagonals without `shift`,
+    which no commutator sees.  baths: (first mode, diagonal, flips); the first entry is H.  Also the sum of the
+    absolute values of the coefficients of any element."""
+    ld = np.clongdouble
+    d = u.shape[-1]
+    bits = range(d.bit_length() - 1)
+    r = np.arange(d)
+
+    def comm(v, w, x):
+        v = (v - shift).astype(np.longdouble)
+        y = (v[:, None] - v[None, :]) * x
+        for i in bits:
+            y = y + np.longdouble(w[i]) * (x[:, r ^ (1 << i), :] - x[:, :, r ^ (1 << i)])
+        return y
+
+    def norm(v, w):
+        return float(np.max(v) - np.min(v) + 2 * np.sum(np.abs(w)))
+
+    M, H = rows.shape[1], rows.shape[0]
+    x = u.astype(ld)
+    g = (rows * nu).sum(axis=1).astype(np.longdouble)
+    out = -1j * comm(*baths[0][1:], x) - g[:, None, None] * x
+    size = norm(*baths[0][1:]) + float(g.max())
+    for k, (m0, v, w) in enumerate(baths[1:]):
+        m1 = baths[k + 2][0] if k + 2 < len(baths) else M
+        for m in range(m0, m1):
+            up = edges[:, m]
+            ok = up < H
+            s = np.zeros_like(x)
+            s[ok] = x[up[ok]]
+            out = out - 1j * comm(v, w, s)
+            size += norm(v, w)
+    return out, size
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 7, 8])
+def test_large_common_part_of_the_diagonals_costs_no_digits(n):
+    """H and V_j with a common 2^24 on their diagonals, which no commutator sees
+    (bath strengths of 1e-40 leave nothing else of V_j): right-hand side, and
+    one step (whole steps in one launch at d <= 32).  Every term is a difference
+    times a coefficient, so the error of a right-hand side is at most one
+    rounding per operation (64 is more than any element has) of the sum of the
+    coefficients times the largest element, and a step's Taylor sum adds those
+    of its stages to the rounding of the base."""
+    shift, eps = 2.0 ** 24, 2.0 ** -53
+    p = S.spin_glass(n, seed=90 + n, depth=2, K=1, h=0.6, dt=0.005)
+    p.baths = p.baths[:2]
+    rng = np.random.default_rng(n)
+    p.h_diag = shift + rng.uniform(-2.0, 2.0, p.dim)
+    p.h_flip = rng.uniform(0.2, 1.0, n)
+    nu, offsets = [], []
+    for b in p.baths:
+        b.v_diag = shift + rng.uniform(-1.0, 1.0, p.dim)
+        b.v_flip = rng.uniform(0.2, 0.6, n)
+        b.zeta = 1e-40
+        offsets.append(len(nu))
+        nu += list(O.bath_coefficients(b.beta, b.gamma, b.zeta, b.K)["nu"])
+    rows, edges = capi.hierarchy_tables(len(nu), p.max_depth)
+    M = len(nu)
+    rows, edges = np.asarray(rows).reshape(-1, M), np.asarray(edges).reshape(-1, 2 * M)
+    ops = [(0, p.h_diag, p.h_flip)] + [(o, b.v_diag, b.v_flip) for o, b in zip(offsets, p.baths)]
+    x = rng.standard_normal((len(rows), p.dim, p.dim)) + 1j * rng.standard_normal((len(rows), p.dim, p.dim))
+
+    def rhs(u):
+        return _flip_rhs_exact(u, rows, edges, np.array(nu), ops, shift)
+
+    with capi.Context(p) as ctx:
+        assert ctx.stage_path == "flip" and ctx.get_info().kernels_per_step == (1 if n <= 5 else 8)
+        ctx.set_state(x)
+        got = ctx.rhs()
+        want, size = rhs(x)
+        big = np.max(np.abs(x))
+        assert np.max(np.abs(got - want)) <= 64 * eps * size * big
+        ctx.step(1)
+        total, term, bound = x.astype(np.clongdouble), x.astype(np.clongdouble), 4 * eps * big
+        for k in range(1, 5):
+            term = rhs(term)[0] * (np.longdouble(p.dt) / k)
+            total = total + term
+            bound += 64 * eps * big * (p.dt * size) ** k / float(np.prod(range(1, k + 1)))
+        assert np.max(np.abs(ctx.state() - total)) <= bound
