@@ -369,6 +369,8 @@ def _distance(a, b):
 @pytest.mark.parametrize("kind,n,baths,K,depth", [
     ("flip", 2, 1, 2, 3), ("flip", 3, 2, 1, 3), ("flip", 5, 3, 1, 2),  # whole steps in one launch
     ("flip", 6, 2, 1, 3), ("flip", 7, 1, 2, 3),                        # two passes
+    ("sparse", 3, 2, 1, 3), ("sparse", 5, 5, 1, 2), ("sparse", 6, 2, 2, 4),  # a slab per CTA
+    ("sparse", 7, 2, 0, 2),                                                  # two passes
 ])
 def test_no_more_rounding_than_term_by_term_sums(kind, n, baths, K, depth):
     """Right-hand side and one step of length 1/4 against long double, from a
