@@ -471,30 +471,15 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
         bool on[E];
         const C* sp = sx + (r0 + 8 * k0) * 64;  // the pass's first row; + 512 per k
         const int cs = c ^ (r0 & 7);
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            on[k] = !diag || r0 + 8 * (k0 + k) <= c;
+            z[k] = mk<R>(0, 0);
+        }
         {
             C x[E];
 #pragma unroll
-            for (int k = 0; k < E; ++k) {
-                on[k] = !diag || r0 + 8 * (k0 + k) <= c;
-                x[k] = sp[cs + 512 * k];
-            }
-            // ---- diagonal term
-#pragma unroll
-            for (int k = 0; k < E; ++k) {
-                const int r = gr0 + 8 * (k0 + k);
-                R tr, ti;
-                if (PAULI) {
-                    tr = sX[r ^ gc];
-                    ti = static_cast<R>(sE[gc] - sE[r]);
-                } else {
-                    const C t = on[k] ? __ldg(a.diag + own + (k0 + k) * step) : mk<R>(0, 0);
-                    tr = t.x;
-                    ti = t.y;
-                }
-                tr -= g;
-                z[k].x = -(tr * x[k].y + ti * x[k].x);
-                z[k].y = tr * x[k].x - ti * x[k].y;
-            }
+            for (int k = 0; k < E; ++k) x[k] = sp[cs + 512 * k];
             // ---- flips inside the tile: z += h (row partner - column partner)
 #pragma unroll
             for (int b = 0; b < 6; ++b) {
@@ -620,6 +605,24 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
                 z[k].x -= y[k].y;
                 z[k].y += y[k].x;
             }
+        }
+        // ---- diagonal term, last: everything before is rounded at its own, smaller size
+#pragma unroll
+        for (int k = 0; k < E; ++k) {
+            const int r = gr0 + 8 * (k0 + k);
+            const C x = sp[cs + 512 * k];
+            R tr, ti;
+            if (PAULI) {
+                tr = sX[r ^ gc];
+                ti = static_cast<R>(sE[gc] - sE[r]);
+            } else {
+                const C t = on[k] ? __ldg(a.diag + own + (k0 + k) * step) : mk<R>(0, 0);
+                tr = t.x;
+                ti = t.y;
+            }
+            tr -= g;
+            z[k].x -= tr * x.y + ti * x.x;
+            z[k].y += tr * x.x - ti * x.y;
         }
         // ---- Horner epilogue
         C* on_ = out + n * P + own + k0 * step;

@@ -371,14 +371,16 @@ def _distance(a, b):
     ("flip", 6, 2, 1, 3), ("flip", 7, 1, 2, 3),                        # two passes
     ("sparse", 3, 2, 1, 3), ("sparse", 5, 5, 1, 2), ("sparse", 6, 2, 2, 4),  # a slab per CTA
     ("sparse", 7, 2, 0, 2),                                                  # two passes
+    ("spin", 7, 7, 0, 2), ("spin", 8, 3, 0, 2), ("collective", 7, 2, 1, 2),  # a CTA per tile
 ])
 def test_no_more_rounding_than_term_by_term_sums(kind, n, baths, K, depth):
     """Right-hand side and one step of length 1/4 against long double, from a
     random Hermitian state.  The measure is the error of plain double-precision
     sums on the host, every operator's terms by themselves: the kernels have a
     rounding fewer per product, and half as much again is left for the order in
-    which they add the parts."""
-    bar = 1.5
+    which they add the parts (a quarter with diagonal couplings, which have
+    three parts only)."""
+    bar = 1.5 if kind in ("flip", "sparse") else 1.25
     p = _rounding_problem(kind, n, baths, K, depth)
     M = sum(b.K + 1 for b in p.baths)
     rows, edges = capi.hierarchy_tables(M, p.max_depth)
