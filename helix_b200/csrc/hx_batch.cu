@@ -522,7 +522,7 @@ __global__ void batch_gsum_kernel(const int32_t* rows, const int32_t* bath_off, 
 // elements one after the other: 23 us for 128 instances, 7 with the lanes on the diagonal);
 // fixed summation order, so the result does not depend on timing.
 // logd[i] carries bit 8 when instance i keeps Hermitian-packed slabs.
-constexpr int kObsWarps = 32;
+constexpr int kObsWarps = 32;  // one per lane of the last sum
 
 __global__ void __launch_bounds__(kObsWarps * 32)
     batch_obs_kernel(const double2* const* rho0, const int* logd, int count, int spin, double* trace, int* counter,
@@ -544,9 +544,11 @@ __global__ void __launch_bounds__(kObsWarps * 32)
     __shared__ double red[kObsWarps];
     if (lane == 0) red[warp] = s;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        double v = 0.0;
-        for (int w = 0; w < kObsWarps; ++w) v += red[w];
+    if (warp > 0) return;
+    // pairwise: one sum after the other rounds at the size of the total all the way
+    double v = red[lane];
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
+    if (lane == 0) {
         const int t = *counter;
         trace[t % cap] = v;
         *counter = t + 1;
