@@ -524,8 +524,7 @@ template <int LOGD, bool PAULI>
 bool prepare_herm_t(int M, int J)
 {
     const size_t smem = herm_smem<LOGD>(M, J);
-    // a slab's bytes below the limit: the tables of (M, J) accepted do not depend on how the slab is staged
-    if (smem + static_cast<size_t>(herm_elems(LOGD)) * sizeof(double2) + 16 > 227 * 1024) return false;
+    if (smem > 227 * 1024) return false;
     static size_t configured[64] = {};
     int dev = 0;
     cudaGetDevice(&dev);
