@@ -164,8 +164,9 @@ __global__ void __launch_bounds__(256)
 
 // out[0] = Re Tr(H rho_0) = Re sum_r sum_{p in row r} conj(H_p) rho0_{r, col p} (H is Hermitian), so the
 // reads run along rows of rho_0; out[1..2] = Tr rho_0.  A warp per row, the blocks' sums in scratch[3 b ..],
-// added in block order by the block that finishes last (*ticket counts them and goes back to zero): one block
-// over columns of rho_0 took 55 us for a dense H of d = 256, this takes 10.
+// added pairwise in a fixed order by the block that finishes last (*ticket counts them and goes back to zero; one
+// after the other they are rounded at the size of the total all the way): one block over columns of rho_0 took 55 us
+// for a dense H of d = 256, this takes 10.
 constexpr int kObsBlocks = 64;
 
 __global__ void __launch_bounds__(256)
@@ -196,19 +197,21 @@ __global__ void __launch_bounds__(256)
     __shared__ bool last;
     if (threadIdx.x == 0) {
         for (int q = 0; q < 3; ++q) {
-            double t = 0.0;
-            for (int w = 0; w < 8; ++w) t += red[w][q];
-            scratch[3 * blockIdx.x + q] = t;
+            scratch[3 * blockIdx.x + q] = ((red[0][q] + red[1][q]) + (red[2][q] + red[3][q])) +
+                                          ((red[4][q] + red[5][q]) + (red[6][q] + red[7][q]));
         }
         __threadfence();
         last = atomicAdd(ticket, 1u) == gridDim.x - 1;
     }
     __syncthreads();
-    if (!last || threadIdx.x >= 3) return;
+    if (!last || warp >= 3) return;
     __threadfence();
     double t = 0.0;
-    for (unsigned b = 0; b < gridDim.x; ++b) t += __ldcg(scratch + 3 * b + threadIdx.x);
-    out[threadIdx.x] = t;
+#pragma unroll
+    for (int b = lane; b < kObsBlocks; b += 32)
+        if (b < static_cast<int>(gridDim.x)) t += __ldcg(scratch + 3 * b + warp);
+    for (int off = 16; off > 0; off >>= 1) t += __shfl_down_sync(0xffffffffu, t, off);
+    if (lane == 0) out[warp] = t;
     if (threadIdx.x == 0) *ticket = 0u;
 }
 
