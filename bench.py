@@ -236,6 +236,8 @@ def stage_kernels_label(ctx, p, packed: bool, per_stage: int) -> str:
     """The kernels one stage of this context launches (from its stage path)."""
     logd = p.dim.bit_length() - 1
     path = ctx.stage_path
+    if path == "flip" and int(ctx.info.kernels_per_step) == 1:
+        return f"flip_run_kernel<{logd}> (whole steps in one cooperative launch, spin-flip coupling path)"
     if path == "flip":
         return "comm_kernel + combine_kernel per stage (spin-flip coupling path)"
     if path == "csr":

@@ -285,8 +285,8 @@ int launch_large_stage(hx_ctx* c, const double2* u, const double2* rho, double2*
     const float2* u32 = b32[buffer_id(c, u)];
     float2* o32 = b32[buffer_id(c, out)];
     // ADO 0 in FP64 reads and writes nothing that the rest writes: its kernels, which fill a fraction of the
-    // SMs, run beside the rest of the stage.  d = 256, 969 ADOs: 2171 us a step, one after the
-    // other 2230; d = 128, 120 ADOs 144 and 183; dense H at d = 256, 969 ADOs, 4500 and 4600
+    // SMs, run beside the rest of the stage.  d = 256, 969 ADOs: 2108 us a step, one after the
+    // other 2182; d = 128, 120 ADOs 124 and 172; dense H at d = 256, 969 ADOs, 4650 and 4707
     cudaEventRecord(c->ev_fork, c->stream);
     cudaStreamWaitEvent(c->side_stream, c->ev_fork, 0);
     if (c->dense) {
@@ -324,9 +324,10 @@ int launch_stage_any(hx_ctx* c, const double2* u, const double2* rho, double2* o
     return k;
 }
 
-// One stage: the two-pass flip path when V has spin-flip parts or d > 64; for
-// d = 32, 64 the up-term kernel of tier L-1 followed by the fused multi-CTA
-// kernel; the generic kernel otherwise.  Returns kernels launched.
+// One stage, without the closure: the tile kernels from d = 128 on; with sparse operators a slab per CTA (d <= 64)
+// or the two passes; with flips in a coupling, or d > 1024, the two passes; else at d = 32 and 64 the up-term
+// kernel of tier L-1 (unless the entry lists hold its neighbours) and the fused kernel, at d <= 16 the small-slab
+// kernel (sigma_z) or the generic one.  Returns kernels launched.
 int launch_stage_core(hx_ctx* c, const double2* u, const double2* rho, double2* out, double alpha, int base)
 {
     if (c->use_large) return launch_large_stage(c, u, rho, out, alpha, base);

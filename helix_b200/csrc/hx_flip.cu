@@ -27,9 +27,9 @@
 // is 16 MB).  Bound by the 20 reads of 16 bytes per element and pass; with one
 // element per thread and one flip after the other they waited on each other.
 // Per step at d = 1024, 10 ADOs: 2.99 ms with one element per thread, 2.03 with
-// four rows (two rows 3.2, eight rows 2.99: fewer warps hide the latency); with
-// flips in H too 2.32.  Couplings with flips at d <= 32 run whole
-// steps in one launch (flip_run_kernel).
+// four rows (two rows 3.2, eight rows 2.99: fewer warps hide the latency); 1.91
+// as it is now, 2.31 with flips in H too.  Couplings with flips at d <= 32 run
+// whole steps in one launch (flip_run_kernel).
 
 #include <cuda_runtime.h>
 

@@ -304,8 +304,8 @@ __global__ void __launch_bounds__(256, MINB)
 // the packed slab that all warps waited for, flips first, needed a second
 // buffer in shared memory: 1374 us a step at d = 64, 7315 ADOs, against 1340
 // with the L1 cache the buffer leaves free, and 801 against 772 at d = 32,
-// 15504 ADOs.)  Bound by the load-store unit: 65% of its wavefronts, three
-// quarters of them shared memory, at 2.7 TB/s of DRAM traffic.
+// 15504 ADOs.)  Bound by the load-store unit (69% of its wavefronts, two thirds
+// of them shared memory; DRAM at 40%) and the latency of what goes through it.
 // With that swizzle every flip is one XOR of the slot with a constant
 // (row bit b: d 2^b, plus 2^b when b < 3; column bit b: 2^b), and the
 // accesses stay free of bank conflicts: a run of consecutive columns of one

@@ -228,21 +228,25 @@ __device__ __forceinline__ C packed_at(const C* __restrict__ slab, int r, int c,
 //    leave no room for the buffers at two CTAs per SM;
 //  * the sum is kept times i: then a flip and a commutator entry are one
 //    packed multiply-add in complex64, and an entry whose weight is zero on
-//    all of a warp's rows is left out (the kernel issues 67% of the time);
+//    all of a warp's rows is left out (the kernel issues 61% of the time);
 //  * a thread owns 8 elements of one column, 8 rows apart, in NP passes: the
 //    flips of the rows of a pass are in registers, the other flips inside the
 //    tile in shared memory (element (r, c) at r 64 + (c ^ (r & 7)): free of
 //    bank conflicts for the mirrored writes of a diagonal tile too);
 //  * with sigma_z couplings the weights come from index bits and the diagonal
 //    term from two d-entry tables instead of a third slab-sized stream;
+//  * the diagonal term comes last: started with it, the sum was rounded at its
+//    size by every flip and neighbour (error of a right-hand side at d = 128
+//    1.57e-16 against 1.07e-16, of a complex64 step 2.4e-7 against 1.7e-7; d =
+//    256 in double 4% faster so, in complex64 1% slower);
 //  * diagonal tiles compute their upper triangle only.
 //
-// d = 256, 969 ADOs: 0.69 ms a stage in double, 0.43 in complex64 (bands of
+// d = 256, 969 ADOs: 0.68 ms a stage in double, 0.44 in complex64 (bands of
 // rows: 0.94 and 0.56; complex64 without staged tiles and packed arithmetic
-// 0.48).  Double is at 74% of the load-store unit's wavefronts and 7.4 TB/s
+// 0.48).  Double is at 77% of the load-store unit's wavefronts and 8.8 TB/s
 // between L2 and the SMs.  Full slabs, us per step, bands of 4096 / d rows
-// against tiles: d = 256, 165 ADOs 1260 and 885 in double, 614 and 500 in
-// complex64; d = 128, 680 ADOs 1226 and 841; 604 and 475.  The 64 registers of two CTAs per SM are the limit: one
+// against tiles: d = 256, 165 ADOs 1260 and 855 in double, 614 and 475 in
+// complex64; d = 128, 680 ADOs 1226 and 814; 604 and 465.  The 64 registers of two CTAs per SM are the limit: one
 // pass of 8 rows in double spills or leaves one CTA (0.85 ms).
 template <typename R, int LOGD> struct TileShape;
 template <int LOGD> struct TileShape<double, LOGD> { static constexpr int NP = 2, MINB = 2, LR = LOGD == 7 ? 1 : 4; };
@@ -768,7 +772,7 @@ __global__ void __launch_bounds__(256)
 // tiles, two outputs of one row per thread, K staged through shared memory 32
 // at a time with the next block's loads under way.  d^3 complex multiply-adds
 // in d^2 / 512 CTAs (d = 256: 48 us with 64 CTAs of 16 x 4 outputs a warp,
-// ZGEMM us).
+// 18 so).
 __global__ void __launch_bounds__(256) zgemm_kernel(const double2* __restrict__ x, const double2* __restrict__ h,
                                                     double2* __restrict__ z, int logd)
 {
@@ -879,7 +883,7 @@ bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* ou
     constexpr long long kBlocks = (1 << LOGD) / 64;
     const long long nb = (a.H - a.first_ado) * (a.herm ? kBlocks * (kBlocks + 1) / 2 : kBlocks * kBlocks);
     if (nb <= 0) return true;
-    // fewer tiles than SMs: a CTA per half of a tile's rows (d = 128, 28 ADOs 103 us a step, 119 without)
+    // fewer tiles than SMs: a CTA per half of a tile's rows (d = 128, 28 ADOs 99 us a step, 113 without)
     LargeArgs<R> t = a;
     t.halves = sizeof(R) == sizeof(double) && nb <= 148 ? 1 : 0;
     kernel<<<static_cast<unsigned>(t.halves ? 2 * nb : nb), kTileT, smem, s>>>(t, u, rho, out, alpha, base);

@@ -456,7 +456,7 @@ __global__ void __launch_bounds__(kRunThreads, 1)
 }
 
 // order[k] = the ADO with the k-th most entries (ties by index): ranks by
-// counting, one thread per ADO; H is a few thousand at most.
+// counting, one thread per ADO, once per context.  A hundred thousand ADOs at most fit a run (d = 2).
 __global__ void run_order_kernel(const int* __restrict__ count, int H, int32_t* order)
 {
     const int n = blockIdx.x * blockDim.x + threadIdx.x;

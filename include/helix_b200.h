@@ -143,7 +143,7 @@ typedef struct hx_info {
 #define HX_PATH_GENERIC 0u  /* stage_kernel: d <= 64 outside the fused shapes */
 #define HX_PATH_FUSED 1u    /* herm_run_kernel, or herm_kernel / fused_kernel (+ upterm_kernel): d = 32, 64 */
 #define HX_PATH_BAND 2u     /* tile_kernel: 128 <= d <= 1024, diagonal couplings */
-#define HX_PATH_FLIP 3u     /* couplings with spin flips: slab_run_kernel (d <= 32), comm_kernel + combine_kernel */
+#define HX_PATH_FLIP 3u     /* couplings with spin flips: flip_run_kernel (d <= 32), comm_kernel + combine_kernel */
 #define HX_PATH_CSR 4u      /* general sparse operators: slab_kernel (d <= 64), csr_comm_kernel + csr_combine_kernel */
 #define HX_PATH_SMALL 5u    /* small_step_kernel, small_kernel: d <= 16, diagonal couplings */
 #define HX_PATH_DENSE 6u    /* HX_FLAG_DENSE_H: tc_split_gemm_kernel + zgemm_kernel + dense_tile_kernel */
