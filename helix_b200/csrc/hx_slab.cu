@@ -313,9 +313,9 @@ bool prepare_slab_t(int J, int nnz)
     }
 
 // At d = 64 the two-pass kernels, which spread every ADO over the GPU, stay ahead while most SMs would have no
-// slab: us per four steps, two passes against a slab per CTA, 28 ADOs of six baths 1066 and 1522, 35 of four 839
-// and 1123, 45 of four 1131 and 1102, 55 of three 1215 and 990, 91 of six 2588 and 1779; at d = 32 a slab per
-// CTA is ahead from 2 ADOs (299 and 297) on, 20 ADOs 531 and 436.
+// slab, whatever the number of baths: us per step, two passes against a slab per CTA, 35 ADOs of one bath 91 and 123, of
+// four 189 and 271; 45 ADOs of one 124 and 122, of four 280 and 275; 55 of one 148 and 130, of three 287 and 229; 91 of
+// six 629 and 453; at d = 32 a slab per CTA is ahead from 2 ADOs (per four steps 299 and 297) on, 20 ADOs 531 and 436.
 int prepare_slab(const CsrArgs& a, int nnz)
 {
     if (a.logd == 6 && a.H < 45) return 0;
