@@ -444,6 +444,7 @@ size_t flip_run_smem(int J)
 }
 
 constexpr size_t kFlipRunSmem = 227 * 1024;
+constexpr long long kFlipRunMost = 3000;  // ADOs
 
 template <int LOGD>
 bool prepare_flip_run_t(const FlipArgs& a, int sms)
@@ -492,10 +493,13 @@ int launch_flip_run_t(const FlipArgs& a, double2* rho, double2* ua, double2* ub,
 
 // Whole steps while every ADO has a CTA of its own (at d = 32 an SM of its own).  us per step, two passes against a
 // run, one bath: d = 4, 20 ADOs 38 and 14; d = 16, 120 ADOs 42 and 17, 560 50 and 26; d = 32, 35 ADOs 50 and 27, 120
-// 55 and 27; five baths, d = 32, 66 ADOs 95 and 70.  At d = 64 the two passes with four rows per thread were ahead
+// 55 and 27; five baths, d = 32, 66 ADOs 95 and 70.  Thousands of arrivals at every barrier take longer than the two
+// launches: d = 4, 1771 ADOs 42 and 26, 3654 42 and 47, so the line lies at 3000 (d <= 4 alone has room for more).
+// At d = 64 the two passes with four rows per thread were ahead
 // of a CTA per ADO at any count (per four steps 275 and 517 at 20 ADOs, 502 and 626 at 126).
 bool prepare_flip_run(const FlipArgs& a, int sms)
 {
+    if (a.H > kFlipRunMost) return false;
 #define HX_CALL(L) prepare_flip_run_t<L>(a, sms)
     HX_FLIP_SWITCH(HX_CALL, false)
 #undef HX_CALL

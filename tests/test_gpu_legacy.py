@@ -179,3 +179,21 @@ def test_large_common_part_of_the_diagonals_costs_no_digits(n):
             total = total + term
             bound += 64 * eps * big * (p.dt * size) ** k / float(np.prod(range(1, k + 1)))
         assert np.max(np.abs(ctx.state() - total)) <= bound
+
+
+@pytest.mark.parametrize("n", [1, 2])
+def test_thousands_of_small_slabs_take_the_two_passes(n):
+    """Couplings with flips at d = 2 and 4: 2925 ADOs run whole steps in one
+    launch, 3654 a launch per pass, where barriers over that many CTAs took 72 us a
+    step and two passes take 42; both as the oracle has it."""
+    for depth, size, per_step in ((24, 2925, 1), (26, 3654, 8)):
+        p = S.spin_glass(n, seed=7 + n, depth=depth, K=2, h=0.6, dt=0.002)
+        p.baths = p.baths[:1]
+        p.baths[0].v_flip = np.full(n, 0.3)
+        o = O.Oracle(p)
+        rho_ref, en_ref = o.run(3, trace=True)
+        o.close()
+        with capi.Context(p) as ctx:
+            assert ctx.stage_path == "flip" and ctx.size == size and ctx.get_info().kernels_per_step == per_step
+            rho, en = ctx.step_trace(3)
+        assert np.max(np.abs(rho - rho_ref)) <= TOL and np.max(np.abs(en - en_ref)) <= TOL
