@@ -316,9 +316,14 @@ bool prepare_slab_t(int J, int nnz)
 // slab, whatever the number of baths: us per step, two passes against a slab per CTA, 35 ADOs of one bath 91 and 123, of
 // four 189 and 271; 45 ADOs of one 124 and 122, of four 280 and 275; 55 of one 148 and 130, of three 287 and 229; 91 of
 // six 629 and 453; at d = 32 a slab per CTA is ahead from 2 ADOs (per four steps 299 and 297) on, 20 ADOs 531 and 436.
+// At d = 2 and 4 a CTA per slab of 4 or 16 elements leaves most of its threads idle, and with thousands of them the
+// two passes are ahead: d = 2, 1330 ADOs 42 and 42, 3654 42 and 48, 52360 72 and 173; d = 4, 1330 50 and 46, 2300 50
+// and 54, 10660 82 and 107, two baths 1820 66 and 60, 3003 67 and 73.  At d = 8 the slabs stay ahead (10660 199 and
+// 164).
 int prepare_slab(const CsrArgs& a, int nnz)
 {
     if (a.logd == 6 && a.H < 45) return 0;
+    if (a.logd <= 2 && a.H > (a.logd == 1 ? 1024 : 2000)) return 0;
 #define HX_CALL(L) (prepare_slab_t<L>(a.J, nnz) ? 1 : 0)
     HX_SLAB_SWITCH(HX_CALL)
 #undef HX_CALL

@@ -434,3 +434,18 @@ def test_observables_of_sparse_operators_are_summed_pairwise():
             want = math.fsum(np.real(np.diagonal(ctx.rho0())))
             err.append((np.real(ctx.observables()[1]) - want) / want * 2.0 ** 53)
     assert np.sqrt(np.mean(np.square(err))) <= 1.1
+
+
+@pytest.mark.parametrize("n,K,depth,size", [(1, 2, 16, 969), (1, 2, 17, 1140), (2, 2, 20, 1771), (2, 2, 21, 2024)])
+def test_many_small_slabs_of_sparse_operators_match_oracle(n, K, depth, size):
+    """Sparse operators at d = 2 and 4, on both sides of the number of ADOs from
+    which the two passes take over from a slab per CTA."""
+    p = S.sparse_problem(n, seed=20 + n, depth=depth, K=K, dt=0.002)
+    p.baths = p.baths[:1]
+    o = O.Oracle(p)
+    rho_ref, en_ref = o.run(3, trace=True)
+    o.close()
+    with capi.Context(p) as ctx:
+        assert ctx.stage_path == "csr" and ctx.size == size
+        rho, en = ctx.step_trace(3)
+    assert np.max(np.abs(rho - rho_ref)) <= TOL and np.max(np.abs(en - en_ref)) <= TOL
