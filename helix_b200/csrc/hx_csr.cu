@@ -20,10 +20,13 @@
 // the last line being -Xi [V, B] - i kappa {V, B}.  One thread per element;
 // the gathered rows and columns of a slab are read through L1/L2.
 // Bound by the latency of index, value and gather one after the other, so two
-// entries are asked for at once: 2 to 10% of a step (d = 128, three baths, 28
-// ADOs 593 -> 578 us; one bath, 2 ADOs 124 -> 112).  Four entries, or four rows
-// of a column per thread, take the registers of the warps that hide the latency
-// (d = 128, 7 ADOs 203 -> 255 us).
+// entries are asked for at once, in the registers that leave six CTAs per SM
+// (first pass) and five (second).  us per step, one entry at a time and five
+// CTAs, two entries and four, and now: d = 128, three baths, 13 ADOs 263, 303 and
+// 252, 28 ADOs 477, 472 and 425; d = 256, 3 ADOs 205, 224 and 194, 10 ADOs 652, 673
+// and 586; d = 512, 10 ADOs 2536, 2492 and 2300.  Six CTAs for both spill (d = 128, 6
+// ADOs 84 -> 93).  Four entries, or four rows of a column per thread, take the
+// registers of the warps that hide the latency.
 
 #include <cuda_runtime.h>
 
@@ -47,18 +50,19 @@ __device__ __forceinline__ double2 cmulc(double2 a, double2 b)
     return make_double2(a.x * b.x + a.y * b.y, a.y * b.x - a.x * b.y);
 }
 
-// (A X)_rc and (X A)_rc of operator k for slab X (row-major, d = 2^logd).
+// (A X)_rc and (X A)_rc of operator k for slab X (row-major, d = 2^logd), U entries at a time.
 struct Sides {
     double2 left, right;
 };
 
+template <int U>
 __device__ __forceinline__ Sides sides(const CsrArgs& a, int k, const double2* __restrict__ X, int r, int c)
 {
     const int D = 1 << a.logd;
     const int32_t* ptr = a.ptr + static_cast<long long>(k) * (D + 1);
     double2 L = make_double2(0.0, 0.0), R = make_double2(0.0, 0.0);
     const int r1 = __ldg(ptr + r + 1), c1 = __ldg(ptr + c + 1);
-#pragma unroll 2
+#pragma unroll U
     for (int p = __ldg(ptr + r); p < r1; ++p) {
         const double2 v = __ldg(a.val + p);
         const double2 x = __ldg(X + (static_cast<long long>(__ldg(a.col + p)) << a.logd) + c);
@@ -66,7 +70,7 @@ __device__ __forceinline__ Sides sides(const CsrArgs& a, int k, const double2* _
         L.x += t.x;
         L.y += t.y;
     }
-#pragma unroll 2
+#pragma unroll U
     for (int p = __ldg(ptr + c); p < c1; ++p) {
         const double2 v = __ldg(a.val + p);
         const double2 x = __ldg(X + (static_cast<long long>(r) << a.logd) + __ldg(a.col + p));
@@ -77,7 +81,8 @@ __device__ __forceinline__ Sides sides(const CsrArgs& a, int k, const double2* _
     return Sides{L, R};
 }
 
-__global__ void __launch_bounds__(256) csr_comm_kernel(CsrArgs a, const double2* __restrict__ u, double2* __restrict__ B)
+template <int U>
+__global__ void __launch_bounds__(256, 6) csr_comm_kernel(CsrArgs a, const double2* __restrict__ u, double2* __restrict__ B)
 {
     const int D = 1 << a.logd;
     const long long D2 = static_cast<long long>(D) * D;
@@ -89,7 +94,7 @@ __global__ void __launch_bounds__(256) csr_comm_kernel(CsrArgs a, const double2*
         const long long e = ne & (D2 - 1);
         const int r = static_cast<int>(e >> a.logd), c = static_cast<int>(e & (D - 1));
         for (int j = 0; j < a.J; ++j) {
-            const Sides s = sides(a, 1 + j, u + n * D2, r, c);
+            const Sides s = sides<U>(a, 1 + j, u + n * D2, r, c);
             const long long idx = static_cast<long long>(j) * HD2 + ne;
             B[idx] = make_double2(s.left.x - s.right.x, s.left.y - s.right.y);
             B[total + idx] = make_double2(s.left.x + s.right.x, s.left.y + s.right.y);
@@ -97,7 +102,8 @@ __global__ void __launch_bounds__(256) csr_comm_kernel(CsrArgs a, const double2*
     }
 }
 
-__global__ void __launch_bounds__(256)
+template <int U>
+__global__ void __launch_bounds__(256, U == 1 ? 4 : 5)
     csr_combine_kernel(CsrArgs a, const double2* __restrict__ u, const double2* __restrict__ B, const double2* rho,
                        double2* out, double alpha, int base_kind)
 {
@@ -114,7 +120,7 @@ __global__ void __launch_bounds__(256)
         const double2 x = un[e];
         // -g u - i [H, u]
         const double g = a.gsum[n];
-        const Sides h = sides(a, 0, un, r, c);
+        const Sides h = sides<U>(a, 0, un, r, c);
         const double cr = h.left.x - h.right.x, ci = h.left.y - h.right.y;
         double re = -g * x.x + ci;
         double im = -g * x.y - cr;
@@ -150,7 +156,7 @@ __global__ void __launch_bounds__(256)
             }
             // -Xi [V, B_n] - i kappa {V, B_n} = (-Xi - i kappa) V B + (Xi - i kappa) B V
             const double xi = a.xi[j], ka = a.counter[j];
-            const Sides s = sides(a, 1 + j, Bj + n * D2, r, c);
+            const Sides s = sides<U>(a, 1 + j, Bj + n * D2, r, c);
             re += -xi * s.left.x + ka * s.left.y + xi * s.right.x + ka * s.right.y;
             im += -xi * s.left.y - ka * s.left.x + xi * s.right.y - ka * s.right.x;
         }
@@ -226,9 +232,16 @@ unsigned grid_for(long long n)
 void launch_csr_stage(const CsrArgs& a, const double2* u, double2* B, const double2* rho, double2* out, double alpha,
                       int base_kind, cudaStream_t s)
 {
-    const long long D2 = 1ll << (2 * a.logd);
-    csr_comm_kernel<<<grid_for(a.H * D2), 256, 0, s>>>(a, u, B);
-    csr_combine_kernel<<<grid_for(a.H * D2), 256, 0, s>>>(a, u, B, rho, out, alpha, base_kind);
+    // the rows of small matrices are too short for two entries side by side (d = 4, two baths, 4845 ADOs 83 us a step
+    // with two, 67 with one)
+    const unsigned grid = grid_for(a.H << (2 * a.logd));
+    if (a.logd >= 6) {
+        csr_comm_kernel<2><<<grid, 256, 0, s>>>(a, u, B);
+        csr_combine_kernel<2><<<grid, 256, 0, s>>>(a, u, B, rho, out, alpha, base_kind);
+    } else {
+        csr_comm_kernel<1><<<grid, 256, 0, s>>>(a, u, B);
+        csr_combine_kernel<1><<<grid, 256, 0, s>>>(a, u, B, rho, out, alpha, base_kind);
+    }
 }
 
 void launch_observables_csr(const double2* rho0, int logd, const int32_t* ptr, const int32_t* col,
