@@ -860,6 +860,19 @@ bool launch_dense(const LargeArgs<float>& a, const float2* u, const float2* rho,
     return true;
 }
 
+// A CTA per half of a tile's rows (double): always while the tiles do not fill the SMs, then while the SM with the most
+// halves has less to do than the one with the most tiles, as long as there are few rounds.  us a step, tiles and halves:
+// d = 128, 28 ADOs (84 tiles) 111 and 96, 66 (198) 148 and 132, but 120 (360) 179 and 185; d = 256, 15 ADOs (150) 155 and
+// 141, 29 (290: two tiles or four halves on an SM) 188 and 198, 45 (450) 232 and 222, 165 (1650) 627 and 663; d = 512, 5
+// ADOs (180) 196 and 174, 9 (324) 239 and 230, 13 (468) 308 and 297.
+inline bool half_tiles(long long tiles, int logd)
+{
+    constexpr long long kSms = 148;
+    if (tiles <= kSms) return true;
+    if (tiles > (logd == 7 ? 3 * kSms / 2 : 13 * kSms / 4)) return false;
+    return (2 * tiles + kSms - 1) / kSms < 2 * ((tiles + kSms - 1) / kSms);
+}
+
 template <typename R, int LOGD>
 bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* out, double alpha, int base,
               cudaStream_t s, bool launch)
@@ -883,9 +896,8 @@ bool launch_t(const LargeArgs<R>& a, const C2<R>* u, const C2<R>* rho, C2<R>* ou
     constexpr long long kBlocks = (1 << LOGD) / 64;
     const long long nb = (a.H - a.first_ado) * (a.herm ? kBlocks * (kBlocks + 1) / 2 : kBlocks * kBlocks);
     if (nb <= 0) return true;
-    // fewer tiles than SMs: a CTA per half of a tile's rows (d = 128, 28 ADOs 99 us a step, 113 without)
     LargeArgs<R> t = a;
-    t.halves = sizeof(R) == sizeof(double) && nb <= 148 ? 1 : 0;
+    t.halves = sizeof(R) == sizeof(double) && half_tiles(nb, LOGD) ? 1 : 0;
     kernel<<<static_cast<unsigned>(t.halves ? 2 * nb : nb), kTileT, smem, s>>>(t, u, rho, out, alpha, base);
     return true;
 }

@@ -244,3 +244,26 @@ def test_few_packed_tiles_match_oracle(n, baths, K, collective):
         ctx.step(2)
         ctx.sync()
         assert np.max(np.abs(ctx.state() - want)) < TOL
+
+
+@pytest.mark.parametrize("n,baths,K,size", [
+    (7, 5, 1, 66),   # 198 tiles: two CTAs per tile
+    (7, 6, 1, 91),   # 273 tiles: one
+    (8, 5, 0, 21),   # 210 tiles: two
+    (8, 6, 0, 28),   # 280 tiles: one
+    (8, 8, 0, 45),   # 450 tiles: two
+])
+def test_tiles_in_rounds_match_oracle(n, baths, K, size):
+    """Packed double-precision tiles in one to four rounds over the SMs, whole or
+    by halves: right-hand side within 1e-12 of its largest element."""
+    p = S.spin_glass(n, seed=90 + n, depth=2, K=K, h=0.5, dt=0.005)
+    p.baths = p.baths[:baths]
+    rng = np.random.default_rng(n)
+    o = O.Oracle(p)
+    assert o.size == size
+    x = _hermitian((rng.standard_normal((o.size, p.dim, p.dim)) + 1j * rng.standard_normal((o.size, p.dim, p.dim))) * 0.05)
+    ref = o.rhs(x)
+    o.close()
+    with capi.Context(p) as ctx:
+        ctx.set_state(x)
+        assert np.max(np.abs(ctx.rhs() - ref)) < 1e-12 * max(1.0, np.max(np.abs(ref)))
