@@ -526,7 +526,7 @@ bool plan_run(int logd, int M, int J, bool pauli, long long H, int sms, bool sol
     p.smem += p.cap * slab;
     // with less room than three entries per slab in hand the run waits on every entry by itself: d = 16, 12 modes,
     // 1820 ADOs 120 us a step, 68 with a launch per stage; 1716 ADOs, where 18 entries fit, 47 and 67
-    return p.cap >= 3 * p.apc;
+    return p.cap >= std::min(3, 2 * M) * p.apc;  // (one mode has two entries at most)
 }
 
 template <int LOGD, bool PAULI, bool SOLO>

@@ -449,3 +449,18 @@ def test_many_small_slabs_of_sparse_operators_match_oracle(n, K, depth, size):
         assert ctx.stage_path == "csr" and ctx.size == size
         rho, en = ctx.step_trace(3)
     assert np.max(np.abs(rho - rho_ref)) <= TOL and np.max(np.abs(en - en_ref)) <= TOL
+
+
+@pytest.mark.parametrize("kind,n,depth", [("spin", 2, 80), ("spin", 3, 37), ("spin", 4, 5), ("spin", 4, 40),
+                                          ("collective", 3, 20)])
+def test_one_mode_runs_whole_steps_in_one_launch(kind, n, depth):
+    """A single mode gives an ADO two neighbours at most: the staging area then
+    holds all of them, however few, and whole steps run in one launch."""
+    p = _run_problem(kind, n, 1, 0, depth)
+    o = O.Oracle(p)
+    rho_ref, en_ref = o.run(5, trace=True)
+    o.close()
+    with capi.Context(p) as ctx:
+        assert ctx.size == depth + 1 and ctx.get_info().kernels_per_step == 1
+        rho, en = ctx.step_trace(5)
+    assert np.max(np.abs(rho - rho_ref)) <= TOL and np.max(np.abs(en - en_ref)) <= TOL
