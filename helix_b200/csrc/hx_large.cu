@@ -645,9 +645,10 @@ __global__ void __launch_bounds__(kTileT, TileShape<R, LOGD>::MINB)
 
 // Up term of tier L-1 in the working precision, tile-major so the top-tier
 // data of the resident tiles stays in L2 (as upterm_kernel, hx_upterm.cu).
-constexpr int kUpWarps = 8, kUpSlots = 4, kUpTile = 32;
+constexpr int kUpWarps = 8, kUpTile = 32;
 
-template <typename R>
+// A warp takes SLOTS slots side by side and asks for MODES neighbours of each at a time.
+template <typename R, int SLOTS, int MODES>
 __global__ void __launch_bounds__(kUpWarps * 32)
     large_upterm_kernel(LargeUpArgs<R> a, const C2<R>* __restrict__ u, C2<R>* __restrict__ U)
 {
@@ -667,13 +668,13 @@ __global__ void __launch_bounds__(kUpWarps * 32)
         if (a.upper && (c >> 6) < (r >> 6)) return;  // a tile that nobody reads
     }
     const C* ue = u + e;
-    const int s0 = (blockIdx.x * kUpWarps + warp) * kUpSlots;
-    const int ns = min(a.S - s0, kUpSlots);
+    const int s0 = (blockIdx.x * kUpWarps + warp) * SLOTS;
+    const int ns = min(a.S - s0, SLOTS);
     if (ns <= 0) return;
-    const int32_t* slab[kUpSlots];
-    R re[kUpSlots], im[kUpSlots];
+    const int32_t* slab[SLOTS];
+    R re[SLOTS], im[SLOTS];
 #pragma unroll
-    for (int t = 0; t < kUpSlots; ++t) {
+    for (int t = 0; t < SLOTS; ++t) {
         slab[t] = a.slab + static_cast<long long>(s0 + min(t, ns - 1)) * a.M;
         re[t] = im[t] = 0;
     }
@@ -681,28 +682,43 @@ __global__ void __launch_bounds__(kUpWarps * 32)
         const R del = __ldg(a.vdiag + j * D + r) - __ldg(a.vdiag + j * D + c);
         if (del == R(0)) continue;
         const int m1 = __ldg(a.bath_off + j + 1);
-        R sr[kUpSlots], si[kUpSlots];
+        R sr[SLOTS], si[SLOTS];
 #pragma unroll
-        for (int t = 0; t < kUpSlots; ++t) sr[t] = si[t] = 0;
-        for (int m = __ldg(a.bath_off + j); m < m1; ++m) {
-            C y[kUpSlots];
+        for (int t = 0; t < SLOTS; ++t) sr[t] = si[t] = 0;
+        for (int m = __ldg(a.bath_off + j); m < m1; m += MODES) {
+            C y[MODES][SLOTS];
 #pragma unroll
-            for (int t = 0; t < kUpSlots; ++t) y[t] = __ldg(ue + static_cast<long long>(__ldg(slab[t] + m)) * D2);
+            for (int i = 0; i < MODES; ++i)
 #pragma unroll
-            for (int t = 0; t < kUpSlots; ++t) {
-                sr[t] += y[t].x;
-                si[t] += y[t].y;
-            }
+                for (int t = 0; t < SLOTS; ++t)
+                    if (m + i < m1) y[i][t] = __ldg(ue + static_cast<long long>(__ldg(slab[t] + m + i)) * D2);
+#pragma unroll
+            for (int i = 0; i < MODES; ++i)
+#pragma unroll
+                for (int t = 0; t < SLOTS; ++t)
+                    if (m + i < m1) {
+                        sr[t] += y[i][t].x;
+                        si[t] += y[i][t].y;
+                    }
         }
 #pragma unroll
-        for (int t = 0; t < kUpSlots; ++t) {
+        for (int t = 0; t < SLOTS; ++t) {
             re[t] += del * si[t];  // -i del S
             im[t] -= del * sr[t];
         }
     }
 #pragma unroll
-    for (int t = 0; t < kUpSlots; ++t)
+    for (int t = 0; t < SLOTS; ++t)
         if (t < ns) U[static_cast<long long>(s0 + t) * D2 + e] = mk<R>(re[t], im[t]);
+}
+
+template <typename R, int SLOTS, int MODES>
+void launch_upterm_t(const LargeUpArgs<R>& a, const C2<R>* u, C2<R>* U, cudaStream_t s)
+{
+    const long long D2 = a.herm ? herm_elems(a.logd) : 1ll << (2 * a.logd);
+    constexpr int per = kUpWarps * SLOTS;
+    const dim3 grid((a.S + per - 1) / per, static_cast<unsigned>((D2 + kUpTile - 1) / kUpTile));
+    large_upterm_kernel<R, SLOTS, MODES><<<grid, kUpWarps * 32, 0, s>>>(a, u, U);
 }
 
 // Tier-0 ADO of the mixed-precision propagator in double precision: its own
@@ -952,10 +968,12 @@ template <typename R>
 void launch_large_upterm(const LargeUpArgs<R>& a, const C2<R>* u, C2<R>* U, cudaStream_t s)
 {
     if (a.S <= 0) return;
-    const long long D2 = a.herm ? herm_elems(a.logd) : 1ll << (2 * a.logd);
-    const int per = kUpWarps * kUpSlots;
-    dim3 grid((a.S + per - 1) / per, static_cast<unsigned>((D2 + kUpTile - 1) / kUpTile));
-    large_upterm_kernel<R><<<grid, kUpWarps * 32, 0, s>>>(a, u, U);
+    // few slots: four modes of one slot at a time, else the warps wait on one neighbour after the other.  us a step in
+    // double, four slots side by side and this: d = 128, 28 modes 1 slot 112 and 92, 12 modes 12 slots 162 and 140, 14
+    // modes 14 slots 179 and 171, but 8 modes 36 slots 214 and 219; d = 256, 8 modes 8 slots 224 and 206, 36 slots 626
+    // and 644; eight modes at a time 116, 152, 179, 241, 220 and 726.
+    if (a.S <= 16) launch_upterm_t<R, 1, 4>(a, u, U, s);
+    else launch_upterm_t<R, 4, 1>(a, u, U, s);
 }
 
 template bool prepare_large<double>(const LargeArgs<double>&);

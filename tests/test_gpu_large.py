@@ -267,3 +267,24 @@ def test_tiles_in_rounds_match_oracle(n, baths, K, size):
     with capi.Context(p) as ctx:
         ctx.set_state(x)
         assert np.max(np.abs(ctx.rhs() - ref)) < 1e-12 * max(1.0, np.max(np.abs(ref)))
+
+
+@pytest.mark.parametrize("baths,K,depth,slots", [
+    (7, 3, 1, 1), (5, 2, 1, 1), (3, 0, 2, 3),    # four modes of a bath at a time: four, three, one of them
+    (4, 3, 2, 16), (2, 2, 3, 21), (6, 0, 3, 21),  # the most slots that take that form; four slots at a time
+])
+def test_up_terms_of_few_and_many_slots_match_oracle(baths, K, depth, slots):
+    """Up terms of tier L-1 at d = 128 with one slot per warp and with four:
+    right-hand side within 1e-12 of its largest element."""
+    p = S.spin_glass(7, seed=97, depth=depth, K=K, h=0.5, dt=0.005)
+    p.baths = p.baths[:baths]
+    rng = np.random.default_rng(slots)
+    o = O.Oracle(p)
+    modes = baths * (K + 1)
+    assert slots == S.hierarchy_size(modes, depth) - S.hierarchy_size(modes, depth - 1)  # ADOs of the tier below the top
+    x = _hermitian((rng.standard_normal((o.size, p.dim, p.dim)) + 1j * rng.standard_normal((o.size, p.dim, p.dim))) * 0.05)
+    ref = o.rhs(x)
+    o.close()
+    with capi.Context(p) as ctx:
+        ctx.set_state(x)
+        assert np.max(np.abs(ctx.rhs() - ref)) < 1e-12 * max(1.0, np.max(np.abs(ref)))
