@@ -44,17 +44,19 @@ __device__ __forceinline__ bool grid_barrier(unsigned* count, unsigned k, const 
 {
     const unsigned all = k * gridDim.x;
     int late = 0;
-    if (grid_arrive(count) & kRunAborted) {
-        late = 1;
-    } else if (threadIdx.x == 0) {
+    // looked at only where a mark is found, so that the polling does not wait for it (0.2 us a barrier: 6 ADOs at d = 32
+    // 15.2 us a step, 14.4 so)
+    const unsigned before = grid_arrive(count);
+    if (threadIdx.x == 0) {
+        const unsigned target = all + w.skew;
         for (uint32_t it = 0;; ++it) {
             unsigned v;
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+            if (static_cast<int>(v - target) >= 0 && !(v & kRunAborted)) break;
             if (v & kRunAborted) {
-                late = (v & ~kRunAborted) < all + gridDim.x;  // at this barrier, not at the next
+                late = (v & ~kRunAborted) < all + gridDim.x || (before & kRunAborted);
                 break;
             }
-            if (static_cast<int>(v - all - w.skew) >= 0) break;
             if (it >= w.max_polls && atomicCAS(count, v, kRunAborted | all) == v) {
                 late = 1;
                 break;
